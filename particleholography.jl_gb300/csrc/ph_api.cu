@@ -952,6 +952,27 @@ int recon_group(int nbatch, int nx_rows_a, bool chain, int cap_override = 0) {
     return std::max(1, std::min(cap, nbatch / groups));
 }
 
+// Slices one pass B CTA transforms.  Where pass B runs the two-stage transform
+// its CTAs are small and equal, so the launch takes about ceil(CTAs / resident
+// CTAs) rounds of (group + 2) slice times (a start and a merge per CTA weigh
+// about two slices): the group of least time, at most 64 slices.  `group`:
+// pass A's choice, kept at the other lengths and under the tuner's cap.
+int recon_group_b(int nbatch, int n, int rows, int items, int group, int cap_override) {
+    const int ctas = recon_b_ctas(n, rows) * items;
+    if (cap_override > 0 || ctas <= 0) return group;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 1;
+    const long long slots = (long long)sms * recon_b_ctas_per_sm(n);
+    int best = 1;
+    long long cost = -1;
+    for (int g = 1; g <= std::min(nbatch, 64); ++g) {
+        const long long c = ((long long)ctas * ((nbatch + g - 1) / g) + slots - 1) / slots * (g + 2);
+        if (cost < 0 || c <= cost) { cost = c; best = g; }
+    }
+    return best;
+}
+
 // Tensor map of the slice intermediate T = [nb][ny_out][nx] float2 (8-byte
 // elements) for pass A's tiled store: boxes of box_kx kx x 256 y x 1 slice.
 bool t_store_map(CUtensorMap *tm, float2 *t, int nx, int ny_out, int nb, int box_kx) {
@@ -1011,6 +1032,7 @@ int issue_recon_slices(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin
         const ph_tuning *tu = tuning_of(ctx, nx, ny);
         const bool ts_shape = recon_a_tstore(ny) && y0 == 0 && ny_out == ny;   // the tensor-map store form
         const int group = recon_group(nb, row_blocks_a, recon_a_chain(ny, ts_shape), tu ? tu->group_cap : 0);
+        const int group_b = recon_group_b(nb, nx, ny_out, 1, group, tu ? tu->group_cap : 0);
         const auto fill_a = [&](auto &a) {
             a.state = state;
             a.t = t;
@@ -1043,20 +1065,20 @@ int issue_recon_slices(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin
         } else if (kind == RK_PROJ) {
             ReconB<EPI_PROJ> b{};
             b.t = t; b.tw = tw_x; b.proj64 = p64; b.rows = ny_out; b.nx_out = nx_out; b.x0 = 0;
-            b.k0 = k0; b.nbatch = nb; b.group = group; b.vol_slice_stride = (long long)nx_out * ny_out;
+            b.k0 = k0; b.nbatch = nb; b.group = group_b; b.vol_slice_stride = (long long)nx_out * ny_out;
             b.err = static_cast<int *>(ctx->small);
             PH_TRY(pass(ctx, s, "recon_b",[&] { return launch_recon_b(nx, b, s); }));
         } else if (kind == RK_SUB) {
             ReconB<EPI_SUB> b{};
             b.t = t; b.tw = tw_x; b.vol = vol; b.rows = ny_out; b.nx_out = nx_out; b.x0 = 0;
-            b.k0 = k0; b.nbatch = nb; b.group = group;
+            b.k0 = k0; b.nbatch = nb; b.group = group_b;
             b.row_ptr = sub->row_ptr; b.row_box = sub->row_box; b.boxes = sub->boxes;
             b.err = static_cast<int *>(ctx->small);
             PH_TRY(pass(ctx, s, "recon_b",[&] { return launch_recon_b(nx, b, s); }));
         } else if (kind == RK_CVOL) {
             ReconB<EPI_CVOL> b{};
             b.t = t; b.tw = tw_x; b.vol = vol; b.rows = ny_out; b.nx_out = nx_out; b.x0 = 0;
-            b.k0 = k0; b.nbatch = nb; b.group = group; b.vol_slice_stride = (long long)nx_out * ny_out;
+            b.k0 = k0; b.nbatch = nb; b.group = group_b; b.vol_slice_stride = (long long)nx_out * ny_out;
             b.err = static_cast<int *>(ctx->small);
             PH_TRY(pass(ctx, s, "recon_b",[&] { return launch_recon_b(nx, b, s); }));
         } else {
@@ -1064,7 +1086,7 @@ int issue_recon_slices(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin
             b.t = t; b.tw = tw_x; b.vol = vol; b.vol_dtype = vol_dtype; b.proj64 = want_proj ? p64 : nullptr;
             b.threshold = threshold;
             b.rows = ny_out; b.nx_out = nx_out; b.x0 = x0;
-            b.k0 = k0; b.nbatch = nb; b.group = group; b.vol_slice_stride = (long long)nx_out * ny_out;
+            b.k0 = k0; b.nbatch = nb; b.group = group_b; b.vol_slice_stride = (long long)nx_out * ny_out;
             b.err = static_cast<int *>(ctx->small);
             PH_TRY(pass(ctx, s, "recon_b",[&] { return launch_recon_b(nx, b, s); }));
         }
@@ -1259,7 +1281,7 @@ int issue_recon_group(ph_ctx *ctx, const std::vector<const ph_recon_item *> &its
             const int nb = std::max(0, std::min(L.batch, (int)its[i]->slices - k0));
             const int grp = nb > 0 ? recon_group(nb, row_blocks_a, recon_a_chain(ny), tu ? tu->group_cap : 0) : 1;
             a.set_item(i, nb, grp);
-            b.set_item(i, nb, grp);
+            b.set_item(i, nb, nb > 0 ? recon_group_b(nb, nx, ny, G, grp, tu ? tu->group_cap : 0) : 1);
         }
         a.state = reinterpret_cast<const float4 *>(slot(0, L.state));
         a.t = reinterpret_cast<float2 *>(slot(0, L.t));

@@ -1,7 +1,7 @@
 // Grouped launches of reconstruction passes A and B (projection): one launch
 // for up to kMaxItems holograms of one transform shape, grid z = item, grid y
 // = the largest item's slice groups (ph_passes.cuh, GROUPED forms).
-#include "ph_launch.cuh"
+#include "ph_two_b.cuh"
 
 namespace ph {
 
@@ -28,7 +28,14 @@ cudaError_t launch_recon_a_group_tstore(int n, const ReconAGroupedTStore &b, con
 cudaError_t launch_recon_b_group(int n, const ReconB<EPI_PROJ, true> &b, cudaStream_t s) {
     int gy = 1;
     for (int i = 0; i < b.nitems; ++i) gy = std::max(gy, (b.item_nb(i) + b.item_group(i) - 1) / b.item_group(i));
-    return launch_len<false>(n, b, b.rows, gy, s, b.nitems);
+    switch (n) {
+        case 256: return two::launch_b<256>(b, gy, b.nitems, s);
+        case 512: return two::launch_b<512>(b, gy, b.nitems, s);
+        case 1024: return two::launch_b<1024>(b, gy, b.nitems, s);
+        case 2048: return two::launch_b<2048>(b, gy, b.nitems, s);
+        case 4096: return two::launch_b<4096>(b, gy, b.nitems, s);
+    }
+    return launch_engine_len<false>(n, b, b.rows, gy, s, b.nitems);
 }
 
 }  // namespace ph

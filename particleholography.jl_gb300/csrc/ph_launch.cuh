@@ -13,6 +13,12 @@ namespace ph {
     X(1) X(2) X(4) X(8) X(16) X(32) X(64) X(128) X(256) X(512) X(1024) X(2048) X(4096) X(8192) X(3) X(6) \
         X(12) X(24) X(48) X(96) X(192) X(384) X(768) X(1536) X(3072) X(6144)
 
+// The lengths whose pass B runs the row engine of ph_fft.cuh (256 .. 4096 run
+// the two-stage transform of ph_two.cuh).
+#define PH_FOR_EACH_N_ENGINE(X)                                                                          \
+    X(1) X(2) X(4) X(8) X(16) X(32) X(64) X(128) X(8192) X(3) X(6) X(12) X(24) X(48) X(96) X(192) X(384) \
+        X(768) X(1536) X(3072) X(6144)
+
 inline bool supported_len(int n) {
     if (n < 1) return false;
     if ((n & (n - 1)) == 0) return n <= 8192;
@@ -225,6 +231,17 @@ cudaError_t launch_len(int n, const Body &body, int nrows, int grid_y, cudaStrea
     return cudaErrorInvalidValue;
 }
 
+// launch_len over PH_FOR_EACH_N_ENGINE.
+template <bool ROW_FAST, class Body>
+cudaError_t launch_engine_len(int n, const Body &body, int nrows, int grid_y, cudaStream_t s, int grid_z = 1) {
+    switch (n) {
+#define PH_LAUNCH_CASE(N) case N: return launch_one<N, ROW_FAST>(body, nrows, grid_y, s, grid_z);
+        PH_FOR_EACH_N_ENGINE(PH_LAUNCH_CASE)
+#undef PH_LAUNCH_CASE
+    }
+    return cudaErrorInvalidValue;
+}
+
 // ---- launchers, one translation unit each (compiled in parallel)
 
 // (grouped launches: grid z = b.nitems; pass A / pass B grid y = the largest item's slice groups)
@@ -261,6 +278,10 @@ cudaError_t launch_recon_b_group(int n, const ReconB<EPI_PROJ, true> &b, cudaStr
 int recon_a_rows(int n);   // rows per pass A CTA for transform length n
 bool recon_a_chain(int n, bool tstore = false);   // whether pass A at length n (in the tensor-map
                                                   // store form) advances X by the product chain
+// Pass B at 256 .. 4096 runs the two-stage transform (ph_two_b.cuh): its CTAs
+// per slice group over `rows` rows, and per SM (0 at the other lengths).
+int recon_b_ctas(int n, int rows);
+int recon_b_ctas_per_sm(int n);
 cudaError_t launch_recon_b(int n, const ReconB<EPI_PROJ> &b, cudaStream_t s);
 cudaError_t launch_recon_b(int n, const ReconB<EPI_VOL> &b, cudaStream_t s);
 cudaError_t launch_recon_b(int n, const ReconB<EPI_CVOL> &b, cudaStream_t s);

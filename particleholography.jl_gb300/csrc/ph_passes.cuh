@@ -794,7 +794,9 @@ __device__ __forceinline__ float clamp01(float v) { return fminf(fmaxf(v, 0.0f),
 // first the bulk-copy target (dense rows) and then, after the first stage has
 // read it, the exchange rows of that slice's transform.  CTAs are small (128
 // threads: one row at N >= 2048) so that the barriers of the FFT stages span
-// only the warps that exchange data, and RTS / 128 CTAs share an SM.
+// only the warps that exchange data, and RTS / 128 CTAs share an SM.  The
+// lengths 256 .. 4096 run the two-stage transform instead (ph_two_b.cuh), with
+// these parameters.
 template <int EPI, bool GROUPED = false>   // GROUPED: the grouped-launch form (EPI_PROJ, grid z = item)
 struct ReconB : PassBase, std::conditional_t<GROUPED, ReconItems, NoItems> {
     static constexpr int TT = 128;

@@ -1,0 +1,38 @@
+"""The two-stage row transform of pass B (lengths 256 .. 4096) against the oracle
+at its edges: a CTA with fewer rows than it holds, a warp of two rows with one,
+one slice, slice counts that leave the last group short."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import ref_semantics as ref
+from phtest import rel_l2, to_dev, to_np
+
+pytestmark = pytest.mark.gpu
+LAM, DX = 0.6328, 10.0
+# An FP32 FFT of 2^22 points is good to ~ eps log2(n) / sqrt(2) ~ 1e-6 in relative L2, on
+# either side; pass A's product chain adds eps / 2 per slice.
+TOL = 5e-6
+
+
+@pytest.mark.parametrize("nx,ny,slices", [(256, 1, 1), (256, 3, 5), (256, 24, 33), (512, 1, 2), (512, 6, 65),
+                                          (512, 96, 7), (1024, 3, 3), (1024, 6, 34), (2048, 1, 5), (2048, 3, 3),
+                                          (2048, 12, 17), (4096, 1, 2), (4096, 3, 9)])
+def test_rows_and_slices_at_the_edges(ph, cuda, nx, ny, slices):
+    rng = np.random.default_rng(nx + ny)
+    holo = rng.uniform(0.1, 1.0, (ny, nx)).astype(np.float32)
+    d = ref.transfer_sqrt_arr(nx, LAM, DX, n_slow=ny)
+    hf, hdz = ref.transfer(-1000.0, nx, LAM, d), ref.transfer(-200.0, nx, LAM, d)
+    args = (ph.cu_gabor_wavefront(to_dev(holo, cuda)), ph.CuTransfer(to_dev(hf, cuda)), ph.CuTransfer(to_dev(hdz, cuda)),
+            slices)
+    wave = ref.gabor_wavefront(holo)
+    field = ref.reconst_complex_vol(wave, hf, hdz, slices)
+    assert rel_l2(to_np(ph.cu_get_reconst_complex_vol(*args)), field) < TOL
+    proj, arg = ph.cu_get_reconst_xyprojection(*args, return_argmin=True)
+    p_ref, a_ref = ref.reconst_xyprojection(wave, hf, hdz, slices, with_argmin=True)
+    assert rel_l2(to_np(proj), p_ref) < TOL
+    assert np.mean(to_np(arg) == a_ref) >= 0.999
+    vol, vproj = ph.cu_get_reconst_vol_and_xyprojection(*args, torch.float32)
+    want = np.clip(np.abs(field.astype(np.complex128)) ** 2, 0.0, 1.0)
+    assert rel_l2(to_np(vol), want) < TOL
+    assert torch.equal(vproj, vol.amin(0))
