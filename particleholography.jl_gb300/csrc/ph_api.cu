@@ -952,38 +952,51 @@ int recon_group(int nbatch, int nx_rows_a, bool chain, int cap_override = 0) {
     return std::max(1, std::min(cap, nbatch / groups));
 }
 
-// Slices one pass B CTA transforms.  Where pass B runs the two-stage transform
-// its CTAs are small and equal, so the launch takes about ceil(CTAs / resident
-// CTAs) rounds of (group + 2) slice times (a start and a merge per CTA weigh
-// about two slices): the group of least time, at most 64 slices.  `group`:
-// pass A's choice, kept at the other lengths and under the tuner's cap.
-int recon_group_b(int nbatch, int n, int rows, int items, int group, int cap_override) {
-    const int ctas = recon_b_ctas(n, rows) * items;
-    if (cap_override > 0 || ctas <= 0) return group;
+// Slices per CTA of a two-stage pass (small and equal CTAs, `ctas` per slice
+// group, `per_sm` resident): a launch takes about ceil(CTAs / resident) rounds
+// of (group + start) slice times, where `start` is what a CTA's beginning and
+// end weigh (pass A: forming Hdz and X, 3 slices; pass B: the merge of the
+// minima, 2).  The group of least time, at most 64 slices.
+int rounds_group(int nbatch, int ctas, int per_sm, int start, int cap_override) {
+    if (cap_override > 0) return std::max(1, std::min(cap_override, nbatch));
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 1;
-    const long long slots = (long long)sms * recon_b_ctas_per_sm(n);
+    const long long slots = (long long)sms * per_sm;
     int best = 1;
     long long cost = -1;
     for (int g = 1; g <= std::min(nbatch, 64); ++g) {
-        const long long c = ((long long)ctas * ((nbatch + g - 1) / g) + slots - 1) / slots * (g + 2);
+        const long long c = ((long long)ctas * ((nbatch + g - 1) / g) + slots - 1) / slots * (g + start);
         if (cost < 0 || c <= cost) { cost = c; best = g; }
     }
     return best;
+}
+
+// Slices per CTA of pass A (rows kx of length ny) and of pass B (`items` frames
+// of rows y of length nx) over a batch of nbatch slices.
+int recon_group_a(int nbatch, int nx, int ny, int y0, int ny_out, int cap_override) {
+    if (recon_a_two(ny, y0, ny_out)) {
+        const int box = recon_a_two_box(ny);
+        return rounds_group(nbatch, (nx + box - 1) / box, recon_a_two_ctas_per_sm(ny), 3, cap_override);
+    }
+    return recon_group(nbatch, (nx + recon_a_rows(ny) - 1) / recon_a_rows(ny), recon_a_chain(ny), cap_override);
+}
+int recon_group_b(int nbatch, int nx, int rows, int items, int group_a, int cap_override) {
+    const int ctas = recon_b_ctas(nx, rows) * items;
+    return ctas > 0 ? rounds_group(nbatch, ctas, recon_b_ctas_per_sm(nx), 2, cap_override) : group_a;
 }
 
 // Tensor map of the slice intermediate T = [nb][ny_out][nx] float2 (8-byte
 // elements) for pass A's tiled store: boxes of box_kx kx x 256 y x 1 slice.
 bool t_store_map(CUtensorMap *tm, float2 *t, int nx, int ny_out, int nb, int box_kx) {
     const EncodeTiledFn enc = encode_tiled();
-    if (enc == nullptr || ((uintptr_t)t & 15) != 0 || nx % 4 != 0 || box_kx < 4 || box_kx > 32) return false;
+    if (enc == nullptr || ((uintptr_t)t & 15) != 0 || nx % 4 != 0 || (box_kx != 4 && box_kx != 8 && box_kx != 16)) return false;
     const cuuint64_t dims[3] = {(cuuint64_t)nx, (cuuint64_t)ny_out, (cuuint64_t)nb};
     const cuuint64_t strides[2] = {(cuuint64_t)nx * 8, (cuuint64_t)nx * ny_out * 8};
-    const cuuint32_t box[3] = {(cuuint32_t)box_kx, (cuuint32_t)ReconATStore::kBoxY, 1};
+    const cuuint32_t box[3] = {(cuuint32_t)box_kx, (cuuint32_t)kTwoBoxY, 1};
     const cuuint32_t estr[3] = {1, 1, 1};
     return enc(tm, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, t, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+               box_kx == 16 ? CU_TENSOR_MAP_SWIZZLE_128B : box_kx == 8 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -1006,15 +1019,15 @@ bool gs_store_map(CUtensorMap *tm, float2 *p, int inner, int outer, int rows) {
 bool t_store_map_items(CUtensorMap *tm, float2 *t, int nx, int ny, int nb, int nitems, size_t item_bytes,
                        int box_kx) {
     const EncodeTiledFn enc = encode_tiled();
-    if (enc == nullptr || ((uintptr_t)t & 15) != 0 || nx % 4 != 0 || box_kx < 4 || box_kx > 32 ||
+    if (enc == nullptr || ((uintptr_t)t & 15) != 0 || nx % 4 != 0 || (box_kx != 4 && box_kx != 8 && box_kx != 16) ||
         item_bytes % 16 != 0)
         return false;
     const cuuint64_t dims[4] = {(cuuint64_t)nx, (cuuint64_t)ny, (cuuint64_t)nb, (cuuint64_t)nitems};
     const cuuint64_t strides[3] = {(cuuint64_t)nx * 8, (cuuint64_t)nx * ny * 8, (cuuint64_t)item_bytes};
-    const cuuint32_t box[4] = {(cuuint32_t)box_kx, (cuuint32_t)ReconATStore::kBoxY, 1, 1};
+    const cuuint32_t box[4] = {(cuuint32_t)box_kx, (cuuint32_t)kTwoBoxY, 1, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     return enc(tm, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4, t, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+               box_kx == 16 ? CU_TENSOR_MAP_SWIZZLE_128B : box_kx == 8 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -1026,33 +1039,20 @@ int issue_recon_slices(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin
                        cudaStream_t s, float threshold, int first, const SubArgs *sub) {
     ReconLayout L{};
     L.batch = batch;
-    const int row_blocks_a = (nx + recon_a_rows(ny) - 1) / recon_a_rows(ny);
     for (int k0 = first; k0 < first + slices; k0 += L.batch) {
         const int nb = std::min(L.batch, first + slices - k0);
         const ph_tuning *tu = tuning_of(ctx, nx, ny);
-        const bool ts_shape = recon_a_tstore(ny) && y0 == 0 && ny_out == ny;   // the tensor-map store form
-        const int group = recon_group(nb, row_blocks_a, recon_a_chain(ny, ts_shape), tu ? tu->group_cap : 0);
-        const int group_b = recon_group_b(nb, nx, ny_out, 1, group, tu ? tu->group_cap : 0);
-        const auto fill_a = [&](auto &a) {
-            a.state = state;
-            a.t = t;
-            a.tw = tw_y;
-            a.nx = nx;
-            a.ny_out = ny_out;
-            a.y0 = y0;
-            a.k0 = k0;
-            a.nbatch = nb;
-            a.group = group;
-            a.err = static_cast<int *>(ctx->small);
-        };
+        const int cap = tu ? tu->group_cap : 0;
+        const int group = recon_group_a(nb, nx, ny, y0, ny_out, cap);
+        const int group_b = recon_group_b(nb, nx, ny_out, 1, group, cap);
+        ReconA a{};
+        a.state = state; a.t = t; a.tw = tw_y; a.nx = nx; a.ny_out = ny_out; a.y0 = y0;
+        a.k0 = k0; a.nbatch = nb; a.group = group;
+        a.err = static_cast<int *>(ctx->small);
         CUtensorMap tm;
-        if (ts_shape && t_store_map(&tm, t, nx, ny_out, nb, recon_a_tstore_box(ny))) {
-            ReconATStore a{};
-            fill_a(a);
-            PH_TRY(pass(ctx, s, "recon_a", [&] { return launch_recon_a_tstore(ny, a, tm, nb, s); }));
+        if (recon_a_two(ny, y0, ny_out) && t_store_map(&tm, t, nx, ny_out, nb, recon_a_two_box(ny))) {
+            PH_TRY(pass(ctx, s, "recon_a", [&] { return launch_recon_a_two(ny, a, tm, nb, s); }));
         } else {
-            ReconA a{};
-            fill_a(a);
             PH_TRY(pass(ctx, s, "recon_a", [&] { return launch_recon_a(ny, a, nb, s); }));
         }
         if (kind == RK_PROJ && effective_form(ctx, nx, ny) != PH_FORM_FP32) {
@@ -1272,16 +1272,16 @@ int issue_recon_group(ph_ctx *ctx, const std::vector<const ph_recon_item *> &its
     const size_t npix = (size_t)nx * ny;
     for (int i = 0; i < G; ++i)
         PH_CUDA(cudaMemsetAsync(slot(i, L.p64), 0xff, sizeof(unsigned long long) * npix, s), "cudaMemsetAsync");
-    const int row_blocks_a = (nx + recon_a_rows(ny) - 1) / recon_a_rows(ny);
     const ph_tuning *tu = tuning_of(ctx, nx, ny);
+    const int cap = tu ? tu->group_cap : 0;
     for (int k0 = 0; k0 < smax; k0 += L.batch) {
         ReconAGrouped a{};
         ReconB<EPI_PROJ, true> b{};
         for (int i = 0; i < G; ++i) {
             const int nb = std::max(0, std::min(L.batch, (int)its[i]->slices - k0));
-            const int grp = nb > 0 ? recon_group(nb, row_blocks_a, recon_a_chain(ny), tu ? tu->group_cap : 0) : 1;
+            const int grp = nb > 0 ? recon_group_a(nb, nx, ny, 0, ny, cap) : 1;
             a.set_item(i, nb, grp);
-            b.set_item(i, nb, nb > 0 ? recon_group_b(nb, nx, ny, G, grp, tu ? tu->group_cap : 0) : 1);
+            b.set_item(i, nb, nb > 0 ? recon_group_b(nb, nx, ny, G, grp, cap) : 1);
         }
         a.state = reinterpret_cast<const float4 *>(slot(0, L.state));
         a.t = reinterpret_cast<float2 *>(slot(0, L.t));
@@ -1297,21 +1297,8 @@ int issue_recon_group(ph_ctx *ctx, const std::vector<const ph_recon_item *> &its
         a.nitems = G;
         a.err = static_cast<int *>(ctx->small);
         CUtensorMap tm;
-        if (recon_a_group_tstore(ny) &&
-            t_store_map_items(&tm, a.t, nx, ny, L.batch, G, ib, recon_a_tstore_box(ny))) {
-            ReconAGroupedTStore at{};
-            static_cast<ReconItems &>(at) = static_cast<const ReconItems &>(a);
-            at.state = a.state;
-            at.t = a.t;
-            at.tw = a.tw;
-            at.err = a.err;
-            at.nx = a.nx;
-            at.ny_out = a.ny_out;
-            at.y0 = a.y0;
-            at.k0 = a.k0;
-            at.nbatch = a.nbatch;
-            at.group = a.group;
-            PH_TRY(pass(ctx, s, "recon_a", [&] { return launch_recon_a_group_tstore(ny, at, tm, s); }));
+        if (recon_a_two(ny, 0, ny) && t_store_map_items(&tm, a.t, nx, ny, L.batch, G, ib, recon_a_two_box(ny))) {
+            PH_TRY(pass(ctx, s, "recon_a", [&] { return launch_recon_a_group_two(ny, a, tm, s); }));
         } else {
             PH_TRY(pass(ctx, s, "recon_a", [&] { return launch_recon_a_group(ny, a, s); }));
         }

@@ -256,17 +256,18 @@ int spectrum_staged_rows(int n);
 cudaError_t launch_spectrum_staged(int n, const SpectrumColsT &b, const CUtensorMap &tm_hf, const CUtensorMap &tm_hdz,
                                    cudaStream_t s);
 cudaError_t launch_recon_a(int n, const ReconA &b, int nbatch, cudaStream_t s);
-// Pass A with the tensor-map transposed store (lengths where recon_a_tstore holds;
-// tm: T as [nbatch][ny_out = n][nx] 8-byte elements, boxes of 4 x 256 x 1).
-bool recon_a_tstore(int n);
-int recon_a_tstore_box(int n);   // kx per box (rows per CTA x CTAs per cluster)
-cudaError_t launch_recon_a_tstore(int n, const ReconATStore &b, const CUtensorMap &tm, int nbatch, cudaStream_t s);
+// Pass A on the two-stage transform with the tensor-map store (ph_two_a.cuh):
+// lengths 256 .. 4096, frames whose stored rows [y0, y0 + ny_out) are whole
+// boxes.  tm: T as (kx, y, slice) or, grouped, (kx, y, slice, item), 8-byte
+// elements, boxes of recon_a_two_box(n) kx x kTwoBoxY y, swizzled by the box's
+// row of kx.  Its CTAs per slice group over nx rows, and per SM.
+constexpr int kTwoBoxY = 256;
+bool recon_a_two(int n, int y0, int ny_out);
+int recon_a_two_box(int n);
+int recon_a_two_ctas_per_sm(int n);
+cudaError_t launch_recon_a_two(int n, const ReconA &b, const CUtensorMap &tm, int nbatch, cudaStream_t s);
+cudaError_t launch_recon_a_group_two(int n, const ReconAGrouped &b, const CUtensorMap &tm, cudaStream_t s);
 cudaError_t launch_recon_a_group(int n, const ReconAGrouped &b, cudaStream_t s);
-// The grouped form with the tensor-map store, at the lengths where
-// recon_a_tstore holds with one CTA per box (256 .. 2048); tm: the items' T
-// slots as (kx, y, slice, item), boxes of recon_a_tstore_box(n) kx x 256 y.
-bool recon_a_group_tstore(int n);
-cudaError_t launch_recon_a_group_tstore(int n, const ReconAGroupedTStore &b, const CUtensorMap &tm, cudaStream_t s);
 // The persistent GS passes with the tensor-map store (lengths where
 // gs_tstore_len holds; tm: dst as a 2-D tensor of 8-byte elements, inner
 // dimension the rows' index, boxes of rows-per-block x 256).
@@ -276,8 +277,7 @@ cudaError_t launch_gs_col_ts(int n, const GsColT &b, const CUtensorMap &tm, cuda
 cudaError_t launch_gs_row_ts(int n, const GsRowMidT &b, const CUtensorMap &tm, cudaStream_t s);
 cudaError_t launch_recon_b_group(int n, const ReconB<EPI_PROJ, true> &b, cudaStream_t s);
 int recon_a_rows(int n);   // rows per pass A CTA for transform length n
-bool recon_a_chain(int n, bool tstore = false);   // whether pass A at length n (in the tensor-map
-                                                  // store form) advances X by the product chain
+bool recon_a_chain(int n);   // whether the row engine's pass A at length n advances X by the product chain
 // Pass B at 256 .. 4096 runs the two-stage transform (ph_two_b.cuh): its CTAs
 // per slice group over `rows` rows, and per SM (0 at the other lengths).
 int recon_b_ctas(int n, int rows);

@@ -155,12 +155,12 @@ struct Plan {
 };
 
 // The factors of a thread's stage twiddles: W_N^(l (k1 + P k2)) = a[k1] b[k2].
-// H = 2: the transform is half h of one of length 2 N (the inputs of h = 1 still
-// lack the lane's factor W_2N^l, which goes into a).
+// H = 2: the transform is half h (the even or odd outputs) of one of length 2 N;
+// the inputs of h = 1 still lack the lane's factor W_2N^l, which goes into a.
 template <int N, bool INV, int H = 1>
 struct Factors {
     using PL = Plan<N>;
-    static constexpr int P0 = H > 1 ? 0 : 1;                  // the first factor that is not 1
+    static constexpr int P0 = H > 1 ? 0 : 1;          // the first factor that is not 1
     static constexpr int COUNT = PL::P - P0 + PL::Q - 1;
     static constexpr size_t BYTES = (size_t)COUNT * H * PL::L * 8;
     float2 a[PL::P], b[PL::Q];
@@ -183,9 +183,9 @@ struct Factors {
     // v times the twiddle of output k
     __device__ __forceinline__ float2 apply(int k, float2 v) const {
         const int p = k % PL::P, q = k / PL::P;
-        if (H == 1 && p == 0 && q == 0) return v;
+        if (P0 == 1 && p == 0 && q == 0) return v;
         if (q == 0) return cmul2(v, a[p]);
-        if (H == 1 && p == 0) return cmul2(v, b[q]);
+        if (P0 == 1 && p == 0) return cmul2(v, b[q]);
         return cmul2(v, cmul2(a[p], b[q]));
     }
 };
@@ -247,12 +247,25 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
         : "r"(taddr)
         : "memory");
 }
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[16]) {   // the first 8; the others are 0
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                 : "r"(taddr)
+                 : "memory");
+#pragma unroll
+    for (int i = 8; i < 16; ++i) v[i] = 0.0f;
+}
 // Waits for the loads issued so far; the values pass through it, so that no use moves above it.
 __device__ __forceinline__ void tmem_wait(float (&v)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;"
                  : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]),
                    "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]),
                    "+f"(v[15])::"memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const float2 (&v)[4]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};" ::"f"(v[0].x),
+                 "f"(v[0].y), "f"(v[1].x), "f"(v[1].y), "f"(v[2].x), "f"(v[2].y), "f"(v[3].x), "f"(v[3].y), "r"(taddr)
+                 : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 

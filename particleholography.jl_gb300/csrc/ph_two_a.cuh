@@ -1,0 +1,283 @@
+// ph_two_a.cuh -- reconstruction pass A on the two-stage row transform.
+#pragma once
+
+
+#include "ph_launch.cuh"
+#include "ph_two.cuh"
+
+namespace ph {
+namespace two {
+
+// X_k = X_0 Hdz^k, inverse FFT along ky, transposed tensor-map store of T.  A CTA
+// holds the RB rows kx of one box; a row belongs to one warp (two rows per warp
+// at 256 and 512, two warps per row at 4096), so that the exchange needs no CTA
+// barrier.  X_k and Hdz of a thread's values live in tensor memory (4 E columns
+// of its own lane): every slice reads both and writes back X_{k+1} = X_k Hdz.  X
+// is formed anew from the spectrum state at every multiple of CHAIN slices, which
+// keeps the chain's rounding at the transform's own: CHAIN = 8, and 16 with 64
+// values per thread, where forming X costs more (2048^2 x 256: 2.21 ms, 2.30 at 8).
+//
+// In the row engine this pass moved 87 bytes per voxel through the shared-memory
+// data path (chain 24, two exchanges 32, staging 16, twiddles 15); here 32 to 40.
+// Per launch, before and now: 1024^2 x 256 0.68 and 0.48 ms, 2048^2 x 512 5.43
+// and 4.55 ms, 4096^2 x 128 9.3 and 5.06 ms (no more clusters).  What is left:
+// arithmetic and its latency (50 % of the FP32 pipe, 45 to 54 % of issue slots),
+// then the stores: without them 0.46 ms at 1024.
+//
+// Boxes of 8 kx (64 bytes): of 4 kx at 1024, 0.77 ms (32-byte pieces of lines
+// that other CTAs complete); of 16 kx, 0.60 ms (one CTA per SM).  4096 keeps 4:
+// a box's rows have to fit the CTA.  The stores evict T first, since the next
+// pass reads it long after: 0.56 -> 0.49 ms at 1024, 2.29 -> 2.21 ms at 2048^2 x
+// 256.  Measured slower at 2048: 2 x 1024 with 32 values per thread (2.57 ms);
+// two groups of tensor-memory columns per wait.
+template <int N>
+struct PassA {
+    using PL = Plan<N>;
+    using F = Factors<N, true>;
+    static constexpr int RB = N <= 2048 ? 8 : 4;             // rows kx per CTA: one box
+    static constexpr int THREADS = RB * PL::L;
+    static constexpr int CTAS = (PL::E == 64 ? 256 : 512) / THREADS;
+    static constexpr uint32_t WCOLS = 4 * PL::E;             // tensor-memory columns of a warp
+    static constexpr uint32_t COLS = WCOLS * (THREADS / 128);
+    static constexpr size_t STAGE = (size_t)RB * N * 8;
+    static constexpr size_t XB = (size_t)PL::XWORDS * 4;
+    static constexpr size_t SMEM = STAGE + RB * XB + F::BYTES + 24;
+    static constexpr int BOX_Y = kTwoBoxY;
+    static constexpr uint32_t CHAIN = PL::E == 64 ? 16 : 8;   // slices between two formations of X
+};
+
+// Byte offset of (y, row r) in the staging [y][RB], with the tensor map's
+// swizzle (16-byte chunks exchanged by the address bits above 128 bytes): lanes
+// of consecutive y are RB x 8 bytes apart, and would meet in 4 (2) banks.  The
+// exchange has a period of 1024 bytes, so a multiple of that may be added after.
+template <int RB>
+__device__ __forceinline__ uint32_t stage_offset(int y, int r) {
+    const uint32_t a = (uint32_t)(y * RB + r) * 8;
+    return a ^ ((a >> 3) & (RB == 16 ? 0x70u : RB == 8 ? 0x30u : 0x10u));
+}
+
+template <int N, bool GROUPED>
+__global__ void __launch_bounds__(PassA<N>::THREADS, PassA<N>::CTAS)
+    k_two_a(const ReconAT<GROUPED> p, const __grid_constant__ CUtensorMap tmap) {
+    using C = PassA<N>;
+    using PL = typename C::PL;
+    constexpr int E = PL::E, L = PL::L, RB = C::RB, P = PL::P, Q = PL::Q;
+    extern __shared__ __align__(1024) unsigned char ph_smem[];
+    unsigned char *stage = ph_smem;
+    float2 *tab = reinterpret_cast<float2 *>(ph_smem + C::STAGE + RB * C::XB);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(reinterpret_cast<unsigned char *>(tab) + C::F::BYTES);
+    uint32_t *slot = reinterpret_cast<uint32_t *>(bar + 1);
+
+    // Launch order: two slice groups at a time, the groups of one row block
+    // consecutive, so that they share its state rows in L2 and neighbouring row
+    // blocks write the neighbouring pieces of T's rows together (2048^2 x 512: 4.55
+    // ms; all 8 groups at a time 4.77, one 4.73).
+    constexpr int AT_ONCE = 2;
+    const int lin = blockIdx.y * gridDim.x + blockIdx.x;
+    const int chunk = lin / (AT_ONCE * (int)gridDim.x), at = lin % (AT_ONCE * (int)gridDim.x);
+    const int wide = min(AT_ONCE, (int)gridDim.y - chunk * AT_ONCE);
+    const int g = chunk * AT_ONCE + at % wide, kx0 = at / wide * RB;
+    int group = p.group, b1max = p.nbatch;
+    const float4 *state = p.state;
+    if constexpr (GROUPED) {
+        const int z = (int)blockIdx.z;
+        group = p.item_group(z);
+        b1max = p.item_nb(z);
+        state += (size_t)z * p.item_state_stride;
+    }
+    const int b0 = g * group, b1 = min(b0 + group, b1max);
+    if (b0 >= b1) return;
+
+    const int warp = threadIdx.x >> 5;
+    const int r = threadIdx.x / L, l = threadIdx.x % L;
+    if (warp == 0) tc::tmem_alloc(slot, C::COLS);
+    C::F::fill(tab, p.tw);
+    if (threadIdx.x == 0) {
+        mbar_init(bar, 1);
+        mbar_fence_init();
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    // columns of this warp; group n2 of the first butterflies: X of its P inputs, then Hdz of them
+    const uint32_t tm = *slot + ((uint32_t)(warp & 3) << 21) + (uint32_t)(warp >> 2) * C::WCOLS;
+    // (rows beyond nx transform row nx - 1 again; the tensor map drops their columns)
+    const float4 *srow = state + (size_t)min(kx0 + r, p.nx - 1) * N;
+    float *ex = reinterpret_cast<float *>(ph_smem + C::STAGE + r * C::XB);
+    const auto sync = [&] {
+        if constexpr (L <= 32) __syncwarp();
+        else named_bar_sync(2 + r, L);
+    };
+
+    // f(i) over a group's inputs i = Q n1 + n2 -> tensor-memory columns at `at`
+    const auto put = [&](uint32_t at, const float2 (&t)[P]) {
+        if constexpr (P == 4) {
+            tmem_st8(at, t);
+        } else {
+            float q[16];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { q[2 * i] = t[i].x; q[2 * i + 1] = t[i].y; }
+            tmem_st16(at, q);
+        }
+    };
+    const auto get = [&](uint32_t at, float2 (&t)[P]) {
+        float q[16];
+        if constexpr (P == 4) tmem_ld8(at, q);
+        else tmem_ld16(at, q);
+        tmem_wait(q);
+#pragma unroll
+        for (int i = 0; i < P; ++i) t[i] = make_float2(q[2 * i], q[2 * i + 1]);
+    };
+#pragma unroll 1
+    for (int n2 = 0; n2 < Q; ++n2) {   // Hdz: the accurate sin/cos, as its error grows along the chain
+        float2 t[P];
+#pragma unroll
+        for (int n1 = 0; n1 < P; ++n1) {
+            const float4 st = srow[l + L * (Q * n1 + n2)];
+            float sn, cs;
+            sincospif((float)(int32_t)__float_as_uint(st.z) * 4.656612873077392578125e-10f, &sn, &cs);
+            const float mag = exp2f(st.w);
+            t[n1] = make_float2(cs * mag, sn * mag);
+        }
+        put(tm + n2 * 4 * P + 2 * P, t);
+    }
+
+    const uint64_t policy = l2_evict_first();   // T is read by the next pass, long after
+    for (int b = b0; b < b1; ++b) {
+        tmem_wait_st();
+        const uint32_t k = (uint32_t)(p.k0 + b), ahead = k % C::CHAIN;
+        if (ahead == 0 || b == b0) {
+            // X at the last multiple of CHAIN, then the chain's own products: X_k does
+            // not depend on where a group or a range of slices starts
+            float4 st[P];
+            const auto read = [&](int n2) {
+#pragma unroll
+                for (int n1 = 0; n1 < P; ++n1) st[n1] = srow[l + L * (Q * n1 + n2)];
+            };
+            read(0);
+#pragma unroll 1
+            for (int n2 = 0; n2 < Q; ++n2) {
+                float4 cur[P];
+#pragma unroll
+                for (int n1 = 0; n1 < P; ++n1) cur[n1] = st[n1];
+                if (n2 + 1 < Q) read(n2 + 1);   // the next group's state is on its way
+                float2 t[P];
+#pragma unroll
+                for (int n1 = 0; n1 < P; ++n1) t[n1] = ReconAT<GROUPED>::direct(cur[n1], k - ahead);
+                if (ahead != 0) {
+                    float2 hd[P];
+                    get(tm + n2 * 4 * P + 2 * P, hd);
+#pragma unroll 1
+                    for (uint32_t i = 0; i < ahead; ++i)
+#pragma unroll
+                        for (int n1 = 0; n1 < P; ++n1) t[n1] = cmul2(t[n1], hd[n1]);
+                }
+                put(tm + n2 * 4 * P, t);
+            }
+            tmem_wait_st();
+        }
+        float2 v[E];
+        {
+            float2 w[E];
+            constexpr int V = P / 4;    // loads of 16 columns per group
+            float x[2][V][16];          // X and Hdz of two groups: the next is on its way while one is used
+            const auto fetch = [&](int n2) {
+#pragma unroll
+                for (int i = 0; i < V; ++i) tmem_ld16(tm + n2 * 4 * P + 16 * i, x[n2 & 1][i]);
+            };
+            fetch(0);
+            static_for<Q>([&](auto N2) {
+                constexpr int n2 = decltype(N2)::value, H0 = P == 4 ? 8 : 0;   // P = 8: Hdz in the second 16
+                auto &xx = x[n2 & 1];
+#pragma unroll
+                for (int i = 0; i < V; ++i) tmem_wait(xx[i]);
+                if constexpr (n2 + 1 < Q) fetch(n2 + 1);
+                float2 t[P], next[P];
+#pragma unroll
+                for (int n1 = 0; n1 < P; ++n1) {
+                    t[n1] = make_float2(xx[0][2 * n1], xx[0][2 * n1 + 1]);
+                    next[n1] = cmul2(t[n1], make_float2(xx[V - 1][H0 + 2 * n1], xx[V - 1][H0 + 2 * n1 + 1]));
+                }
+                put(tm + n2 * 4 * P, next);
+                bfly<P, true>(t);
+                static_for<P>([&](auto K1) {
+                    constexpr int k1 = decltype(K1)::value;
+                    w[P * n2 + k1] = ctw<n2 * k1, E, true>(t[k1]);
+                });
+            });
+            typename C::F f;
+            f.load(opaque(tab), l);
+            level2<E, true>(w, [&](int o, float2 y) { v[o] = f.apply(o, y); });
+        }
+        sync();   // every thread has read the previous exchange
+        exchange<N>(v, ex + l, ex + l * PL::PITCH, sync);
+        float2 u[E];   // u[m L + o] = value of y = l + L m + E o
+#pragma unroll
+        for (int m = 0; m < PL::M; ++m) {
+            float2 w[L];
+            level1<L, true>(w, [&](int i) { return v[m * L + i]; });
+            level2<L, true>(w, [&](int o, float2 y) { u[m * L + o] = y; });
+        }
+        // the previous slice's boxes have left the staging
+        if (threadIdx.x == 0) {
+            bulk_wait_read_all();
+            mbar_arrive(bar);
+        }
+        mbar_wait(bar, (uint32_t)(b - b0) & 1u, p.err);
+        unsigned char *out = stage + stage_offset<RB>(l, r);
+#pragma unroll
+        for (int m = 0; m < PL::M; ++m)
+#pragma unroll
+            for (int o = 0; o < L; ++o) {
+                const int dy = L * m + E * o;
+                static_assert(L * RB * 8 % 1024 == 0 && E * RB * 8 % 1024 == 0, "whole periods of the swizzle");
+                *reinterpret_cast<float2 *>(out + dy * RB * 8) = u[m * L + o];
+            }
+        fence_proxy_async_smem();
+        if (warp == 0) {
+            named_bar_sync(1, C::THREADS);
+            if (threadIdx.x == 0) {
+#pragma unroll 1
+                for (int q = 0; q < N / C::BOX_Y; ++q) {
+                    const unsigned char *box = stage + (size_t)q * C::BOX_Y * RB * 8;
+                    const int yo = q * C::BOX_Y - p.y0;   // (a cropped frame: whole boxes inside it)
+                    if (yo < 0 || yo >= p.ny_out) continue;
+                    if constexpr (GROUPED) tma_store_4d(&tmap, box, kx0, yo, b, (int)blockIdx.z, policy);
+                    else tma_store_3d(&tmap, box, kx0, yo, b, policy);
+                }
+                bulk_commit();
+            }
+        } else {
+            named_bar_arrive(1, C::THREADS);
+        }
+    }
+    if (threadIdx.x == 0) bulk_wait_all();   // the shared memory outlives the last boxes' reads
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    if (warp == 0) tc::tmem_dealloc(*slot, C::COLS);
+}
+
+template <int N, bool GROUPED>
+cudaError_t launch_a(const ReconAT<GROUPED> &p, const CUtensorMap &tm, int groups, int items, cudaStream_t s) {
+    using C = PassA<N>;
+    static_assert(C::SMEM + 1024 <= 228 * 1024 / C::CTAS, "the CTAs of an SM share its shared memory");
+    static_assert(C::COLS * C::CTAS <= 512, "and its tensor memory");
+    auto kern = k_two_a<N, GROUPED>;
+    static unsigned long long done_mask = 0;   // per-device opt-in to more than 48 KB of dynamic shared memory
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const unsigned long long bit = 1ull << (dev & 63);
+    if (!(__atomic_load_n(&done_mask, __ATOMIC_ACQUIRE) & bit)) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+        if (e != cudaSuccess) return e;
+        __atomic_fetch_or(&done_mask, bit, __ATOMIC_ACQ_REL);
+    }
+    const int gx = (p.nx + C::RB - 1) / C::RB;
+    if (gx == 0 || groups == 0) return cudaSuccess;
+    kern<<<dim3(gx, groups, items), C::THREADS, C::SMEM, s>>>(p, tm);
+    return cudaGetLastError();
+}
+
+}  // namespace two
+}  // namespace ph

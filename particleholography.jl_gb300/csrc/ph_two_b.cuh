@@ -18,10 +18,10 @@ namespace two {
 // 2048 = 2 x 1024: one warp transforms x[n] + x[n + 1024] (the even outputs),
 // the other (x[n] - x[n + 1024]) W^n (the odd ones).  Each row is read twice (8
 // bytes per voxel more), but 32 values per thread leave room for 16 warps per
-// SM: 3.21 ms per 2048^2 x 512 launch, against 3.64 ms with 64 values per
+// SM: 3.19 ms per 2048^2 x 512 launch, against 3.64 ms with 64 values per
 // thread and 8 warps (latency: 54 % of issue slots), and 3.86 ms in the
-// three-stage row engine.  1024^2 x 256: 0.373 ms (0.483 in the engine; the
-// copy peak would take 0.316).  4096^2 x 128, 64 values: 3.86 ms (4.37).
+// three-stage row engine.  1024^2 x 256: 0.365 ms (0.483 in the engine; the
+// copy peak would take 0.316).  4096^2 x 128, 64 values: 3.82 ms (4.37).
 // Measured slower: the stage factors read from the W^i table (gathers of up to
 // 32 lines: 3.77 ms at 2048) or held in registers across slices (spills).
 template <int N, int EPI, bool GROUPED>
@@ -93,10 +93,11 @@ __global__ void __launch_bounds__(128, PassB<N, EPI, GROUPED>::CTAS) k_two_b(con
             if constexpr (C::TPR <= 32) __syncwarp();
             else named_bar_sync(1 + r, C::TPR);
         };
+        const uint64_t policy = l2_evict_first();   // T is read once
         const auto issue = [&](int b) {   // one thread per row: the row of slice b
             fence_proxy_async_smem();
             mbar_arrive_expect_tx(bars + r, N * 8);
-            bulk_g2s(in, t + ((size_t)b * p.rows + y) * N, N * 8, bars + r);
+            bulk_g2s(in, t + ((size_t)b * p.rows + y) * N, N * 8, bars + r, policy);
         };
         if (l == 0 && h == 0 && valid) issue(b0);
         if constexpr (C::MIN) {
