@@ -151,23 +151,108 @@ __device__ __forceinline__ double sqr_term(int i1, int n, double wavlen, double 
     return __dmul_rn(t, t);
 }
 
-__global__ void k_transfer_sqrt(float *out, int nx, int ny, double wavlen, double dx) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= nx || y >= ny) return;
-    const double v = __dsub_rn(__dsub_rn(1.0, sqr_term(x + 1, nx, wavlen, dx)), sqr_term(y + 1, ny, wavlen, dx));
-    out[(size_t)y * nx + x] = __double2float_rn(v);
+// GB300 runs FP64 at 1/64 of its FP32 rate: the terms of a row and a column are
+// formed once per 256 columns and kSqrtRows rows (four FP64 divisions per pixel
+// otherwise, the same values).
+constexpr int kSqrtRows = 16;
+__global__ void __launch_bounds__(256) k_transfer_sqrt(float *out, int nx, int ny, double wavlen, double dx) {
+    __shared__ double ty[kSqrtRows];
+    const int x = blockIdx.x * 256 + threadIdx.x;
+    const int y0 = blockIdx.y * kSqrtRows;
+    if (threadIdx.x < kSqrtRows) ty[threadIdx.x] = sqr_term(y0 + (int)threadIdx.x + 1, ny, wavlen, dx);
+    __syncthreads();
+    if (x >= nx) return;
+    const double a = __dsub_rn(1.0, sqr_term(x + 1, nx, wavlen, dx));
+    for (int y = y0; y < min(y0 + kSqrtRows, ny); ++y) out[(size_t)y * nx + x] = __double2float_rn(__dsub_rn(a, ty[y - y0]));
+}
+cudaError_t transfer_sqrt_launch(float *out, int nx, int ny, double wavlen, double dx, cudaStream_t s) {
+    k_transfer_sqrt<<<dim3((nx + 255) / 256, (ny + kSqrtRows - 1) / kSqrtRows), 256, 0, s>>>(out, nx, ny, wavlen, dx);
+    return cudaGetLastError();
 }
 
-// holofunc.jl:38-45: exp(i * c * sqrt(Float32 d)), c = 2 pi z0 / lambda (FP64).
-__global__ void k_transfer(float2 *out, const float *d_sqr, size_t n, double c) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float s = sqrtf(d_sqr[i]);
-    const double phase = __dmul_rn(c, (double)s);
+// holofunc.jl:38-45: exp(i c sqrt(Float32 d)), c = 2 pi z0 / lambda (FP64).
+//
+// In FP64 (sincos of the product) this was bound by the FP64 pipe: 0.22 ms at
+// 2048^2, where the memory takes 0.007.  Here the phase is a fixed-point fraction
+// of a turn: c / 2 pi as a 128-bit integer `a` (units of 2^-41 turn per 2^-23; the
+// host forms it in double-double), times the 24-bit mantissa of s = sqrt(d),
+// shifted by its exponent, modulo 2^64: exact to 2^-40 turn.  The nearest of 256
+// table angles, as FP32 pairs hi + lo, is rotated by the rest (below pi / 256) in
+// FP32 with short Taylor series, whose result enters as a correction below 0.013:
+// the sum is within 1e-9 of the exact value before its one rounding.
+// s outside [2^-30, 1], NaN: the FP64 form.
+struct TurnRate {
+    unsigned long long lo;
+    long long hi;
+    double c;
+    bool fixed;   // |c / 2 pi| < 2^40: the fixed-point form holds
+};
+TurnRate turn_rate(double c) {
+    const double inv_hi = 0x1.45f306dc9c883p-3, inv_lo = -0x1.6b01ec5417056p-57;   // 1 / (2 pi)
+    TurnRate r{0, 0, c, false};
+    const double qh = c * inv_hi;
+    if (!(fabs(qh) < 0x1p40)) return r;   // (NaN too)
+    const double ql = fma(c, inv_hi, -qh) + c * inv_lo;
+    const double ah = qh * 0x1p41, fl = floor(ah);
+    const __int128 a = (__int128)fl + (__int128)llrint((ah - fl) + ql * 0x1p41);
+    r.lo = (unsigned long long)a;
+    r.hi = (long long)(a >> 64);
+    r.fixed = true;
+    return r;
+}
+
+__device__ __noinline__ float2 transfer_value_fp64(float s, double c) {
     double sn, cs;
-    sincos(phase, &sn, &cs);
-    out[i] = make_float2(__double2float_rn(cs), __double2float_rn(sn));
+    sincos(__dmul_rn(c, (double)s), &sn, &cs);
+    return make_float2(__double2float_rn(cs), __double2float_rn(sn));
+}
+
+constexpr int kTurnTable = 256;
+__device__ __forceinline__ float2 transfer_value(float d, const TurnRate &a, const float4 *tab) {
+    const float s = sqrtf(d);
+    if (!(a.fixed && s >= 0x1p-30f && s <= 1.0f)) return transfer_value_fp64(s, a.c);
+    const uint32_t bits = __float_as_uint(s), m = (bits & 0x7fffffu) | 0x800000u, j = 127u - (bits >> 23);
+    const uint32_t w0 = (uint32_t)a.lo, w1 = (uint32_t)(a.lo >> 32), w2 = (uint32_t)a.hi;
+    const unsigned long long f =
+        ((unsigned long long)__funnelshift_r(w1, w2, j) << 32) | __funnelshift_r(w0, w1, j);
+    const unsigned long long p = f * m;                       // the phase, 2^64 per turn
+    const uint32_t i = (uint32_t)((p + (1ull << 55)) >> 56);  // nearest table angle
+    const int32_t rest = (int32_t)((long long)(p - ((unsigned long long)i << 56)) >> 24);
+    const float x = (float)rest * (6.28318530717958647692f * 0x1p-40f), x2 = x * x;
+    const float sn = fmaf(x * x2, fmaf(x2, 1.0f / 120.0f, -1.0f / 6.0f), x);
+    const float cs1 = x2 * fmaf(x2, 1.0f / 24.0f, -0.5f);     // cos - 1
+    const float4 w = tab[i & (kTurnTable - 1)];               // (cos hi, cos lo, sin hi, sin lo)
+    return make_float2(w.x + (w.y + fmaf(w.x, cs1, -w.z * sn)), w.z + (w.w + fmaf(w.z, cs1, w.x * sn)));
+}
+
+// VEC: four pixels per load (16-byte aligned arrays, n a multiple of 4).
+template <bool VEC>
+__global__ void __launch_bounds__(256)
+    k_transfer(float2 *out, const float *__restrict__ d_sqr, size_t n, const TurnRate a, const float4 *__restrict__ ptab) {
+    __shared__ float4 tab[kTurnTable];
+    tab[threadIdx.x] = __ldg(ptab + threadIdx.x * (kPhaseTable / kTurnTable));
+    __syncthreads();
+    const size_t step = (size_t)gridDim.x * 256, first = (size_t)blockIdx.x * 256 + threadIdx.x;
+    if constexpr (VEC) {
+        for (size_t i = first; i < n / 4; i += step) {
+            const float4 d = __ldg(reinterpret_cast<const float4 *>(d_sqr) + i);
+            const float2 v0 = transfer_value(d.x, a, tab), v1 = transfer_value(d.y, a, tab);
+            const float2 v2 = transfer_value(d.z, a, tab), v3 = transfer_value(d.w, a, tab);
+            reinterpret_cast<float4 *>(out)[2 * i] = make_float4(v0.x, v0.y, v1.x, v1.y);
+            reinterpret_cast<float4 *>(out)[2 * i + 1] = make_float4(v2.x, v2.y, v3.x, v3.y);
+        }
+    } else {
+        for (size_t i = first; i < n; i += step) out[i] = transfer_value(d_sqr[i], a, tab);
+    }
+}
+cudaError_t transfer_launch(float2 *out, const float *d_sqr, size_t n, double c, const float4 *ptab, cudaStream_t s) {
+    static_assert(kTurnTable == 256, "one table entry per thread");
+    const bool vec = n % 4 == 0 && (((uintptr_t)out | (uintptr_t)d_sqr) & 15) == 0;
+    const size_t work = vec ? n / 4 : n;
+    const unsigned g = (unsigned)std::min<size_t>((work + 255) / 256, 2048);
+    if (vec) k_transfer<true><<<g, 256, 0, s>>>(out, d_sqr, n, turn_rate(c), ptab);
+    else k_transfer<false><<<g, 256, 0, s>>>(out, d_sqr, n, turn_rate(c), ptab);
+    return cudaGetLastError();
 }
 
 // Exact physics: the square-root term in FP64, evanescent waves set to 0.
@@ -1191,11 +1276,10 @@ int serve_transfer(ph_server *srv, cudaStream_t ls, float *dsqr, int nx, int ny,
             cudaFree(e.buf);
             return cuda_status(ctx, cudaGetLastError(), "cudaEventCreate");
         }
-        dim3 b(32, 8);
-        k_transfer_sqrt<<<grid2d(nx, ny, b), b, 0, ls>>>(dsqr, nx, ny, wavlen, dx);
+        PH_TRY(launched(ctx, transfer_sqrt_launch(dsqr, nx, ny, wavlen, dx, ls), "serve transfer"));
         const size_t n = (size_t)nx * ny;
-        k_transfer<<<(unsigned)((n + 255) / 256), 256, 0, ls>>>(e.buf, dsqr, n, (2.0 * M_PI * (-z)) / wavlen);
-        PH_TRY(launched(ctx, cudaGetLastError(), "serve transfer", 2));
+        PH_TRY(launched(ctx, transfer_launch(e.buf, dsqr, n, (2.0 * M_PI * (-z)) / wavlen, ctx->phase_tab, ls),
+                        "serve transfer"));
         PH_CUDA(cudaEventRecord(e.ready, ls), "cudaEventRecord");
         it = srv->tfs.emplace(key, e).first;
     } else {
@@ -1489,9 +1573,7 @@ int32_t ph_transfer_sqrt(ph_ctx *ctx, float *out, int32_t n_fast, int32_t n_slow
     PH_ENTER(ctx, stream);
     PH_NONNULL(out, "out");
     if (n_fast <= 0 || n_slow <= 0) { set_err(ctx, "sizes must be positive"); return PH_ERR_SIZE; }
-    dim3 b(32, 8);
-    k_transfer_sqrt<<<grid2d(n_fast, n_slow, b), b, 0, s>>>(out, n_fast, n_slow, wavlen, dx);
-    PH_TRY(launched(ctx, cudaGetLastError(), "transfer_sqrt"));
+    PH_TRY(launched(ctx, transfer_sqrt_launch(out, n_fast, n_slow, wavlen, dx, s), "transfer_sqrt"));
     PH_LEAVE(ctx);
 }
 
@@ -1503,8 +1585,7 @@ int32_t ph_transfer(ph_ctx *ctx, void *out, const float *d_sqr, int32_t n_fast, 
     if (n_fast <= 0 || n_slow <= 0) { set_err(ctx, "sizes must be positive"); return PH_ERR_SIZE; }
     const size_t n = (size_t)n_fast * n_slow;
     const double c = (2.0 * M_PI * z0) / wavlen;
-    k_transfer<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(static_cast<float2 *>(out), d_sqr, n, c);
-    PH_TRY(launched(ctx, cudaGetLastError(), "transfer"));
+    PH_TRY(launched(ctx, transfer_launch(static_cast<float2 *>(out), d_sqr, n, c, ctx->phase_tab, s), "transfer"));
     PH_LEAVE(ctx);
 }
 
@@ -1693,8 +1774,7 @@ int32_t ph_asm_prop(ph_ctx *ctx, void *out, const void *in, const float *d_sqr, 
     PH_TRY(get_twiddles(ctx, ny, s, &tw_y));
     float2 *h = at<float2>(ctx, oh);
     const double c = (2.0 * M_PI * zprop) / wavlen;
-    k_transfer<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(h, d_sqr, n, c);
-    PH_TRY(launched(ctx, cudaGetLastError(), "transfer"));
+    PH_TRY(launched(ctx, transfer_launch(h, d_sqr, n, c, ctx->phase_tab, s), "transfer"));
     PH_TRY(issue_propagate(ctx, static_cast<float2 *>(out), static_cast<const float2 *>(in), h, nullptr, nx, ny,
                            at<float2>(ctx, oa), at<float2>(ctx, ob), tw_x, tw_y, s));
     PH_LEAVE(ctx);
@@ -1951,12 +2031,10 @@ int32_t ph_autotune(ph_ctx *ctx, int32_t n_fast, int32_t n_slow, int32_t slices,
         return cuda_status(ctx, cudaGetLastError(), "cudaMalloc(tuning outputs)");
     }
     float2 *wf = buf, *hf = buf + n, *hdz = buf + 2 * n;
-    dim3 b2(32, 8);
-    k_transfer_sqrt<<<grid2d(n_fast, n_slow, b2), b2, 0, s>>>(dsqr, n_fast, n_slow, 0.6328, 10.0);
-    k_transfer<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(wf, dsqr, n, (2.0 * M_PI * 3000.0) / 0.6328);
-    k_transfer<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(hf, dsqr, n, (2.0 * M_PI * -1000.0) / 0.6328);
-    k_transfer<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(hdz, dsqr, n, (2.0 * M_PI * -200.0) / 0.6328);
-    if (cudaGetLastError() != cudaSuccess) { cleanup(); return cuda_status(ctx, cudaErrorLaunchFailure, "tuning inputs"); }
+    if (transfer_sqrt_launch(dsqr, n_fast, n_slow, 0.6328, 10.0, s) != cudaSuccess ||
+        transfer_launch(wf, dsqr, n, (2.0 * M_PI * 3000.0) / 0.6328, ctx->phase_tab, s) != cudaSuccess ||
+        transfer_launch(hf, dsqr, n, (2.0 * M_PI * -1000.0) / 0.6328, ctx->phase_tab, s) != cudaSuccess ||
+        transfer_launch(hdz, dsqr, n, (2.0 * M_PI * -200.0) / 0.6328, ctx->phase_tab, s) != cudaSuccess) { cleanup(); return cuda_status(ctx, cudaErrorLaunchFailure, "tuning inputs"); }
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
