@@ -85,11 +85,16 @@ def cu_bounding_rectangles(labels: torch.Tensor) -> np.ndarray:
     ctx = _lib.default_context(dev)
     s = torch.cuda.current_stream(dev).cuda_stream
     count = ctypes.c_int64(0)
-    ctx.call("ph_ccl_boxes", None, 0, ctypes.byref(count), lab.data_ptr(), slices, rows, cols, s)
-    out = np.empty((max(count.value, 1), 5), dtype=np.int64)
-    ctx.call("ph_ccl_boxes", out.ctypes.data, int(count.value), ctypes.byref(count), lab.data_ptr(), slices, rows,
-             cols, s)
-    return out[:count.value]
+    room = _ROOM
+    while True:   # a second call only where there are more components than room
+        out = np.empty((room, 5), dtype=np.int64)
+        ctx.call("ph_ccl_boxes", out.ctypes.data, room, ctypes.byref(count), lab.data_ptr(), slices, rows, cols, s)
+        if count.value <= room:
+            return out[:count.value]
+        room = count.value
+
+
+_ROOM = 1 << 16   # components a query makes room for before it knows their number
 
 
 def _labels_on_device(labels) -> torch.Tensor:
@@ -120,6 +125,8 @@ def count_labels(labels) -> int:
 
 def cu_find_valid_labels(labels) -> np.ndarray:
     """ccl.jl:224-238: sorted 1-based root indices as a host Int64 vector."""
-    c, _ = _roots(labels, 0)
-    _, buf = _roots(labels, c)
+    labels = _labels_on_device(labels)
+    c, buf = _roots(labels, _ROOM)
+    if c > _ROOM:
+        c, buf = _roots(labels, c)
     return buf[:c]

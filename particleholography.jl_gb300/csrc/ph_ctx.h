@@ -56,6 +56,9 @@ struct ph_ctx {
     // small fixed device area: [0] loop-limit error flag (int), [8..) 4 doubles of accumulators
     void *small = nullptr;
 
+    // pinned host staging of the root and box queries (kPinnedBytes, made on first use)
+    void *pinned = nullptr;
+
     // stream ordering between calls on different streams
     cudaStream_t last_stream = nullptr;
     bool has_last = false;

@@ -25,7 +25,7 @@
 
 namespace ph {
 cudaError_t roots_count_launch(const uint32_t *lab, int64_t n, int64_t slice_n, unsigned *counts,
-                               unsigned long long *total, cudaStream_t s, int64_t *launches);
+                               unsigned long long *total, const int *flag, cudaStream_t s, int64_t *launches);
 int64_t roots_blocks(int64_t n);
 }  // namespace ph
 
@@ -87,6 +87,6 @@ extern "C" int32_t ph_ccl_count_noalloc(int64_t *count, const uint32_t *labels, 
     // nothing left over from an earlier call is read.
     int64_t launches = 0;
     const cudaError_t e = ph::roots_count_launch(labels, n, n, scratch, reinterpret_cast<unsigned long long *>(count),
-                                                 s, &launches);
+                                                 nullptr, s, &launches);
     return e == cudaSuccess ? PH_OK : fail(PH_ERR_CUDA, cudaGetErrorString(e));
 }
