@@ -1074,16 +1074,16 @@ int recon_group_b(int nbatch, int nx, int rows, int items, int group_a, int cap_
 }
 
 // Tensor map of the slice intermediate T = [nb][ny_out][nx] float2 (8-byte
-// elements) for pass A's tiled store: boxes of box_kx kx x 256 y x 1 slice.
-bool t_store_map(CUtensorMap *tm, float2 *t, int nx, int ny_out, int nb, int box_kx) {
+// elements) for pass A's tiled store: boxes of box_kx kx x box_y y x 1 slice.
+bool t_store_map(CUtensorMap *tm, float2 *t, int nx, int ny_out, int nb, int box_kx, int box_y) {
     const EncodeTiledFn enc = encode_tiled();
-    if (enc == nullptr || ((uintptr_t)t & 15) != 0 || nx % 4 != 0 || (box_kx != 4 && box_kx != 8 && box_kx != 16)) return false;
+    if (enc == nullptr || ((uintptr_t)t & 15) != 0 || nx % 4 != 0 || (box_kx != 4 && box_kx != 8)) return false;
     const cuuint64_t dims[3] = {(cuuint64_t)nx, (cuuint64_t)ny_out, (cuuint64_t)nb};
     const cuuint64_t strides[2] = {(cuuint64_t)nx * 8, (cuuint64_t)nx * ny_out * 8};
-    const cuuint32_t box[3] = {(cuuint32_t)box_kx, (cuuint32_t)kTwoBoxY, 1};
+    const cuuint32_t box[3] = {(cuuint32_t)box_kx, (cuuint32_t)box_y, 1};
     const cuuint32_t estr[3] = {1, 1, 1};
     return enc(tm, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, t, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               box_kx == 16 ? CU_TENSOR_MAP_SWIZZLE_128B : box_kx == 8 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+               box_kx == 8 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -1102,19 +1102,19 @@ bool gs_store_map(CUtensorMap *tm, float2 *p, int inner, int outer, int rows) {
 }
 
 // Tensor map of the T slots of a grouped launch: item i's T = [nb][ny][nx]
-// float2 at t + i * item_bytes; boxes of box_kx kx x 256 y x 1 slice x 1 item.
+// float2 at t + i * item_bytes; boxes of box_kx kx x box_y y x 1 slice x 1 item.
 bool t_store_map_items(CUtensorMap *tm, float2 *t, int nx, int ny, int nb, int nitems, size_t item_bytes,
-                       int box_kx) {
+                       int box_kx, int box_y) {
     const EncodeTiledFn enc = encode_tiled();
-    if (enc == nullptr || ((uintptr_t)t & 15) != 0 || nx % 4 != 0 || (box_kx != 4 && box_kx != 8 && box_kx != 16) ||
+    if (enc == nullptr || ((uintptr_t)t & 15) != 0 || nx % 4 != 0 || (box_kx != 4 && box_kx != 8) ||
         item_bytes % 16 != 0)
         return false;
     const cuuint64_t dims[4] = {(cuuint64_t)nx, (cuuint64_t)ny, (cuuint64_t)nb, (cuuint64_t)nitems};
     const cuuint64_t strides[3] = {(cuuint64_t)nx * 8, (cuuint64_t)nx * ny * 8, (cuuint64_t)item_bytes};
-    const cuuint32_t box[4] = {(cuuint32_t)box_kx, (cuuint32_t)kTwoBoxY, 1, 1};
+    const cuuint32_t box[4] = {(cuuint32_t)box_kx, (cuuint32_t)box_y, 1, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     return enc(tm, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4, t, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               box_kx == 16 ? CU_TENSOR_MAP_SWIZZLE_128B : box_kx == 8 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+               box_kx == 8 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -1137,7 +1137,7 @@ int issue_recon_slices(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin
         a.k0 = k0; a.nbatch = nb; a.group = group;
         a.err = static_cast<int *>(ctx->small);
         CUtensorMap tm;
-        if (recon_a_two(ny, y0, ny_out) && t_store_map(&tm, t, nx, ny_out, nb, recon_a_two_box(ny))) {
+        if (recon_a_two(ny, y0, ny_out) && t_store_map(&tm, t, nx, ny_out, nb, recon_a_two_box(ny), recon_a_two_box_y(ny))) {
             PH_TRY(pass(ctx, s, "recon_a", [&] { return launch_recon_a_two(ny, a, tm, nb, s); }));
         } else {
             PH_TRY(pass(ctx, s, "recon_a", [&] { return launch_recon_a(ny, a, nb, s); }));
@@ -1383,7 +1383,7 @@ int issue_recon_group(ph_ctx *ctx, const std::vector<const ph_recon_item *> &its
         a.nitems = G;
         a.err = static_cast<int *>(ctx->small);
         CUtensorMap tm;
-        if (recon_a_two(ny, 0, ny) && t_store_map_items(&tm, a.t, nx, ny, L.batch, G, ib, recon_a_two_box(ny))) {
+        if (recon_a_two(ny, 0, ny) && t_store_map_items(&tm, a.t, nx, ny, L.batch, G, ib, recon_a_two_box(ny), recon_a_two_box_y(ny))) {
             PH_TRY(pass(ctx, s, "recon_a", [&] { return launch_recon_a_group_two(ny, a, tm, s); }));
         } else {
             PH_TRY(pass(ctx, s, "recon_a", [&] { return launch_recon_a_group(ny, a, s); }));

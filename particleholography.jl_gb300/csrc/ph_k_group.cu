@@ -15,11 +15,9 @@ cudaError_t launch_recon_b_group(int n, const ReconB<EPI_PROJ, true> &b, cudaStr
     int gy = 1;
     for (int i = 0; i < b.nitems; ++i) gy = std::max(gy, (b.item_nb(i) + b.item_group(i) - 1) / b.item_group(i));
     switch (n) {
-        case 256: return two::launch_b<256>(b, gy, b.nitems, s);
-        case 512: return two::launch_b<512>(b, gy, b.nitems, s);
-        case 1024: return two::launch_b<1024>(b, gy, b.nitems, s);
-        case 2048: return two::launch_b<2048>(b, gy, b.nitems, s);
-        case 4096: return two::launch_b<4096>(b, gy, b.nitems, s);
+#define PH_TWO_CASE(N) case N: return two::launch_b<N>(b, gy, b.nitems, s);
+        PH_FOR_EACH_N_TWO(PH_TWO_CASE)
+#undef PH_TWO_CASE
     }
     return launch_engine_len<false>(n, b, b.rows, gy, s, b.nitems);
 }

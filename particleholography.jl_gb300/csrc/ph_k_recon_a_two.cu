@@ -1,25 +1,27 @@
-// Reconstruction pass A on the two-stage transform (lengths 256 .. 4096).
+// Reconstruction pass A on the two-stage transform (lengths 192 .. 4096).
 #include "ph_two_a.cuh"
 
 namespace ph {
 
 bool recon_a_two(int n, int y0, int ny_out) {
-    return two::supported(n) && y0 % kTwoBoxY == 0 && ny_out % kTwoBoxY == 0;
+    return two::supported(n) && y0 % two::box_y(n) == 0 && ny_out % two::box_y(n) == 0;
 }
 
 int recon_a_two_box(int n) {
     switch (n) {
 #define PH_BOX_A(N) case N: return two::PassA<N>::RB;
-        PH_BOX_A(256) PH_BOX_A(512) PH_BOX_A(1024) PH_BOX_A(2048) PH_BOX_A(4096)
+        PH_FOR_EACH_N_TWO(PH_BOX_A)
 #undef PH_BOX_A
     }
     return 0;
 }
 
+int recon_a_two_box_y(int n) { return two::box_y(n); }
+
 int recon_a_two_ctas_per_sm(int n) {
     switch (n) {
 #define PH_PER_SM_A(N) case N: return two::PassA<N>::CTAS;
-        PH_PER_SM_A(256) PH_PER_SM_A(512) PH_PER_SM_A(1024) PH_PER_SM_A(2048) PH_PER_SM_A(4096)
+        PH_FOR_EACH_N_TWO(PH_PER_SM_A)
 #undef PH_PER_SM_A
     }
     return 0;
@@ -28,11 +30,9 @@ int recon_a_two_ctas_per_sm(int n) {
 cudaError_t launch_recon_a_two(int n, const ReconA &b, const CUtensorMap &tm, int nbatch, cudaStream_t s) {
     const int gy = (nbatch + b.group - 1) / b.group;
     switch (n) {
-        case 256: return two::launch_a<256>(b, tm, gy, 1, s);
-        case 512: return two::launch_a<512>(b, tm, gy, 1, s);
-        case 1024: return two::launch_a<1024>(b, tm, gy, 1, s);
-        case 2048: return two::launch_a<2048>(b, tm, gy, 1, s);
-        case 4096: return two::launch_a<4096>(b, tm, gy, 1, s);
+#define PH_TWO_CASE(N) case N: return two::launch_a<N>(b, tm, gy, 1, s);
+        PH_FOR_EACH_N_TWO(PH_TWO_CASE)
+#undef PH_TWO_CASE
     }
     return cudaErrorInvalidValue;
 }
@@ -41,11 +41,9 @@ cudaError_t launch_recon_a_group_two(int n, const ReconAGrouped &b, const CUtens
     int gy = 1;
     for (int i = 0; i < b.nitems; ++i) gy = std::max(gy, (b.item_nb(i) + b.item_group(i) - 1) / b.item_group(i));
     switch (n) {
-        case 256: return two::launch_a<256>(b, tm, gy, b.nitems, s);
-        case 512: return two::launch_a<512>(b, tm, gy, b.nitems, s);
-        case 1024: return two::launch_a<1024>(b, tm, gy, b.nitems, s);
-        case 2048: return two::launch_a<2048>(b, tm, gy, b.nitems, s);
-        case 4096: return two::launch_a<4096>(b, tm, gy, b.nitems, s);
+#define PH_TWO_CASE(N) case N: return two::launch_a<N>(b, tm, gy, b.nitems, s);
+        PH_FOR_EACH_N_TWO(PH_TWO_CASE)
+#undef PH_TWO_CASE
     }
     return cudaErrorInvalidValue;
 }

@@ -6,11 +6,9 @@ namespace ph {
 cudaError_t launch_recon_b(int n, const ReconB<EPI_SUB> &b, cudaStream_t s) {
     const int groups = (b.nbatch + b.group - 1) / b.group;
     switch (n) {
-        case 256: return two::launch_b<256>(b, groups, 1, s);
-        case 512: return two::launch_b<512>(b, groups, 1, s);
-        case 1024: return two::launch_b<1024>(b, groups, 1, s);
-        case 2048: return two::launch_b<2048>(b, groups, 1, s);
-        case 4096: return two::launch_b<4096>(b, groups, 1, s);
+#define PH_TWO_CASE(N) case N: return two::launch_b<N>(b, groups, 1, s);
+        PH_FOR_EACH_N_TWO(PH_TWO_CASE)
+#undef PH_TWO_CASE
     }
     return launch_engine_len<false>(n, b, b.rows, groups, s);
 }

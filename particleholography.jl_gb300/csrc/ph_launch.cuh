@@ -13,11 +13,10 @@ namespace ph {
     X(1) X(2) X(4) X(8) X(16) X(32) X(64) X(128) X(256) X(512) X(1024) X(2048) X(4096) X(8192) X(3) X(6) \
         X(12) X(24) X(48) X(96) X(192) X(384) X(768) X(1536) X(3072) X(6144)
 
-// The lengths whose pass B runs the row engine of ph_fft.cuh (256 .. 4096 run
-// the two-stage transform of ph_two.cuh).
-#define PH_FOR_EACH_N_ENGINE(X)                                                                          \
-    X(1) X(2) X(4) X(8) X(16) X(32) X(64) X(128) X(8192) X(3) X(6) X(12) X(24) X(48) X(96) X(192) X(384) \
-        X(768) X(1536) X(3072) X(6144)
+// The lengths whose pass B runs the row engine of ph_fft.cuh (the others run the
+// two-stage transform of ph_two.cuh).
+#define PH_FOR_EACH_N_ENGINE(X) \
+    X(1) X(2) X(4) X(8) X(16) X(32) X(64) X(128) X(8192) X(3) X(6) X(12) X(24) X(48) X(96) X(6144)
 
 inline bool supported_len(int n) {
     if (n < 1) return false;
@@ -257,13 +256,13 @@ cudaError_t launch_spectrum_staged(int n, const SpectrumColsT &b, const CUtensor
                                    cudaStream_t s);
 cudaError_t launch_recon_a(int n, const ReconA &b, int nbatch, cudaStream_t s);
 // Pass A on the two-stage transform with the tensor-map store (ph_two_a.cuh):
-// lengths 256 .. 4096, frames whose stored rows [y0, y0 + ny_out) are whole
+// lengths 192 .. 4096, frames whose stored rows [y0, y0 + ny_out) are whole
 // boxes.  tm: T as (kx, y, slice) or, grouped, (kx, y, slice, item), 8-byte
-// elements, boxes of recon_a_two_box(n) kx x kTwoBoxY y, swizzled by the box's
-// row of kx.  Its CTAs per slice group over nx rows, and per SM.
-constexpr int kTwoBoxY = 256;
+// elements, boxes of recon_a_two_box(n) kx x recon_a_two_box_y(n) y, swizzled by
+// the box's row of kx.  Its CTAs per SM.
 bool recon_a_two(int n, int y0, int ny_out);
 int recon_a_two_box(int n);
+int recon_a_two_box_y(int n);
 int recon_a_two_ctas_per_sm(int n);
 cudaError_t launch_recon_a_two(int n, const ReconA &b, const CUtensorMap &tm, int nbatch, cudaStream_t s);
 cudaError_t launch_recon_a_group_two(int n, const ReconAGrouped &b, const CUtensorMap &tm, cudaStream_t s);
@@ -278,7 +277,7 @@ cudaError_t launch_gs_row_ts(int n, const GsRowMidT &b, const CUtensorMap &tm, c
 cudaError_t launch_recon_b_group(int n, const ReconB<EPI_PROJ, true> &b, cudaStream_t s);
 int recon_a_rows(int n);   // rows per pass A CTA for transform length n
 bool recon_a_chain(int n);   // whether the row engine's pass A at length n advances X by the product chain
-// Pass B at 256 .. 4096 runs the two-stage transform (ph_two_b.cuh): its CTAs
+// Pass B at 192 .. 4096 runs the two-stage transform (ph_two_b.cuh): its CTAs
 // per slice group over `rows` rows, and per SM (0 at the other lengths).
 int recon_b_ctas(int n, int rows);
 int recon_b_ctas_per_sm(int n);

@@ -87,15 +87,38 @@ __device__ __forceinline__ void d8(float2 (&v)[8]) {
     v[7] = fma2s(h, t3, e3);
 }
 
+template <bool INV>
+__device__ __forceinline__ void d3(float2 &a, float2 &b, float2 &c) {
+    constexpr float h = 0.86602540378443864676f;   // sqrt(3) / 2
+    const float2 s = add2(b, c), d = sub2(b, c), m = fma2s(-0.5f, s, a);
+    a = add2(a, s);
+    const float2 p = make_float2(fmaf(-h, d.y, m.x), fmaf(h, d.x, m.y));   // m + i h d
+    const float2 q = make_float2(fmaf(h, d.y, m.x), fmaf(-h, d.x, m.y));   // m - i h d
+    b = INV ? p : q;
+    c = INV ? q : p;
+}
+template <bool INV>
+__device__ __forceinline__ void d6(float2 (&v)[6]) {   // n = 3 n1 + n2, k = k1 + 2 k2
+    float2 e0 = add2(v[0], v[3]), e1 = add2(v[1], v[4]), e2 = add2(v[2], v[5]);
+    float2 o0 = sub2(v[0], v[3]), o1 = ctw<1, 6, INV>(sub2(v[1], v[4])), o2 = ctw<2, 6, INV>(sub2(v[2], v[5]));
+    d3<INV>(e0, e1, e2);
+    d3<INV>(o0, o1, o2);
+    v[0] = e0; v[2] = e1; v[4] = e2;
+    v[1] = o0; v[3] = o1; v[5] = o2;
+}
+
 template <int R, bool INV>
 __device__ __forceinline__ void bfly(float2 (&v)[R]) {
-    if constexpr (R == 4) d4<INV>(v[0], v[1], v[2], v[3]);
+    static_assert(R == 3 || R == 4 || R == 6 || R == 8, "a butterfly of this size");
+    if constexpr (R == 3) d3<INV>(v[0], v[1], v[2]);
+    else if constexpr (R == 4) d4<INV>(v[0], v[1], v[2], v[3]);
+    else if constexpr (R == 6) d6<INV>(v);
     else d8<INV>(v);
 }
 
 // R = P Q: n = Q n1 + n2, k = k1 + P k2.
 template <int R>
-constexpr int split_p() { return R == 64 ? 8 : 4; }
+constexpr int split_p() { return R == 64 || R % 24 == 0 ? 8 : 4; }
 template <int R>
 constexpr int split_q() { return R / split_p<R>(); }
 
@@ -138,19 +161,29 @@ __device__ __forceinline__ void level2(const float2 (&y)[R], Out &&out) {
 
 // ---------------------------------------------------------------- shape
 
-// Values per thread and threads per row of length N.
-__host__ __device__ constexpr int values(int n) { return n <= 256 ? 16 : n <= 1024 ? 32 : 64; }
+// The lengths that have a two-stage transform.
+#define PH_FOR_EACH_N_TWO(X) X(192) X(256) X(384) X(512) X(768) X(1024) X(1536) X(2048) X(3072) X(4096)
+
+// Values per thread, threads per row, and transforms of length L per thread in
+// stage 2.  At 3 * 2^a lengths the last of these (all, where M = 1) has only the
+// threads t < E - (M - 1) L: the others compute on whatever follows the row's
+// exchange region (within the CTA's shared memory) and drop it.
+__host__ __device__ constexpr int values(int n) {
+    return n % 3 == 0 ? (n <= 192 ? 12 : n <= 768 ? 24 : 48) : n <= 256 ? 16 : n <= 1024 ? 32 : 64;
+}
 __host__ __device__ constexpr bool supported(int n) {
-    return n == 256 || n == 512 || n == 1024 || n == 2048 || n == 4096;
+    return n == 192 || n == 256 || n == 384 || n == 512 || n == 768 || n == 1024 || n == 1536 || n == 2048 ||
+           n == 3072 || n == 4096;
 }
 
 template <int N>
 struct Plan {
-    static constexpr int E = values(N), L = N / E, M = E / L;
-    static_assert(M * L == E && L >= 16 && L <= 64, "E a multiple of L");
+    static constexpr int E = values(N), L = N / E, M = (E + L - 1) / L;
+    static_assert(L == 16 || L == 32 || L == 64, "a row is half a warp, a warp or two");
     static constexpr int PITCH = L + 4;                      // words between the exchange rows of k1, k1 + 1
     // words of a row's exchange region; two rows of one warp (L = 16) sit 16 banks apart
     static constexpr int XWORDS = E * PITCH + (L == 16 && (E * PITCH) % 32 == 0 ? 16 : 0);
+    static constexpr int BEYOND = (M * L - E) * PITCH * 4;   // bytes that the idle threads read past it
     static constexpr int P = split_p<E>(), Q = split_q<E>();
 };
 
@@ -194,7 +227,8 @@ struct Factors {
 // wr: this thread's write base (region + l), rd: its read base (region + t PITCH); sync covers the
 // threads of the region.
 template <int N, class Sync>
-__device__ __forceinline__ void exchange(float2 (&v)[Plan<N>::E], float *wr, const float *rd, const Sync &sync) {
+__device__ __forceinline__ void exchange(const float2 (&v)[Plan<N>::E], float2 (&u)[Plan<N>::M * Plan<N>::L], float *wr,
+                                         const float *rd, const Sync &sync) {
     using PL = Plan<N>;
 #pragma unroll
     for (int k = 0; k < PL::E; ++k) wr[k * PL::PITCH] = v[k].x;
@@ -204,10 +238,10 @@ __device__ __forceinline__ void exchange(float2 (&v)[Plan<N>::E], float *wr, con
 #pragma unroll
         for (int i = 0; i < PL::L; i += 4) {
             const float4 q = *reinterpret_cast<const float4 *>(rd + m * PL::L * PL::PITCH + i);
-            v[m * PL::L + i].x = q.x;
-            v[m * PL::L + i + 1].x = q.y;
-            v[m * PL::L + i + 2].x = q.z;
-            v[m * PL::L + i + 3].x = q.w;
+            u[m * PL::L + i].x = q.x;
+            u[m * PL::L + i + 1].x = q.y;
+            u[m * PL::L + i + 2].x = q.z;
+            u[m * PL::L + i + 3].x = q.w;
         }
     sync();
 #pragma unroll
@@ -218,16 +252,12 @@ __device__ __forceinline__ void exchange(float2 (&v)[Plan<N>::E], float *wr, con
 #pragma unroll
         for (int i = 0; i < PL::L; i += 4) {
             const float4 q = *reinterpret_cast<const float4 *>(rd + m * PL::L * PL::PITCH + i);
-            v[m * PL::L + i].y = q.x;
-            v[m * PL::L + i + 1].y = q.y;
-            v[m * PL::L + i + 2].y = q.z;
-            v[m * PL::L + i + 3].y = q.w;
+            u[m * PL::L + i].y = q.x;
+            u[m * PL::L + i + 1].y = q.y;
+            u[m * PL::L + i + 2].y = q.z;
+            u[m * PL::L + i + 3].y = q.w;
         }
 }
-
-struct WarpSync {
-    __device__ __forceinline__ void operator()() const { __syncwarp(); }
-};
 
 // ---------------------------------------------------------------- tensor memory as thread-private storage
 

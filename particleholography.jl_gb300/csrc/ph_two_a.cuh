@@ -10,12 +10,16 @@ namespace two {
 
 // X_k = X_0 Hdz^k, inverse FFT along ky, transposed tensor-map store of T.  A CTA
 // holds the RB rows kx of one box; a row belongs to one warp (two rows per warp
-// at 256 and 512, two warps per row at 4096), so that the exchange needs no CTA
+// at 192 .. 512, two warps per row at 3072 and 4096), so that the exchange needs no CTA
 // barrier.  X_k and Hdz of a thread's values live in tensor memory (4 E columns
 // of its own lane): every slice reads both and writes back X_{k+1} = X_k Hdz.  X
-// is formed anew from the spectrum state at every multiple of CHAIN slices, which
-// keeps the chain's rounding at the transform's own: CHAIN = 8, and 16 with 64
-// values per thread, where forming X costs more (2048^2 x 256: 2.21 ms, 2.30 at 8).
+// is formed anew from the spectrum state at every multiple of CHAIN slices, so
+// that a projection is as near to the 64-bit one as with every slice formed
+// directly: relative error 4.1e-7 at 1024^2 (CHAIN = 8; 4.2e-7 direct), 2.7e-7 at
+// the short lengths (CHAIN = 4; 2.3e-7 direct, 4.0e-7 at 8).  At 2048 and 4096,
+// where the row engine ran chains of 64 slices (5.1e-6 at 4096, now 1.4e-6), 16.
+// Shorter chains cost: 1024^2 x 256 0.49 ms at 8, 0.51 at 4; 2048^2 x 256 2.21 ms
+// at 16, 2.30 at 8.
 //
 // In the row engine this pass moved 87 bytes per voxel through the shared-memory
 // data path (chain 24, two exchanges 32, staging 16, twiddles 15); here 32 to 40.
@@ -30,30 +34,43 @@ namespace two {
 // pass reads it long after: 0.56 -> 0.49 ms at 1024, 2.29 -> 2.21 ms at 2048^2 x
 // 256.  Measured slower at 2048: 2 x 1024 with 32 values per thread (2.57 ms);
 // two groups of tensor-memory columns per wait.
+//
+// 3 * 2^a lengths (12, 24 or 48 values per thread; a quarter of the threads idle
+// in stage 2), per launch in the row engine and here: 384^2 x 512 0.83 and 0.15 ms,
+// 768^2 x 256 1.13 and 0.31 ms, 1536^2 x 256 3.25 and 1.42 ms, 3072^2 x 64 3.49 and
+// 1.63 ms (the engine has no tensor-map store there and reads the phase rates from
+// L2 for every slice).
+
+// y per box: the largest of 256, 128, 64 that divides the length.
+__host__ __device__ constexpr int box_y(int n) { return n % 256 == 0 ? 256 : n % 128 == 0 ? 128 : 64; }
+
 template <int N>
 struct PassA {
     using PL = Plan<N>;
     using F = Factors<N, true>;
     static constexpr int RB = N <= 2048 ? 8 : 4;             // rows kx per CTA: one box
     static constexpr int THREADS = RB * PL::L;
-    static constexpr int CTAS = (PL::E == 64 ? 256 : 512) / THREADS;
+    static constexpr int CTAS = (PL::E >= 48 ? 256 : 512) / THREADS;
     static constexpr uint32_t WCOLS = 4 * PL::E;             // tensor-memory columns of a warp
-    static constexpr uint32_t COLS = WCOLS * (THREADS / 128);
+    // (an allocation is a power of two)
+    static constexpr uint32_t COLS = 1u << ilog2c(2 * (int)(WCOLS * (THREADS / 128)) - 1);
     static constexpr size_t STAGE = (size_t)RB * N * 8;
     static constexpr size_t XB = (size_t)PL::XWORDS * 4;
     static constexpr size_t SMEM = STAGE + RB * XB + F::BYTES + 24;
-    static constexpr int BOX_Y = kTwoBoxY;
-    static constexpr uint32_t CHAIN = PL::E == 64 ? 16 : 8;   // slices between two formations of X
+    static constexpr int BOX_Y = box_y(N);
+    static_assert(PL::BEYOND <= (int)F::BYTES, "idle threads read within the CTA's shared memory");
+    // slices between two formations of X
+    static constexpr uint32_t CHAIN = N <= 768 ? 4 : PL::E == 64 ? 16 : 8;
 };
 
 // Byte offset of (y, row r) in the staging [y][RB], with the tensor map's
 // swizzle (16-byte chunks exchanged by the address bits above 128 bytes): lanes
-// of consecutive y are RB x 8 bytes apart, and would meet in 4 (2) banks.  The
-// exchange has a period of 1024 bytes, so a multiple of that may be added after.
+// of consecutive y are RB x 8 bytes apart, and would meet in few banks.  The
+// exchange has a period of 512 (256) bytes, so a multiple of that may be added after.
 template <int RB>
 __device__ __forceinline__ uint32_t stage_offset(int y, int r) {
     const uint32_t a = (uint32_t)(y * RB + r) * 8;
-    return a ^ ((a >> 3) & (RB == 16 ? 0x70u : RB == 8 ? 0x30u : 0x10u));
+    return a ^ ((a >> 3) & (RB == 8 ? 0x30u : 0x10u));
 }
 
 template <int N, bool GROUPED>
@@ -176,9 +193,9 @@ __global__ void __launch_bounds__(PassA<N>::THREADS, PassA<N>::CTAS)
             }
             tmem_wait_st();
         }
-        float2 v[E];
+        float2 z[PL::M * L];
         {
-            float2 w[E];
+            float2 v[E], w[E];
             constexpr int V = P / 4;    // loads of 16 columns per group
             float x[2][V][16];          // X and Hdz of two groups: the next is on its way while one is used
             const auto fetch = [&](int n2) {
@@ -208,14 +225,14 @@ __global__ void __launch_bounds__(PassA<N>::THREADS, PassA<N>::CTAS)
             typename C::F f;
             f.load(opaque(tab), l);
             level2<E, true>(w, [&](int o, float2 y) { v[o] = f.apply(o, y); });
+            sync();   // every thread has read the previous exchange
+            exchange<N>(v, z, ex + l, ex + l * PL::PITCH, sync);
         }
-        sync();   // every thread has read the previous exchange
-        exchange<N>(v, ex + l, ex + l * PL::PITCH, sync);
-        float2 u[E];   // u[m L + o] = value of y = l + L m + E o
+        float2 u[PL::M * L];   // u[m L + o] = value of y = l + L m + E o
 #pragma unroll
         for (int m = 0; m < PL::M; ++m) {
             float2 w[L];
-            level1<L, true>(w, [&](int i) { return v[m * L + i]; });
+            level1<L, true>(w, [&](int i) { return z[m * L + i]; });
             level2<L, true>(w, [&](int o, float2 y) { u[m * L + o] = y; });
         }
         // the previous slice's boxes have left the staging
@@ -224,14 +241,19 @@ __global__ void __launch_bounds__(PassA<N>::THREADS, PassA<N>::CTAS)
             mbar_arrive(bar);
         }
         mbar_wait(bar, (uint32_t)(b - b0) & 1u, p.err);
+        // where steps of L and E in y are whole periods of the swizzle, one offset serves all
+        constexpr int PERIOD = RB == 8 ? 512 : 256;
+        constexpr bool WHOLE = L * RB * 8 % PERIOD == 0 && E * RB * 8 % PERIOD == 0;
         unsigned char *out = stage + stage_offset<RB>(l, r);
 #pragma unroll
         for (int m = 0; m < PL::M; ++m)
+            if (PL::M * L == E || l + L * m < E) {
 #pragma unroll
-            for (int o = 0; o < L; ++o) {
-                const int dy = L * m + E * o;
-                static_assert(L * RB * 8 % 1024 == 0 && E * RB * 8 % 1024 == 0, "whole periods of the swizzle");
-                *reinterpret_cast<float2 *>(out + dy * RB * 8) = u[m * L + o];
+                for (int o = 0; o < L; ++o) {
+                    const int dy = L * m + E * o;
+                    *reinterpret_cast<float2 *>(WHOLE ? out + dy * RB * 8 : stage + stage_offset<RB>(l + dy, r)) =
+                        u[m * L + o];
+                }
             }
         fence_proxy_async_smem();
         if (warp == 0) {

@@ -8,35 +8,38 @@ namespace ph {
 namespace two {
 
 // Rows y of T, inverse FFT along kx and the epilogue of ReconB.  A CTA is four
-// warps; a row belongs to one warp (two rows per warp at 256 and 512, two
-// warps per row at 2048 and 4096), so no barrier spans more than its threads.
+// warps; a row belongs to one warp (two rows per warp at 192 .. 512, two
+// warps per row from 1536), so no barrier spans more than its threads.
 // The row of slice b + 1 arrives by bulk copy as soon as slice b's has been
 // read into registers.  The running minima and their slices live in tensor
 // memory, 2 E columns of the thread's own lane: in registers they would not fit
 // beside the transform's 2 E values, and shared memory bounds the pass.
 //
-// 2048 = 2 x 1024: one warp transforms x[n] + x[n + 1024] (the even outputs),
+// 2048 = 2 x 1024 (and 1536 = 2 x 768): one warp transforms x[n] + x[n + 1024] (the even outputs),
 // the other (x[n] - x[n + 1024]) W^n (the odd ones).  Each row is read twice (8
 // bytes per voxel more), but 32 values per thread leave room for 16 warps per
 // SM: 3.19 ms per 2048^2 x 512 launch, against 3.64 ms with 64 values per
 // thread and 8 warps (latency: 54 % of issue slots), and 3.86 ms in the
 // three-stage row engine.  1024^2 x 256: 0.365 ms (0.483 in the engine; the
 // copy peak would take 0.316).  4096^2 x 128, 64 values: 3.82 ms (4.37).
+// 3 * 2^a: 768^2 x 256 0.247 ms (0.357), 1536^2 x 256 1.01 ms (1.35).
 // Measured slower: the stage factors read from the W^i table (gathers of up to
 // 32 lines: 3.77 ms at 2048) or held in registers across slices (spills).
 template <int N, int EPI, bool GROUPED>
 struct PassB {
-    static constexpr int H = N == 2048 ? 2 : 1;                      // transforms a row is split into
+    static constexpr int H = N == 2048 || N == 1536 ? 2 : 1;         // transforms a row is split into
     using PL = Plan<N / H>;
     static constexpr int THREADS = 128;
     static constexpr int TPR = H * PL::L;                    // threads per row
     static constexpr int ROWS = THREADS / TPR;
-    static constexpr int CTAS = PL::E == 64 ? 2 : 4;         // per SM: 255 registers at 64 values, 128 below
+    static constexpr int CTAS = PL::E >= 48 ? 2 : 4;         // per SM: 255 registers at 48 and 64 values, 128 below
+    static constexpr int CC = PL::M * PL::L;                 // outputs per thread (with the idle ones)
     static constexpr bool MIN = EPI == EPI_PROJ || EPI == EPI_VOL;
-    static constexpr uint32_t COLS = 2 * PL::E;              // minima, then slices
+    static constexpr uint32_t COLS = 2 * CC;                 // minima, then slices
     static constexpr size_t IN = (size_t)N * 8;
     static constexpr size_t XB = (size_t)PL::XWORDS * 4;
     using F = Factors<N / H, true, H>;
+    static_assert(PL::BEYOND <= (int)F::BYTES, "idle threads read within the CTA's shared memory");
     static constexpr size_t SMEM = ROWS * (IN + H * XB) + F::BYTES + ROWS * 8 + 16;
 };
 
@@ -106,9 +109,9 @@ __global__ void __launch_bounds__(128, PassB<N, EPI, GROUPED>::CTAS) k_two_b(con
             for (int i = 0; i < 16; ++i) inf[i] = __int_as_float(0x7f800000);
             float zero[16] = {};
 #pragma unroll
-            for (int c = 0; c < E; c += 16) {
+            for (int c = 0; c < C::CC; c += 16) {
                 tmem_st16(tm + c, inf);
-                tmem_st16(tm + E + c, zero);
+                tmem_st16(tm + C::CC + c, zero);
             }
             tmem_wait_st();
         }
@@ -122,9 +125,9 @@ __global__ void __launch_bounds__(128, PassB<N, EPI, GROUPED>::CTAS) k_two_b(con
             if (valid) mbar_wait(bars + r, parity, p.err);
             if constexpr (L < 32) __syncwarp();
             parity ^= 1u;
-            float2 v[E];
+            float2 z[C::CC];
             {
-                float2 w[E];
+                float2 v[E], w[E];
                 if constexpr (H == 1) {
                     level1<E, true>(w, [&](int i) { return in[l + L * i]; });
                 } else {
@@ -147,13 +150,14 @@ __global__ void __launch_bounds__(128, PassB<N, EPI, GROUPED>::CTAS) k_two_b(con
                 sync_row();   // the row is in registers (and the exchange region free): refill it
                 if (l == 0 && h == 0 && valid && b + 1 < b1) issue(b + 1);
                 level2<E, true>(w, [&](int o, float2 x) { v[o] = f.apply(o, x); });
+                exchange<N / H>(v, z, ex + l, ex + l * PL::PITCH, sync);
             }
-            exchange<N / H>(v, ex + l, ex + l * PL::PITCH, sync);
 #pragma unroll
             for (int m = 0; m < PL::M; ++m) {
                 float2 w[L], u[L];
-                level1<L, true>(w, [&](int i) { return v[m * L + i]; });
+                level1<L, true>(w, [&](int i) { return z[m * L + i]; });
                 level2<L, true>(w, [&](int o, float2 x) { u[o] = x; });
+                const bool live = PL::M * L == E || l + L * m < E;   // not an idle thread's
                 // output o is column x = H (l + L m + E o) + h
                 if constexpr (C::MIN) {
 #pragma unroll
@@ -168,7 +172,7 @@ __global__ void __launch_bounds__(128, PassB<N, EPI, GROUPED>::CTAS) k_two_b(con
                             // store() converts and stores one value and gives back what it stored; the
                             // type is chosen once per 16 values
                             const size_t row = (size_t)k * p.vol_slice_stride + (size_t)y * p.nx_out;
-                            const unsigned width = valid ? (unsigned)p.nx_out : 0u;
+                            const unsigned width = valid && live ? (unsigned)p.nx_out : 0u;
                             const auto store16 = [&](auto *vol, auto &&convert) {
                                 auto *out = vol + row;
 #pragma unroll
@@ -207,7 +211,7 @@ __global__ void __launch_bounds__(128, PassB<N, EPI, GROUPED>::CTAS) k_two_b(con
                         if (track) {
                             float mv[16], mk[16];
                             tmem_ld16(tm + m * L + c, mv);
-                            tmem_ld16(tm + E + m * L + c, mk);
+                            tmem_ld16(tm + C::CC + m * L + c, mk);
                             tmem_wait(mv);
                             tmem_wait(mk);
 #pragma unroll
@@ -215,13 +219,14 @@ __global__ void __launch_bounds__(128, PassB<N, EPI, GROUPED>::CTAS) k_two_b(con
                                 if (i2[i] < mv[i]) { mv[i] = i2[i]; mk[i] = __int_as_float(k); }
                             }
                             tmem_st16(tm + m * L + c, mv);
-                            tmem_st16(tm + E + m * L + c, mk);
+                            tmem_st16(tm + C::CC + m * L + c, mk);
                         }
                     }
                 } else {
 #pragma unroll
                     for (int i = 0; i < L; ++i) {
                         const int x = H * (l + L * m + E * i) + h;
+                        if (!live) continue;
                         if constexpr (EPI == EPI_SUB) {
                             if (sub_b == sub_e) continue;
                             const float i2 = clamp01(fmaf(u[i].x, u[i].x, u[i].y * u[i].y));
@@ -247,17 +252,17 @@ __global__ void __launch_bounds__(128, PassB<N, EPI, GROUPED>::CTAS) k_two_b(con
         if constexpr (C::MIN) {
             if (track) {
 #pragma unroll
-                for (int c = 0; c < E; c += 16) {
+                for (int c = 0; c < C::CC; c += 16) {
                     float mv[16], mk[16];
                     tmem_ld16(tm + c, mv);
-                    tmem_ld16(tm + E + c, mk);
+                    tmem_ld16(tm + C::CC + c, mk);
                     tmem_wait(mv);
                     tmem_wait(mk);
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
                         const int m = (c + i) / L, o = (c + i) % L;
                         const int xo = H * (l + L * m + E * o) + h - p.x0;
-                        if (valid && xo >= 0 && xo < p.nx_out)
+                        if (valid && (PL::M * L == E || l + L * m < E) && xo >= 0 && xo < p.nx_out)
                             atomicMin(proj64 + (size_t)y * p.nx_out + xo, pack_min(mv[i], __float_as_int(mk[i])));
                     }
                 }
@@ -275,7 +280,7 @@ __global__ void __launch_bounds__(128, PassB<N, EPI, GROUPED>::CTAS) k_two_b(con
 template <int N, int EPI, bool GROUPED>
 cudaError_t launch_b(const ReconB<EPI, GROUPED> &p, int groups, int items, cudaStream_t s) {
     using C = PassB<N, EPI, GROUPED>;
-    static_assert(C::SMEM <= kSmemMax / C::CTAS, "the CTAs of an SM share its shared memory");
+    static_assert((C::SMEM + 1024) * C::CTAS <= 228 * 1024, "the CTAs of an SM share its shared memory");
     auto kern = k_two_b<N, EPI, GROUPED>;
     static unsigned long long done_mask = 0;   // per-device opt-in to more than 48 KB of dynamic shared memory
     int dev = 0;

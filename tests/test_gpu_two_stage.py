@@ -1,6 +1,8 @@
-"""The two-stage row transform of pass B (lengths 256 .. 4096) against the oracle
-at its edges: a CTA with fewer rows than it holds, a warp of two rows with one,
-one slice, slice counts that leave the last group short."""
+"""The two-stage row transform of passes A and B (lengths 192 .. 4096) against the
+oracle at its edges: a CTA with fewer rows than it holds, a warp of two rows with
+one, threads without a transform of their own (3 * 2^a), a box of kx that ends
+outside the frame, one slice, slice counts that leave the last group short and
+cross the lengths of the product chain."""
 import numpy as np
 import pytest
 import torch
@@ -17,7 +19,12 @@ TOL = 5e-6
 
 @pytest.mark.parametrize("nx,ny,slices", [(256, 1, 1), (256, 3, 5), (256, 24, 33), (512, 1, 2), (512, 6, 65),
                                           (512, 96, 7), (1024, 3, 3), (1024, 6, 34), (2048, 1, 5), (2048, 3, 3),
-                                          (2048, 12, 17), (4096, 1, 2), (4096, 3, 9)])
+                                          (2048, 12, 17), (4096, 1, 2), (4096, 3, 9), (192, 1, 2), (192, 6, 33),
+                                          (384, 3, 5), (768, 1, 3), (768, 6, 34), (1536, 3, 17), (3072, 1, 2),
+                                          (3072, 3, 9),
+                                          (4, 192, 3), (24, 192, 18), (4, 256, 1), (12, 256, 35), (12, 384, 9),
+                                          (12, 512, 17), (24, 768, 18), (4, 1024, 9), (12, 1024, 33), (8, 1536, 34),
+                                          (12, 2048, 17), (4, 3072, 18), (4, 4096, 17)])
 def test_rows_and_slices_at_the_edges(ph, cuda, nx, ny, slices):
     rng = np.random.default_rng(nx + ny)
     holo = rng.uniform(0.1, 1.0, (ny, nx)).astype(np.float32)
