@@ -808,20 +808,6 @@ EncodeTiledFn encode_tiled() {
     return fn;
 }
 
-// Tensor map of a centred transfer [ny][nx] (8-byte elements) for the staged
-// spectrum pass: boxes of `rows` columns x 256 rows.
-bool tf_load_map(CUtensorMap *tm, const float2 *h, int nx, int ny, int rows) {
-    const EncodeTiledFn enc = encode_tiled();
-    if (enc == nullptr || ((uintptr_t)h & 15) != 0 || nx % 2 != 0 || rows < 2 || rows > 32) return false;
-    const cuuint64_t dims[2] = {(cuuint64_t)nx, (cuuint64_t)ny};
-    const cuuint64_t strides[1] = {(cuuint64_t)nx * 8};
-    const cuuint32_t box[2] = {(cuuint32_t)rows, 256};
-    const cuuint32_t estr[2] = {1, 1};
-    return enc(tm, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, const_cast<float2 *>(h), dims, strides, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 // Forward FFT of the (optionally mean-padded) wavefront and the spectrum state.
 // nx, ny: transform size; a1: scratch [nx][ny] complex.  With `holo` (and wf
 // NULL) the wavefront is sqrt(holo) + 0i, formed in the first FFT stage.
@@ -870,18 +856,7 @@ int issue_spectrum(ph_ctx *ctx, const float2 *wf, const float2 *hf, const float2
     c.nx = nx;
     c.ny = ny;
     c.scale = (float)(1.0 / ((double)nx * (double)ny));
-    // the transfers staged by tensor-map boxes where the lengths allow it
-    const int rows = spectrum_staged_rows(ny);
-    CUtensorMap tm_hf, tm_hdz;
-    if (lpf == nullptr && rows > 0 && nx % (2 * rows) == 0 &&
-        tf_load_map(&tm_hf, hf, nx, ny, rows) && tf_load_map(&tm_hdz, hdz, nx, ny, rows)) {
-        SpectrumColsT ct{};
-        static_cast<SpectrumCols &>(ct) = c;
-        ct.err = static_cast<int *>(ctx->small);
-        PH_TRY(pass(ctx, s, "spectrum", [&] { return launch_spectrum_staged(ny, ct, tm_hf, tm_hdz, s); }));
-        return PH_OK;
-    }
-    PH_TRY(pass(ctx, s, "spectrum", [&] { return launch_spectrum(ny, c, s); }));
+    PH_TRY(pass(ctx, s, "spectrum", [&] { return launch_spectrum(ny, c, s); }, spectrum_launches(ny)));
     return PH_OK;
 }
 
@@ -1354,7 +1329,7 @@ int issue_recon_group(ph_ctx *ctx, const std::vector<const ph_recon_item *> &its
     c.ny = ny;
     c.scale = (float)(1.0 / ((double)nx * (double)ny));
     c.nitems = G;
-    PH_TRY(pass(ctx, s, "spectrum", [&] { return launch_spectrum(ny, c, s); }));
+    PH_TRY(pass(ctx, s, "spectrum", [&] { return launch_spectrum(ny, c, s); }, spectrum_launches(ny)));
     const size_t npix = (size_t)nx * ny;
     for (int i = 0; i < G; ++i)
         PH_CUDA(cudaMemsetAsync(slot(i, L.p64), 0xff, sizeof(unsigned long long) * npix, s), "cudaMemsetAsync");

@@ -1,4 +1,4 @@
-// Reconstruction pass A on the two-stage transform (lengths 192 .. 4096).
+// Reconstruction pass A on the two-stage transform (lengths 128 .. 4096).
 #include "ph_two_a.cuh"
 
 namespace ph {

@@ -16,7 +16,7 @@ namespace ph {
 // The lengths whose pass B runs the row engine of ph_fft.cuh (the others run the
 // two-stage transform of ph_two.cuh).
 #define PH_FOR_EACH_N_ENGINE(X) \
-    X(1) X(2) X(4) X(8) X(16) X(32) X(64) X(128) X(8192) X(3) X(6) X(12) X(24) X(48) X(96) X(6144)
+    X(1) X(2) X(4) X(8) X(16) X(32) X(64) X(8192) X(3) X(6) X(12) X(24) X(48) X(96) X(6144)
 
 inline bool supported_len(int n) {
     if (n < 1) return false;
@@ -171,31 +171,6 @@ cudaError_t launch_one_tm(const Body &body, const CUtensorMap &tm, int nrows, in
     return cudaLaunchKernelEx(&cfg, kern, body, tm);
 }
 
-// A plain launch of k_pass_tm2 (two tensor maps), one grid row.
-template <int N, bool ROW_FAST, class Body>
-cudaError_t launch_one_tm2(const Body &body, const CUtensorMap &tm0, const CUtensorMap &tm1, int nrows,
-                           cudaStream_t s) {
-    auto kern = k_pass_tm2<N, ROW_FAST, Body>;
-    constexpr size_t smem = Body::template smem<N, ROW_FAST>();
-    static_assert(smem <= kSmemMax, "pass needs more shared memory than a CTA has");
-    if constexpr (smem > 48 * 1024) {
-        static unsigned long long done_mask = 0;
-        int dev = 0;
-        cudaGetDevice(&dev);
-        const unsigned long long bit = 1ull << (dev & 63);
-        if (!(__atomic_load_n(&done_mask, __ATOMIC_ACQUIRE) & bit)) {
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-            if (e != cudaSuccess) return e;
-            __atomic_fetch_or(&done_mask, bit, __ATOMIC_ACQ_REL);
-        }
-    }
-    using S = Shape<N, Body::EPT, Body::TT>;
-    const int gx = (nrows + S::ROWS - 1) / S::ROWS;
-    if (gx == 0) return cudaSuccess;
-    kern<<<gx, S::THREADS, smem, s>>>(body, tm0, tm1);
-    return cudaGetLastError();
-}
-
 // Launch of a pass that exists only for the lengths where Body::staged<N>() holds.
 template <bool ROW_FAST, class Body>
 cudaError_t launch_staged_len(int n, const Body &body, int nrows, cudaStream_t s) {
@@ -247,16 +222,11 @@ cudaError_t launch_engine_len(int n, const Body &body, int nrows, int grid_y, cu
 cudaError_t launch_fwd_rows(int n, const FwdRowsT<FWD_COMPLEX> &b, cudaStream_t s);
 cudaError_t launch_fwd_rows(int n, const FwdRowsT<FWD_SQRT_REAL> &b, cudaStream_t s);
 cudaError_t launch_fwd_rows(int n, const FwdRowsT<FWD_PADDED> &b, cudaStream_t s);
-cudaError_t launch_spectrum(int n, const SpectrumCols &b, cudaStream_t s);
-// The spectrum pass with staged transfers (lengths 512 .. 2048; spectrum_staged_rows
-// gives the rows per CTA, 0 elsewhere); tm_hf, tm_hdz: the centred transfers
-// as [n_slow][n_fast] 8-byte elements, boxes of rows x 256.
-int spectrum_staged_rows(int n);
-cudaError_t launch_spectrum_staged(int n, const SpectrumColsT &b, const CUtensorMap &tm_hf, const CUtensorMap &tm_hdz,
-                                   cudaStream_t s);
+cudaError_t launch_spectrum(int n, const SpectrumCols &b, cudaStream_t s);   // overwrites a1 at the two-stage lengths
+int spectrum_launches(int n);   // its kernels
 cudaError_t launch_recon_a(int n, const ReconA &b, int nbatch, cudaStream_t s);
 // Pass A on the two-stage transform with the tensor-map store (ph_two_a.cuh):
-// lengths 192 .. 4096, frames whose stored rows [y0, y0 + ny_out) are whole
+// lengths 128 .. 4096, frames whose stored rows [y0, y0 + ny_out) are whole
 // boxes.  tm: T as (kx, y, slice) or, grouped, (kx, y, slice, item), 8-byte
 // elements, boxes of recon_a_two_box(n) kx x recon_a_two_box_y(n) y, swizzled by
 // the box's row of kx.  Its CTAs per SM.
@@ -277,7 +247,7 @@ cudaError_t launch_gs_row_ts(int n, const GsRowMidT &b, const CUtensorMap &tm, c
 cudaError_t launch_recon_b_group(int n, const ReconB<EPI_PROJ, true> &b, cudaStream_t s);
 int recon_a_rows(int n);   // rows per pass A CTA for transform length n
 bool recon_a_chain(int n);   // whether the row engine's pass A at length n advances X by the product chain
-// Pass B at 192 .. 4096 runs the two-stage transform (ph_two_b.cuh): its CTAs
+// Pass B at 128 .. 4096 runs the two-stage transform (ph_two_b.cuh): its CTAs
 // per slice group over `rows` rows, and per SM (0 at the other lengths).
 int recon_b_ctas(int n, int rows);
 int recon_b_ctas_per_sm(int n);

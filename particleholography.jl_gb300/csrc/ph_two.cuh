@@ -109,8 +109,12 @@ __device__ __forceinline__ void d6(float2 (&v)[6]) {   // n = 3 n1 + n2, k = k1 
 
 template <int R, bool INV>
 __device__ __forceinline__ void bfly(float2 (&v)[R]) {
-    static_assert(R == 3 || R == 4 || R == 6 || R == 8, "a butterfly of this size");
-    if constexpr (R == 3) d3<INV>(v[0], v[1], v[2]);
+    static_assert(R == 2 || R == 3 || R == 4 || R == 6 || R == 8, "a butterfly of this size");
+    if constexpr (R == 2) {
+        const float2 t = v[0];
+        v[0] = add2(t, v[1]);
+        v[1] = sub2(t, v[1]);
+    } else if constexpr (R == 3) d3<INV>(v[0], v[1], v[2]);
     else if constexpr (R == 4) d4<INV>(v[0], v[1], v[2], v[3]);
     else if constexpr (R == 6) d6<INV>(v);
     else d8<INV>(v);
@@ -162,18 +166,18 @@ __device__ __forceinline__ void level2(const float2 (&y)[R], Out &&out) {
 // ---------------------------------------------------------------- shape
 
 // The lengths that have a two-stage transform.
-#define PH_FOR_EACH_N_TWO(X) X(192) X(256) X(384) X(512) X(768) X(1024) X(1536) X(2048) X(3072) X(4096)
+#define PH_FOR_EACH_N_TWO(X) X(128) X(192) X(256) X(384) X(512) X(768) X(1024) X(1536) X(2048) X(3072) X(4096)
 
 // Values per thread, threads per row, and transforms of length L per thread in
-// stage 2.  At 3 * 2^a lengths the last of these (all, where M = 1) has only the
-// threads t < E - (M - 1) L: the others compute on whatever follows the row's
-// exchange region (within the CTA's shared memory) and drop it.
+// stage 2.  At 128 and the 3 * 2^a lengths the last of these (all, where M = 1)
+// has only the threads t < E - (M - 1) L: the others compute on the last one's
+// values and drop them.
 __host__ __device__ constexpr int values(int n) {
-    return n % 3 == 0 ? (n <= 192 ? 12 : n <= 768 ? 24 : 48) : n <= 256 ? 16 : n <= 1024 ? 32 : 64;
+    return n % 3 == 0 ? (n <= 192 ? 12 : n <= 768 ? 24 : 48) : n <= 128 ? 8 : n <= 256 ? 16 : n <= 1024 ? 32 : 64;
 }
 __host__ __device__ constexpr bool supported(int n) {
-    return n == 192 || n == 256 || n == 384 || n == 512 || n == 768 || n == 1024 || n == 1536 || n == 2048 ||
-           n == 3072 || n == 4096;
+    return n == 128 || n == 192 || n == 256 || n == 384 || n == 512 || n == 768 || n == 1024 || n == 1536 ||
+           n == 2048 || n == 3072 || n == 4096;
 }
 
 template <int N>
@@ -183,7 +187,6 @@ struct Plan {
     static constexpr int PITCH = L + 4;                      // words between the exchange rows of k1, k1 + 1
     // words of a row's exchange region; two rows of one warp (L = 16) sit 16 banks apart
     static constexpr int XWORDS = E * PITCH + (L == 16 && (E * PITCH) % 32 == 0 ? 16 : 0);
-    static constexpr int BEYOND = (M * L - E) * PITCH * 4;   // bytes that the idle threads read past it
     static constexpr int P = split_p<E>(), Q = split_q<E>();
 };
 
@@ -213,6 +216,14 @@ struct Factors {
 #pragma unroll
         for (int q = 1; q < PL::Q; ++q) b[q] = tab[(PL::P - P0 + q - 1) * H * PL::L];
     }
+    // the same from the W^i table
+    __device__ __forceinline__ void load_global(const float2 *__restrict__ tw, int l) {
+        static_assert(H == 1, "whole transforms");
+#pragma unroll
+        for (int p = 1; p < PL::P; ++p) a[p] = load_tw<INV>(tw, l * p);
+#pragma unroll
+        for (int q = 1; q < PL::Q; ++q) b[q] = load_tw<INV>(tw, l * q * PL::P);
+    }
     // v times the twiddle of output k
     __device__ __forceinline__ float2 apply(int k, float2 v) const {
         const int p = k % PL::P, q = k / PL::P;
@@ -223,40 +234,48 @@ struct Factors {
     }
 };
 
-// One exchange: v[k1] of thread l -> u[m L + i] = the value of (l = i, k1 = t + L m) for thread t.
-// wr: this thread's write base (region + l), rd: its read base (region + t PITCH); sync covers the
-// threads of the region.
+// One exchange through the row's region `ex`: v[k1] of thread t -> u[m L + i] =
+// the value of (l = i, k1 = t + L m).  sync covers the threads of the region.
 template <int N, class Sync>
-__device__ __forceinline__ void exchange(const float2 (&v)[Plan<N>::E], float2 (&u)[Plan<N>::M * Plan<N>::L], float *wr,
-                                         const float *rd, const Sync &sync) {
+__device__ __forceinline__ void exchange(const float2 (&v)[Plan<N>::E], float2 (&u)[Plan<N>::M * Plan<N>::L], float *ex,
+                                         int t, const Sync &sync) {
     using PL = Plan<N>;
+    float *wr = ex + t;
+    // (an idle thread reads the last row)
+    const auto row = [&](int m) {
+        return ex + (PL::M * PL::L == PL::E ? t + PL::L * m : min(t + PL::L * m, PL::E - 1)) * PL::PITCH;
+    };
 #pragma unroll
     for (int k = 0; k < PL::E; ++k) wr[k * PL::PITCH] = v[k].x;
     sync();
 #pragma unroll
-    for (int m = 0; m < PL::M; ++m)
+    for (int m = 0; m < PL::M; ++m) {
+        const float *rd = row(m);
 #pragma unroll
         for (int i = 0; i < PL::L; i += 4) {
-            const float4 q = *reinterpret_cast<const float4 *>(rd + m * PL::L * PL::PITCH + i);
+            const float4 q = *reinterpret_cast<const float4 *>(rd + i);
             u[m * PL::L + i].x = q.x;
             u[m * PL::L + i + 1].x = q.y;
             u[m * PL::L + i + 2].x = q.z;
             u[m * PL::L + i + 3].x = q.w;
         }
+    }
     sync();
 #pragma unroll
     for (int k = 0; k < PL::E; ++k) wr[k * PL::PITCH] = v[k].y;
     sync();
 #pragma unroll
-    for (int m = 0; m < PL::M; ++m)
+    for (int m = 0; m < PL::M; ++m) {
+        const float *rd = row(m);
 #pragma unroll
         for (int i = 0; i < PL::L; i += 4) {
-            const float4 q = *reinterpret_cast<const float4 *>(rd + m * PL::L * PL::PITCH + i);
+            const float4 q = *reinterpret_cast<const float4 *>(rd + i);
             u[m * PL::L + i].y = q.x;
             u[m * PL::L + i + 1].y = q.y;
             u[m * PL::L + i + 2].y = q.z;
             u[m * PL::L + i + 3].y = q.w;
         }
+    }
 }
 
 // ---------------------------------------------------------------- tensor memory as thread-private storage

@@ -10,7 +10,7 @@ namespace two {
 
 // X_k = X_0 Hdz^k, inverse FFT along ky, transposed tensor-map store of T.  A CTA
 // holds the RB rows kx of one box; a row belongs to one warp (two rows per warp
-// at 192 .. 512, two warps per row at 3072 and 4096), so that the exchange needs no CTA
+// at 128 .. 512, two warps per row at 3072 and 4096), so that the exchange needs no CTA
 // barrier.  X_k and Hdz of a thread's values live in tensor memory (4 E columns
 // of its own lane): every slice reads both and writes back X_{k+1} = X_k Hdz.  X
 // is formed anew from the spectrum state at every multiple of CHAIN slices, so
@@ -58,7 +58,6 @@ struct PassA {
     static constexpr size_t XB = (size_t)PL::XWORDS * 4;
     static constexpr size_t SMEM = STAGE + RB * XB + F::BYTES + 24;
     static constexpr int BOX_Y = box_y(N);
-    static_assert(PL::BEYOND <= (int)F::BYTES, "idle threads read within the CTA's shared memory");
     // slices between two formations of X
     static constexpr uint32_t CHAIN = N <= 768 ? 4 : PL::E == 64 ? 16 : 8;
 };
@@ -226,7 +225,7 @@ __global__ void __launch_bounds__(PassA<N>::THREADS, PassA<N>::CTAS)
             f.load(opaque(tab), l);
             level2<E, true>(w, [&](int o, float2 y) { v[o] = f.apply(o, y); });
             sync();   // every thread has read the previous exchange
-            exchange<N>(v, z, ex + l, ex + l * PL::PITCH, sync);
+            exchange<N>(v, z, ex, l, sync);
         }
         float2 u[PL::M * L];   // u[m L + o] = value of y = l + L m + E o
 #pragma unroll

@@ -8,7 +8,7 @@ namespace ph {
 namespace two {
 
 // Rows y of T, inverse FFT along kx and the epilogue of ReconB.  A CTA is four
-// warps; a row belongs to one warp (two rows per warp at 192 .. 512, two
+// warps; a row belongs to one warp (two rows per warp at 128 .. 512, two
 // warps per row from 1536), so no barrier spans more than its threads.
 // The row of slice b + 1 arrives by bulk copy as soon as slice b's has been
 // read into registers.  The running minima and their slices live in tensor
@@ -39,7 +39,6 @@ struct PassB {
     static constexpr size_t IN = (size_t)N * 8;
     static constexpr size_t XB = (size_t)PL::XWORDS * 4;
     using F = Factors<N / H, true, H>;
-    static_assert(PL::BEYOND <= (int)F::BYTES, "idle threads read within the CTA's shared memory");
     static constexpr size_t SMEM = ROWS * (IN + H * XB) + F::BYTES + ROWS * 8 + 16;
 };
 
@@ -150,7 +149,7 @@ __global__ void __launch_bounds__(128, PassB<N, EPI, GROUPED>::CTAS) k_two_b(con
                 sync_row();   // the row is in registers (and the exchange region free): refill it
                 if (l == 0 && h == 0 && valid && b + 1 < b1) issue(b + 1);
                 level2<E, true>(w, [&](int o, float2 x) { v[o] = f.apply(o, x); });
-                exchange<N / H>(v, z, ex + l, ex + l * PL::PITCH, sync);
+                exchange<N / H>(v, z, ex, l, sync);
             }
 #pragma unroll
             for (int m = 0; m < PL::M; ++m) {
