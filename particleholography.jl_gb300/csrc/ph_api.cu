@@ -24,6 +24,7 @@
 
 #include "ph_ctx.h"
 #include "ph_launch.cuh"
+#include "ph_two.cuh"
 #include "ph_pass_tc.cuh"
 
 // The serving runtime: work slots (one CUDA stream each), a scratch pool
@@ -142,6 +143,15 @@ __global__ void k_twiddle_stage(float2 *blk, int n, int radix, int ns) {
     if (e >= (radix - 1) * ns) return;
     const int r = e / ns + 1, k = e % ns;
     blk[e] = twiddle_fp64(r * k * (n / (ns * radix)), n);
+}
+
+// The stage factors of the two-stage transform (layout in ph_two.cuh): of length r
+// over `lanes` threads, [factor][l], split r = p q.
+__global__ void k_two_factors(float2 *out, int n, int lanes, int p, int q) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (p + q - 2) * lanes) return;
+    const int l = i % lanes, j = i / lanes;
+    out[i] = twiddle_fp64(l * (j < p - 1 ? j + 1 : p * (j - p + 2)), n);
 }
 
 // holofunc.jl:8-15 with the reference's Float64 operation order; the
@@ -355,11 +365,6 @@ __global__ void k_background_mean(double *out, const uint8_t *__restrict__ image
     out[p] = acc / (double)count;
 }
 
-__global__ void k_sqrt_f32(float *out, const float *in, size_t n) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = sqrtf(in[i]);
-}
-
 __global__ void k_sum_f32(const float *in, size_t n, double *acc) {
     double sx = 0.0;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
@@ -478,21 +483,70 @@ __global__ void k_resid_finish(const double *acc, double *out) {
     *out = acc[1] > 0.0 ? sqrt(acc[0] / acc[1]) : 0.0;
 }
 
-// ht[kx][ky] = scale * h[shift(ky)][shift(kx)]: a centred [ny][nx] transfer
-// rearranged to the [kx][ky] rows the staged column pass multiplies by
-// (32 x 32 tiles through shared memory, both sides coalesced).
-__global__ void k_transfer_rows(float2 *ht, const float2 *h, int nx, int ny, float scale) {
+// What phase retrieval prepares once per call, for both planes (blockIdx.z): ht[kx][ky]
+// = scale * h[shift(ky)][shift(kx)], a centred [ny][nx] transfer rearranged to the
+// [kx][ky] rows that the column pass multiplies by (32 x 32 tiles through shared
+// memory, both sides coalesced), and the amplitudes sqrt(I).
+struct GsSetup {
+    const float2 *h[2];
+    float2 *ht[2];
+    const float *holo[2];
+    float *amp[2];
+};
+__global__ void __launch_bounds__(256) k_gs_setup(const GsSetup g, int nx, int ny, float scale) {
     __shared__ float2 tile[32][33];
+    const int z = blockIdx.z, tx = threadIdx.x % 32, ty = threadIdx.x / 32;
     const int kx0 = blockIdx.x * 32, ky0 = blockIdx.y * 32;
-    for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-        const int ky = ky0 + i, kx = kx0 + threadIdx.x;
-        if (ky < ny && kx < nx) tile[i][threadIdx.x] = h[(size_t)shift_idx(ky, ny) * nx + shift_idx(kx, nx)];
+    const float2 *h = g.h[z];
+    const float *holo = g.holo[z];
+    float i4[4];
+    float2 h4[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int ky = min(ky0 + ty + 8 * i, ny - 1), kx = min(kx0 + tx, nx - 1);
+        h4[i] = h[(size_t)shift_idx(ky, ny) * nx + shift_idx(kx, nx)];
+        i4[i] = holo[(size_t)ky * nx + kx];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int ky = ky0 + ty + 8 * i, kx = kx0 + tx;
+        tile[ty + 8 * i][tx] = h4[i];
+        if (ky < ny && kx < nx) g.amp[z][(size_t)ky * nx + kx] = sqrtf(i4[i]);
     }
     __syncthreads();
-    for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-        const int kx = kx0 + i, ky = ky0 + threadIdx.x;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int kx = kx0 + ty + 8 * i, ky = ky0 + tx;
         if (kx < nx && ky < ny) {
-            const float2 v = tile[threadIdx.x][i];
+            const float2 v = tile[tx][ty + 8 * i];
+            g.ht[z][(size_t)kx * ny + ky] = make_float2(v.x * scale, v.y * scale);
+        }
+    }
+}
+
+// The same rows of a transfer formed on the way from the square-root term
+// (holofunc.jl:383-388): ht[kx][ky] = scale * exp(i c sqrt(d[shift(ky)][shift(kx)])).
+__global__ void __launch_bounds__(256)
+    k_transfer_rows(float2 *ht, const float *__restrict__ d_sqr, int nx, int ny, float scale, const TurnRate a,
+                    const float4 *__restrict__ ptab) {
+    __shared__ float4 tab[kTurnTable];
+    __shared__ float2 tile[32][33];
+    const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;
+    tab[threadIdx.x] = __ldg(ptab + threadIdx.x * (kPhaseTable / kTurnTable));
+    __syncthreads();
+    const int kx0 = blockIdx.x * 32, ky0 = blockIdx.y * 32;
+#pragma unroll
+    for (int i = 0; i < 32; i += 8) {
+        const int ky = ky0 + ty + i, kx = kx0 + tx;
+        if (ky < ny && kx < nx)
+            tile[ty + i][tx] = transfer_value(d_sqr[(size_t)shift_idx(ky, ny) * nx + shift_idx(kx, nx)], a, tab);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 32; i += 8) {
+        const int kx = kx0 + ty + i, ky = ky0 + tx;
+        if (kx < nx && ky < ny) {
+            const float2 v = tile[tx][ty + i];
             ht[(size_t)kx * ny + ky] = make_float2(v.x * scale, v.y * scale);
         }
     }
@@ -627,7 +681,9 @@ int get_twiddles(ph_ctx *ctx, int n, cudaStream_t s, const float2 **out) {
     }
     float2 *p = nullptr;
     const int e = engine_e(n, PassBase::EPT);
-    PH_CUDA(cudaMalloc(&p, sizeof(float2) * (size_t)plan_tw_size(n, e)), "cudaMalloc(twiddles)");
+    const bool two_stage = two::supported(n);
+    const size_t entries = two_stage ? two::table_size(n) : plan_tw_size(n, e);
+    PH_CUDA(cudaMalloc(&p, sizeof(float2) * entries), "cudaMalloc(twiddles)");
     k_twiddle<<<(n + 255) / 256, 256, 0, s>>>(p, n);
     ctx->launches++;
     PH_CUDA(cudaGetLastError(), "k_twiddle");
@@ -637,6 +693,17 @@ int get_twiddles(ph_ctx *ctx, int n, cudaStream_t s, const float2 **out) {
         k_twiddle_stage<<<(cnt + 255) / 256, 256, 0, s>>>(p + plan_tw_offset(n, e, st), n, r, ns);
         ctx->launches++;
         PH_CUDA(cudaGetLastError(), "k_twiddle_stage");
+    }
+    if (two_stage) {
+        const int E = two::values(n), L = n / E;
+        const auto fill = [&](int offset, int r, int lanes) {
+            const int pp = two::split_p_of(r), qq = r / pp, cnt = two::factors_of(r, lanes);
+            k_two_factors<<<(cnt + 255) / 256, 256, 0, s>>>(p + offset, n, lanes, pp, qq);
+            ctx->launches++;
+            return cudaGetLastError();
+        };
+        PH_CUDA(fill(two::factors_offset(n), E, L), "k_two_factors");
+        PH_CUDA(fill(two::mirror_offset(n), L, E), "k_two_factors");
     }
     ctx->tw[n] = p;
     *out = p;
@@ -1636,8 +1703,17 @@ int32_t ph_phase_retrieval(ph_ctx *ctx, void *out, const float *holo1, const flo
         if (residual) PH_CUDA(cudaMemsetAsync(residual, 0, sizeof(double), s), "memset");
         PH_LEAVE(ctx);
     }
-    // The staged persistent passes take the transfers as [kx][ky] rows.
-    const bool staged = gs_row_staged(nx) && gs_col_staged(ny);
+    // The persistent staged passes (1024, 2048 and 4096) and the two-stage passes take
+    // the transfers as [kx][ky] rows and the amplitudes; a context whose budget has no
+    // room for them runs the one-shot passes where it did.  Two-stage where the
+    // persistent form does not exist: per pass, one-shot and two-stage, 12.6 and 3.0 us
+    // at 256^2, 12.3 and 5.8 at 512^2, 19.2 and 6.3 at 768^2, 43.5 and 28.7 at 1536^2;
+    // persistent and two-stage, 8.2 and 8.4 us at 1024^2, 28 and 45 at 2048^2, 149 and
+    // 163 at 4096^2 (there 64 values per thread leave 8 warps per SM).
+    const bool persistent = gs_row_staged(nx) && gs_col_staged(ny);
+    const size_t rows_bytes = n * (4 * sizeof(float2) + 2 * sizeof(float)) + 6 * kAlign;
+    const bool two_stage = !persistent && gs_two(nx) && gs_two(ny) && (ctx->budget == 0 || rows_bytes <= ctx->budget);
+    const bool staged = persistent || two_stage;
     Arena a;
     const size_t oa = a.take<float2>(n), ob = a.take<float2>(n);
     const size_t oh = staged ? a.take<float2>(n) : 0, ohi = staged ? a.take<float2>(n) : 0;
@@ -1657,13 +1733,10 @@ int32_t ph_phase_retrieval(ph_ctx *ctx, void *out, const float *holo1, const flo
     if (residual) PH_CUDA(cudaMemsetAsync(acc, 0, 2 * sizeof(double), s), "memset");
     const float scale = (float)(1.0 / ((double)nx * (double)ny));
     if (staged) {
-        dim3 tb(32, 8), tg((nx + 31) / 32, (ny + 31) / 32);
-        k_transfer_rows<<<tg, tb, 0, s>>>(ht, static_cast<const float2 *>(transfer), nx, ny, scale);
-        k_transfer_rows<<<tg, tb, 0, s>>>(hti, static_cast<const float2 *>(invtransfer), nx, ny, scale);
-        // the amplitudes sqrt(I1), sqrt(I2) once per call, as the row passes would form them
-        k_sqrt_f32<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(amp1, holo1, n);
-        k_sqrt_f32<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(amp2, holo2, n);
-        PH_TRY(launched(ctx, cudaGetLastError(), "transfer rows and amplitudes", 4));
+        const GsSetup g{{static_cast<const float2 *>(transfer), static_cast<const float2 *>(invtransfer)},
+                        {ht, hti}, {holo1, holo2}, {amp1, amp2}};
+        k_gs_setup<<<dim3((nx + 31) / 32, (ny + 31) / 32, 2), 256, 0, s>>>(g, nx, ny, scale);
+        PH_TRY(launched(ctx, cudaGetLastError(), "transfer rows and amplitudes"));
     }
 
     FwdRowsT<FWD_SQRT_REAL> f{};
@@ -1672,6 +1745,26 @@ int32_t ph_phase_retrieval(ph_ctx *ctx, void *out, const float *holo1, const flo
     f.tw = tw_x;
     f.nrows = ny;
     PH_TRY(pass(ctx, s, "fwd_rows",[&] { return launch_fwd_rows(nx, f, s); }));
+    for (int it = 0; it < priter && two_stage; ++it) {
+        const bool last = it == priter - 1;
+        two::GsParams c{};
+        c.src = bufa; c.ht = ht; c.dst = bufb; c.tw = tw_y; c.nrows = nx;
+        PH_TRY(pass(ctx, s, "gs_col", [&] { return launch_gs_two_col(ny, c, s); }));
+        two::GsParams r{};
+        r.src = bufb; r.amp = amp2; r.dst = bufa; r.tw = tw_x; r.nrows = ny;
+        r.resid = (last && residual) ? acc : nullptr;
+        PH_TRY(pass(ctx, s, "gs_row_mid", [&] { return launch_gs_two_row(nx, r, s); }));
+        c.ht = hti;
+        PH_TRY(pass(ctx, s, "gs_col", [&] { return launch_gs_two_col(ny, c, s); }));
+        r.amp = amp1;
+        r.resid = nullptr;
+        if (!last) {
+            PH_TRY(pass(ctx, s, "gs_row_mid", [&] { return launch_gs_two_row(nx, r, s); }));
+        } else {
+            r.dst = o;
+            PH_TRY(pass(ctx, s, "gs_row_final", [&] { return launch_gs_two_final(nx, r, s); }));
+        }
+    }
     // The staged passes store through tensor maps where their blocks allow it:
     // the column pass writes bufb = [ny][nx], the row pass bufa = [nx][ny].
     CUtensorMap tm_col, tm_row;
@@ -1683,7 +1776,7 @@ int32_t ph_phase_retrieval(ph_ctx *ctx, void *out, const float *holo1, const flo
     const auto row = [&](const GsRowMidT &r) {
         return ts_row ? launch_gs_row_ts(nx, r, tm_row, s) : launch_gs_row_t(nx, r, s);
     };
-    for (int it = 0; it < priter && staged; ++it) {
+    for (int it = 0; it < priter && persistent; ++it) {
         const bool last = it == priter - 1;
         GsColT c{};
         c.src = bufa; c.ht = ht; c.dst = bufb; c.tw = tw_y; c.err = err; c.nx = nx;
@@ -1752,6 +1845,24 @@ int32_t ph_asm_prop(ph_ctx *ctx, void *out, const void *in, const float *d_sqr, 
     PH_TRY(get_twiddles(ctx, ny, s, &tw_y));
     float2 *h = at<float2>(ctx, oh);
     const double c = (2.0 * M_PI * zprop) / wavlen;
+    if (gs_two(nx) && gs_two(ny)) {   // the transfer formed as the rows that the column pass multiplies by
+        float2 *bufa = at<float2>(ctx, oa), *bufb = at<float2>(ctx, ob);
+        k_transfer_rows<<<dim3((nx + 31) / 32, (ny + 31) / 32), 256, 0, s>>>(
+            h, d_sqr, nx, ny, (float)(1.0 / ((double)nx * (double)ny)), turn_rate(c), ctx->phase_tab);
+        PH_TRY(launched(ctx, cudaGetLastError(), "transfer rows"));
+        FwdRowsT<FWD_COMPLEX> f{};
+        f.src = static_cast<const float2 *>(in);
+        f.dst = bufa;
+        f.tw = tw_x;
+        f.nrows = ny;
+        PH_TRY(pass(ctx, s, "fwd_rows", [&] { return launch_fwd_rows(nx, f, s); }));
+        two::GsParams g{};
+        g.src = bufa; g.ht = h; g.dst = bufb; g.tw = tw_y; g.nrows = nx;
+        PH_TRY(pass(ctx, s, "gs_col", [&] { return launch_gs_two_col(ny, g, s); }));
+        g.src = bufb; g.dst = static_cast<float2 *>(out); g.tw = tw_x; g.nrows = ny;
+        PH_TRY(pass(ctx, s, "inv_rows", [&] { return launch_gs_two_inv(nx, g, s); }));
+        PH_LEAVE(ctx);
+    }
     PH_TRY(launched(ctx, transfer_launch(h, d_sqr, n, c, ctx->phase_tab, s), "transfer"));
     PH_TRY(issue_propagate(ctx, static_cast<float2 *>(out), static_cast<const float2 *>(in), h, nullptr, nx, ny,
                            at<float2>(ctx, oa), at<float2>(ctx, ob), tw_x, tw_y, s));

@@ -266,6 +266,26 @@ cudaError_t launch_gs_row_t(int n, const GsRowMidT &b, cudaStream_t s);
 // The last plane-1 pass (dst = [ny][nx], natural order), persistent.
 cudaError_t launch_gs_row_final_t(int n, const GsRowMidT &b, cudaStream_t s);
 cudaError_t launch_gs_col_t(int n, const GsColT &b, cudaStream_t s);
+// The passes of phase retrieval and propagation on the two-stage transform
+// (ph_two_gs.cuh), programmatic dependents of the launch before: columns (times ht),
+// rows (amplitude replacement; with resid the FP64 residual too), the last row
+// pass of a call and a plain inverse row pass (natural stores).
+namespace two {
+struct GsParams {
+    const float2 *src;     // rows of length N
+    const float2 *ht;      // GS_COL: [row][N], scale included
+    const float *amp;      // GS_ROW, GS_ROW_FINAL: [row][N] amplitudes
+    float2 *dst;           // transposed [N][nrows], or natural
+    const float2 *tw;
+    double *resid;         // RESID: [0] += (|u| - amp)^2, [1] += amp^2
+    int nrows;
+};
+}  // namespace two
+bool gs_two(int n);
+cudaError_t launch_gs_two_col(int n, const two::GsParams &p, cudaStream_t s);
+cudaError_t launch_gs_two_row(int n, const two::GsParams &p, cudaStream_t s);
+cudaError_t launch_gs_two_final(int n, const two::GsParams &p, cudaStream_t s);
+cudaError_t launch_gs_two_inv(int n, const two::GsParams &p, cudaStream_t s);
 // Split-precision tensor-core pass B (ph_pass_tc.cuh) for the projection.
 struct ReconBTc;
 bool recon_b_tc_supported(int n, int form);

@@ -121,8 +121,9 @@ __device__ __forceinline__ void bfly(float2 (&v)[R]) {
 }
 
 // R = P Q: n = Q n1 + n2, k = k1 + P k2.
+__host__ __device__ constexpr int split_p_of(int r) { return r == 64 || r % 24 == 0 ? 8 : 4; }
 template <int R>
-constexpr int split_p() { return R == 64 || R % 24 == 0 ? 8 : 4; }
+constexpr int split_p() { return split_p_of(R); }
 template <int R>
 constexpr int split_q() { return R / split_p<R>(); }
 
@@ -180,6 +181,15 @@ __host__ __device__ constexpr bool supported(int n) {
            n == 2048 || n == 3072 || n == 4096;
 }
 
+// A length's table in global memory holds, behind the row engine's (ph_fft.cuh),
+// the stage factors of the transform L-major, [factor][l]: W^(l p), p = 1 .. P - 1,
+// then W^(l P q), q = 1 .. Q - 1; and those of its mirror (below), [factor][t], with
+// E and L exchanged.
+__host__ __device__ constexpr int factors_of(int r, int lanes) { return (split_p_of(r) + r / split_p_of(r) - 2) * lanes; }
+__host__ __device__ constexpr int factors_offset(int n) { return plan_tw_size(n, engine_e(n, PassBase::EPT)); }
+__host__ __device__ constexpr int mirror_offset(int n) { return factors_offset(n) + factors_of(values(n), n / values(n)); }
+__host__ __device__ constexpr int table_size(int n) { return mirror_offset(n) + factors_of(n / values(n), values(n)); }
+
 template <int N>
 struct Plan {
     static constexpr int E = values(N), L = N / E, M = (E + L - 1) / L;
@@ -216,13 +226,14 @@ struct Factors {
 #pragma unroll
         for (int q = 1; q < PL::Q; ++q) b[q] = tab[(PL::P - P0 + q - 1) * H * PL::L];
     }
-    // the same from the W^i table
+    // the same from the length's table (two_factors: forward, [factor][l])
     __device__ __forceinline__ void load_global(const float2 *__restrict__ tw, int l) {
         static_assert(H == 1, "whole transforms");
+        tw += factors_offset(N) + l;
 #pragma unroll
-        for (int p = 1; p < PL::P; ++p) a[p] = load_tw<INV>(tw, l * p);
+        for (int p = 1; p < PL::P; ++p) a[p] = load_tw<INV>(tw, (p - 1) * PL::L);
 #pragma unroll
-        for (int q = 1; q < PL::Q; ++q) b[q] = load_tw<INV>(tw, l * q * PL::P);
+        for (int q = 1; q < PL::Q; ++q) b[q] = load_tw<INV>(tw, (PL::P + q - 2) * PL::L);
     }
     // v times the twiddle of output k
     __device__ __forceinline__ float2 apply(int k, float2 v) const {
@@ -276,6 +287,72 @@ __device__ __forceinline__ void exchange(const float2 (&v)[Plan<N>::E], float2 (
             u[m * PL::L + i + 3].y = q.w;
         }
     }
+}
+
+// ---------------------------------------------------------------- the mirrored transform
+
+// The outputs of a transform sit as its mirror's inputs: thread t holds x[t' + E i],
+// t' = t + L m (m < M), i < L.  Stage 1: transforms of length L over i, times
+// W_N^(t' q1).  Exchange through rows q1 of E words (pitch E + 4).  Stage 2: thread
+// t = q1 holds the E values t' and transforms them: output q2 is X[q1 + L q2].  So
+// two transforms with a product between them need one exchange each.
+template <int N>
+struct Mirror {
+    using PL = Plan<N>;
+    static constexpr int PITCH = PL::E + 4;
+    // words of a row's region for both exchanges; two rows of one warp 16 banks apart
+    static constexpr int WORDS = cmax(PL::E * PL::PITCH, PL::L * PITCH);
+    static constexpr int XWORDS = PL::L == 16 ? (WORDS + 31) / 32 * 32 + 16 : WORDS;
+    static constexpr int P = split_p<PL::L>(), Q = split_q<PL::L>();
+};
+template <int N, bool INV>
+struct MirrorFactors {
+    using MR = Mirror<N>;
+    float2 a[MR::P], b[MR::Q];
+    __device__ __forceinline__ void load_global(const float2 *__restrict__ tw, int t) {
+        constexpr int E = Plan<N>::E;
+        tw += mirror_offset(N) + t;
+#pragma unroll
+        for (int p = 1; p < MR::P; ++p) a[p] = load_tw<INV>(tw, (p - 1) * E);
+#pragma unroll
+        for (int q = 1; q < MR::Q; ++q) b[q] = load_tw<INV>(tw, (MR::P + q - 2) * E);
+    }
+    __device__ __forceinline__ float2 apply(int k, float2 v) const {
+        const int p = k % MR::P, q = k / MR::P;
+        if (p == 0 && q == 0) return v;
+        if (q == 0) return cmul2(v, a[p]);
+        if (p == 0) return cmul2(v, b[q]);
+        return cmul2(v, cmul2(a[p], b[q]));
+    }
+};
+// v[m L + q1] of thread t (t' = t + L m) -> y[t'] of thread q1.
+template <int N, class Sync>
+__device__ __forceinline__ void mirror_exchange(const float2 (&v)[Plan<N>::M * Plan<N>::L], float2 (&y)[Plan<N>::E],
+                                                float *ex, int t, const Sync &sync) {
+    using PL = Plan<N>;
+    constexpr int PITCH = Mirror<N>::PITCH;
+    const float *rd = ex + t * PITCH;
+    const auto half = [&](auto part) {
+        constexpr int c = decltype(part)::value;
+        sync();   // the region's last reads
+#pragma unroll
+        for (int m = 0; m < PL::M; ++m)
+            if (PL::M * PL::L == PL::E || t + PL::L * m < PL::E) {
+#pragma unroll
+                for (int q = 0; q < PL::L; ++q) ex[q * PITCH + t + PL::L * m] = c == 0 ? v[m * PL::L + q].x : v[m * PL::L + q].y;
+            }
+        sync();
+#pragma unroll
+        for (int i = 0; i < PL::E; i += 4) {
+            const float4 q = *reinterpret_cast<const float4 *>(rd + i);
+            (c == 0 ? y[i].x : y[i].y) = q.x;
+            (c == 0 ? y[i + 1].x : y[i + 1].y) = q.y;
+            (c == 0 ? y[i + 2].x : y[i + 2].y) = q.z;
+            (c == 0 ? y[i + 3].x : y[i + 3].y) = q.w;
+        }
+    };
+    half(std::integral_constant<int, 0>{});
+    half(std::integral_constant<int, 1>{});
 }
 
 // ---------------------------------------------------------------- tensor memory as thread-private storage

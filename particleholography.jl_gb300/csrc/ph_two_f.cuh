@@ -78,12 +78,19 @@ __global__ void __launch_bounds__(PassF<N>::THREADS, PassF<N>::CTAS) k_two_fwd(c
     const float2 mean = MODE == FWD_PADDED ? *p.pad_mean : make_float2(0.f, 0.f);
     float2 *stage = reinterpret_cast<float2 *>(ph_smem);
     float *ex = reinterpret_cast<float *>(ph_smem + C::STAGE + r * C::XB);
+    // (the square root's rare path is a branch: with each load beside its root, 32
+    // loads ran one after the other)
+    float real[MODE == FWD_SQRT_REAL ? PL::E : 1];
+    if constexpr (MODE == FWD_SQRT_REAL) {
+#pragma unroll
+        for (int i = 0; i < PL::E; ++i) real[i] = __ldg(src_real + (size_t)y * N + l + PL::L * i);
+    }
     const auto load = [&](int i) -> float2 {
         const int x = l + PL::L * i;
         if constexpr (MODE == FWD_COMPLEX) {
             return src[(size_t)y * N + x];
         } else if constexpr (MODE == FWD_SQRT_REAL) {
-            return make_float2(sqrtf(src_real[(size_t)y * N + x]), 0.f);
+            return make_float2(sqrtf(real[i]), 0.f);
         } else {
             const int yi = y - p.pad_off, xi = x - p.pad_off;
             return yi >= 0 && yi < p.ny_in && xi >= 0 && xi < p.nx_in ? src[(size_t)yi * p.nx_in + xi] : mean;

@@ -43,3 +43,28 @@ def test_rows_and_slices_at_the_edges(ph, cuda, nx, ny, slices):
     want = np.clip(np.abs(field.astype(np.complex128)) ** 2, 0.0, 1.0)
     assert rel_l2(to_np(vol), want) < TOL
     assert torch.equal(vproj, vol.amin(0))
+
+
+@pytest.mark.parametrize("n", [128, 192, 256, 384, 512, 768, 1536])
+@pytest.mark.parametrize("iters", [1, 3])
+def test_phase_retrieval(ph, cuda, n, iters):
+    rng = np.random.default_rng(n)
+    h1, h2 = (rng.uniform(0.1, 1.0, (n, n)).astype(np.float32) for _ in range(2))
+    d = ref.transfer_sqrt_arr(n, LAM, DX)
+    tf, tfi = ref.transfer(700.0, n, LAM, d), ref.transfer(-700.0, n, LAM, d)
+    got, res = ph.cu_phase_retrieval_holo(to_dev(h1, cuda), to_dev(h2, cuda), ph.CuTransfer(to_dev(tf, cuda)),
+                                          ph.CuTransfer(to_dev(tfi, cuda)), iters, n, return_residual=True)
+    want = ref.phase_retrieval_holo(h1, h2, tf, tfi, iters, n)
+    # the replacement divides by |u|: rounding of the transforms grows where the field is small
+    assert rel_l2(to_np(got.data), want) < 4 * iters * TOL
+    assert 0.0 < float(res) < 1.0
+
+
+@pytest.mark.parametrize("n", [128, 192, 384, 512, 768, 1024, 1536, 2048])
+def test_propagation(ph, cuda, n):
+    rng = np.random.default_rng(n)
+    u = (rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))).astype(np.complex64)
+    d = ref.transfer_sqrt_arr(n, LAM, DX)
+    out = ph.CuWavefront(torch.empty((n, n), dtype=torch.complex64, device=cuda))
+    ph.cu_asm_prop_(out, ph.CuWavefront(to_dev(u, cuda)), ph.CuTransferSqrtPart(to_dev(d, cuda)), 4321.0, n, LAM)
+    assert rel_l2(to_np(out.data), ref.asm_prop(u, d, 4321.0, n, LAM)) < TOL
