@@ -429,6 +429,7 @@ __global__ void k_ingest_u8(float *out, const uint8_t *frame, int rows, int cols
 }
 
 __global__ void k_proj_finish(const unsigned long long *p64, float *proj, int32_t *argmin, size_t n) {
+    grid_dependency_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const unsigned long long p = p64[i];
@@ -1041,8 +1042,7 @@ int reconstruct(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin, void 
              (const void *)hdz, ctx->scratch, (int)ctx->opt_loop_limit, (const void *)lpf, thr_bits, (void *)packed,
              (int)accumulate, first, effective_form(ctx, nx, ny) * 1000 + (tu ? tu->group_cap : 0));
     return run_graph(ctx, s, key, [&](cudaStream_t s) -> int {
-        PH_TRY(issue_spectrum(ctx, wf, hf, hdz, nx, ny, padded, nin_x, nin_y, at<float2>(ctx, L.a1), state, tw_x,
-                              tw_y, at<double>(ctx, L.acc), at<float2>(ctx, L.mean), s, nullptr, lpf));
+        // (before the passes, so that these follow one another as programmatic dependents)
         const size_t npix = (size_t)nx_out * ny_out;
         if (packed != nullptr) {
             if (!accumulate) {
@@ -1053,6 +1053,8 @@ int reconstruct(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin, void 
         } else if (want_proj) {
             PH_CUDA(cudaMemsetAsync(p64, 0xff, sizeof(unsigned long long) * npix, s), "memset");
         }
+        PH_TRY(issue_spectrum(ctx, wf, hf, hdz, nx, ny, padded, nin_x, nin_y, at<float2>(ctx, L.a1), state, tw_x,
+                              tw_y, at<double>(ctx, L.acc), at<float2>(ctx, L.mean), s, nullptr, lpf));
         return issue_recon_slices(ctx, kind, proj, argmin, vol, vol_dtype, nx, ny, nx_out, ny_out, x0, y0, slices,
                                   L.batch, state, t, p64, tw_x, tw_y, want_proj && packed == nullptr, s, threshold,
                                   first);
@@ -1222,8 +1224,8 @@ int issue_recon_slices(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin
     }
     if (want_proj && (proj != nullptr || argmin != nullptr)) {
         const size_t n = (size_t)nx_out * ny_out;
-        k_proj_finish<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(p64, proj, argmin, n);
-        PH_TRY(launched(ctx, cudaGetLastError(), "projection finish"));
+        PH_TRY(launched(ctx, launch_dependent(k_proj_finish, dim3((unsigned)((n + 255) / 256)), 256, 0, s, p64, proj, argmin,
+                                              n), "projection finish"));
     }
     return PH_OK;
 }
@@ -1356,6 +1358,9 @@ int issue_recon_group(ph_ctx *ctx, const std::vector<const ph_recon_item *> &its
     const size_t ib = group_item_bytes(ctx, nx, ny, smax);
     auto slot = [&](int i, size_t off) { return base + (size_t)i * ib + off; };
     const float2 *tw_x = ctx->tw[nx], *tw_y = ctx->tw[ny];
+    const size_t npix = (size_t)nx * ny;
+    for (int i = 0; i < G; ++i)
+        PH_CUDA(cudaMemsetAsync(slot(i, L.p64), 0xff, sizeof(unsigned long long) * npix, s), "cudaMemsetAsync");
     // forward rows (the wavefront sqrt(I) formed in the first stage for hologram items)
     if (its[0]->hologram != nullptr) {
         FwdRowsT<FWD_SQRT_REAL> f{};
@@ -1397,9 +1402,6 @@ int issue_recon_group(ph_ctx *ctx, const std::vector<const ph_recon_item *> &its
     c.scale = (float)(1.0 / ((double)nx * (double)ny));
     c.nitems = G;
     PH_TRY(pass(ctx, s, "spectrum", [&] { return launch_spectrum(ny, c, s); }, spectrum_launches(ny)));
-    const size_t npix = (size_t)nx * ny;
-    for (int i = 0; i < G; ++i)
-        PH_CUDA(cudaMemsetAsync(slot(i, L.p64), 0xff, sizeof(unsigned long long) * npix, s), "cudaMemsetAsync");
     const ph_tuning *tu = tuning_of(ctx, nx, ny);
     const int cap = tu ? tu->group_cap : 0;
     for (int k0 = 0; k0 < smax; k0 += L.batch) {
@@ -1447,9 +1449,9 @@ int issue_recon_group(ph_ctx *ctx, const std::vector<const ph_recon_item *> &its
         PH_TRY(pass(ctx, s, "recon_b", [&] { return launch_recon_b_group(nx, b, s); }));
     }
     for (int i = 0; i < G; ++i) {
-        k_proj_finish<<<(unsigned)((npix + 255) / 256), 256, 0, s>>>(
-            reinterpret_cast<const unsigned long long *>(slot(i, L.p64)), its[i]->proj, its[i]->argmin, npix);
-        PH_TRY(launched(ctx, cudaGetLastError(), "projection finish"));
+        PH_TRY(launched(ctx, launch_dependent(k_proj_finish, dim3((unsigned)((npix + 255) / 256)), 256, 0, s,
+                                              reinterpret_cast<const unsigned long long *>(slot(i, L.p64)), its[i]->proj,
+                                              its[i]->argmin, npix), "projection finish"));
     }
     return PH_OK;
 }

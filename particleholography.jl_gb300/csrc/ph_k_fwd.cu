@@ -7,7 +7,7 @@ template <int MODE>
 static cudaError_t fwd(int n, const FwdRowsT<MODE> &b, cudaStream_t s) {
     switch (n) {
 #define PH_TWO_CASE(N) \
-    case N: return two::launch_f<N>(two::k_two_fwd<N, MODE>, two::PassF<N>::SMEM, b, b.nrows, b.nitems, s);
+    case N: return two::launch_f<N, false>(two::k_two_fwd<N, MODE>, two::PassF<N>::SMEM, b, b.nrows, b.nitems, s);
         PH_FOR_EACH_N_TWO(PH_TWO_CASE)
 #undef PH_TWO_CASE
     }

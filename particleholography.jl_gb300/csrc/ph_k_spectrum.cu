@@ -7,6 +7,7 @@ namespace ph {
 // centred [ny][nx]: 32 x 32 tiles through shared memory.
 __global__ void __launch_bounds__(256) k_state(const SpectrumCols p) {
     __shared__ float4 tile[32][33];
+    grid_dependents_launch();
     const int z = blockIdx.z, tx = threadIdx.x % 32, ty = threadIdx.x / 32;
     const float2 *hf = p.nitems > 1 ? p.hf_items[z] : p.hf;
     const float2 *hdz = p.nitems > 1 ? p.hdz_items[z] : p.hdz;
@@ -21,6 +22,7 @@ __global__ void __launch_bounds__(256) k_state(const SpectrumCols p) {
         }
     }
     __syncthreads();
+    grid_dependency_wait();   // the transfers above are the caller's; a1 and the state are not
     const float2 *a1 = p.a1 + (size_t)z * p.a1_stride;
     float4 *state = p.state + (size_t)z * p.state_stride;
 #pragma unroll
@@ -40,14 +42,13 @@ cudaError_t launch_spectrum(int n, const SpectrumCols &b, cudaStream_t s) {
     cudaError_t e = cudaErrorInvalidValue;
     switch (n) {
 #define PH_TWO_CASE(N) \
-    case N: e = two::launch_f<N>(two::k_two_cols<N>, two::PassF<N>::RB * two::PassF<N>::XB, b, b.nx, b.nitems, s); break;
+    case N: e = two::launch_f<N, true>(two::k_two_cols<N>, two::PassF<N>::RB * two::PassF<N>::XB, b, b.nx, b.nitems, s); break;
         PH_FOR_EACH_N_TWO(PH_TWO_CASE)
 #undef PH_TWO_CASE
         default: return launch_engine_len<true>(n, b, b.nx, 1, s, b.nitems);
     }
     if (e != cudaSuccess) return e;
-    k_state<<<dim3((b.nx + 31) / 32, (b.ny + 31) / 32, b.nitems), 256, 0, s>>>(b);
-    return cudaGetLastError();
+    return launch_dependent(k_state, dim3((b.nx + 31) / 32, (b.ny + 31) / 32, b.nitems), 256, 0, s, b);
 }
 
 }  // namespace ph

@@ -24,6 +24,25 @@ inline bool supported_len(int n) {
     return n % 3 == 0 && ((n / 3) & (n / 3 - 1)) == 0 && n <= 6144;
 }
 
+// A launch as a programmatic dependent of the kernel before it on the stream: its
+// CTAs may start while that one finishes, and call grid_dependency_wait before they
+// touch anything that it, or a kernel before it, reads or writes.
+template <class... Params, class... Args>
+cudaError_t launch_dependent(void (*kern)(Params...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s,
+                             Args &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+}
+
 // Rows per CTA of the pass compiled for length n.
 inline int rows_per_cta(int n) {
     switch (n) {

@@ -211,8 +211,12 @@ struct Factors {
     static constexpr size_t BYTES = (size_t)COUNT * H * PL::L * 8;
     float2 a[PL::P], b[PL::Q];
     // The CTA's table [factor][h][l], so that a warp's loads are contiguous (from
-    // the W^i table they would be gathers of up to 32 lines).  tw: W_(H N)^i.
+    // the W^i table they would be gathers of up to 32 lines).  tw: the table of H N.
     __device__ __forceinline__ static void fill(float2 *tab, const float2 *__restrict__ tw) {
+        if constexpr (H == 1) {   // as it stands in the length's table
+            for (int i = threadIdx.x; i < COUNT * PL::L; i += blockDim.x) tab[i] = load_tw<INV>(tw, factors_offset(N) + i);
+            return;
+        }
         for (int i = threadIdx.x; i < COUNT * H * PL::L; i += blockDim.x) {
             const int l = i % PL::L, h = i / PL::L % H, j = i / (PL::L * H);
             const int e = j < PL::P - P0 ? H * (j + P0) + h : H * PL::P * (j - (PL::P - P0) + 1);
@@ -372,14 +376,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
           "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
         : "r"(taddr)
         : "memory");
-}
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[16]) {   // the first 8; the others are 0
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
-                 : "r"(taddr)
-                 : "memory");
-#pragma unroll
-    for (int i = 8; i < 16; ++i) v[i] = 0.0f;
 }
 // Waits for the loads issued so far; the values pass through it, so that no use moves above it.
 __device__ __forceinline__ void tmem_wait(float (&v)[16]) {

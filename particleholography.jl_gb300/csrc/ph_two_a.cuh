@@ -115,6 +115,7 @@ __global__ void __launch_bounds__(PassA<N>::THREADS, PassA<N>::CTAS)
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
+    grid_dependency_wait();   // the state is written, and T no longer read
     // columns of this warp; group n2 of the first butterflies: X of its P inputs, then Hdz of them
     const uint32_t tm = *slot + ((uint32_t)(warp & 3) << 21) + (uint32_t)(warp >> 2) * C::WCOLS;
     // (rows beyond nx transform row nx - 1 again; the tensor map drops their columns)
@@ -125,7 +126,7 @@ __global__ void __launch_bounds__(PassA<N>::THREADS, PassA<N>::CTAS)
         else named_bar_sync(2 + r, L);
     };
 
-    // f(i) over a group's inputs i = Q n1 + n2 -> tensor-memory columns at `at`
+    // a group's values (inputs i = Q n1 + n2) -> tensor-memory columns at `at`
     const auto put = [&](uint32_t at, const float2 (&t)[P]) {
         if constexpr (P == 4) {
             tmem_st8(at, t);
@@ -136,35 +137,15 @@ __global__ void __launch_bounds__(PassA<N>::THREADS, PassA<N>::CTAS)
             tmem_st16(at, q);
         }
     };
-    const auto get = [&](uint32_t at, float2 (&t)[P]) {
-        float q[16];
-        if constexpr (P == 4) tmem_ld8(at, q);
-        else tmem_ld16(at, q);
-        tmem_wait(q);
-#pragma unroll
-        for (int i = 0; i < P; ++i) t[i] = make_float2(q[2 * i], q[2 * i + 1]);
-    };
-#pragma unroll 1
-    for (int n2 = 0; n2 < Q; ++n2) {   // Hdz: the accurate sin/cos, as its error grows along the chain
-        float2 t[P];
-#pragma unroll
-        for (int n1 = 0; n1 < P; ++n1) {
-            const float4 st = srow[l + L * (Q * n1 + n2)];
-            float sn, cs;
-            sincospif((float)(int32_t)__float_as_uint(st.z) * 4.656612873077392578125e-10f, &sn, &cs);
-            const float mag = exp2f(st.w);
-            t[n1] = make_float2(cs * mag, sn * mag);
-        }
-        put(tm + n2 * 4 * P + 2 * P, t);
-    }
-
     const uint64_t policy = l2_evict_first();   // T is read by the next pass, long after
     for (int b = b0; b < b1; ++b) {
         tmem_wait_st();
         const uint32_t k = (uint32_t)(p.k0 + b), ahead = k % C::CHAIN;
-        if (ahead == 0 || b == b0) {
+        const bool first = b == b0;
+        if (first || ahead == 0) {
             // X at the last multiple of CHAIN, then the chain's own products: X_k does
-            // not depend on where a group or a range of slices starts
+            // not depend on where a group or a range of slices starts.  The first time
+            // also Hdz, by the accurate sin/cos, as its error grows along the chain.
             float4 st[P];
             const auto read = [&](int n2) {
 #pragma unroll
@@ -180,9 +161,16 @@ __global__ void __launch_bounds__(PassA<N>::THREADS, PassA<N>::CTAS)
                 float2 t[P];
 #pragma unroll
                 for (int n1 = 0; n1 < P; ++n1) t[n1] = ReconAT<GROUPED>::direct(cur[n1], k - ahead);
-                if (ahead != 0) {
+                if (first) {
                     float2 hd[P];
-                    get(tm + n2 * 4 * P + 2 * P, hd);
+#pragma unroll
+                    for (int n1 = 0; n1 < P; ++n1) {
+                        float sn, cs;
+                        sincospif((float)(int32_t)__float_as_uint(cur[n1].z) * 4.656612873077392578125e-10f, &sn, &cs);
+                        const float mag = exp2f(cur[n1].w);
+                        hd[n1] = make_float2(cs * mag, sn * mag);
+                    }
+                    put(tm + n2 * 4 * P + 2 * P, hd);
 #pragma unroll 1
                     for (uint32_t i = 0; i < ahead; ++i)
 #pragma unroll
@@ -296,8 +284,7 @@ cudaError_t launch_a(const ReconAT<GROUPED> &p, const CUtensorMap &tm, int group
     }
     const int gx = (p.nx + C::RB - 1) / C::RB;
     if (gx == 0 || groups == 0) return cudaSuccess;
-    kern<<<dim3(gx, groups, items), C::THREADS, C::SMEM, s>>>(p, tm);
-    return cudaGetLastError();
+    return launch_dependent(kern, dim3(gx, groups, items), C::THREADS, C::SMEM, s, p, tm);
 }
 
 }  // namespace two

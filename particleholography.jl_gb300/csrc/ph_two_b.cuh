@@ -79,6 +79,7 @@ __global__ void __launch_bounds__(128, PassB<N, EPI, GROUPED>::CTAS) k_two_b(con
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
+    grid_dependency_wait();   // T is written
     const uint32_t tm = C::MIN ? *slot + ((uint32_t)(warp & 3) << 21) : 0;
 
     // a warp whose rows all lie beyond the last row has nothing to do (rows are
@@ -292,8 +293,7 @@ cudaError_t launch_b(const ReconB<EPI, GROUPED> &p, int groups, int items, cudaS
     }
     const int gx = (p.rows + C::ROWS - 1) / C::ROWS;
     if (gx == 0 || groups == 0) return cudaSuccess;
-    kern<<<dim3(gx, groups, items), C::THREADS, C::SMEM, s>>>(p);
-    return cudaGetLastError();
+    return launch_dependent(kern, dim3(gx, groups, items), C::THREADS, C::SMEM, s, p);
 }
 
 }  // namespace two

@@ -69,6 +69,7 @@ __global__ void __launch_bounds__(PassF<N>::THREADS, PassF<N>::CTAS) k_two_fwd(c
     using C = PassF<N>;
     using PL = Plan<N>;
     extern __shared__ __align__(128) unsigned char ph_smem[];
+    grid_dependents_launch();
     const int z = blockIdx.z;
     const float2 *src = p.nitems > 1 ? p.src_items[z] : p.src;
     const float *src_real = p.nitems > 1 ? p.src_real_items[z] : p.src_real;
@@ -111,6 +112,8 @@ template <int N>
 __global__ void __launch_bounds__(PassF<N>::THREADS, PassF<N>::CTAS) k_two_cols(const SpectrumCols p) {
     using PL = Plan<N>;
     extern __shared__ __align__(128) unsigned char ph_smem[];
+    grid_dependents_launch();
+    grid_dependency_wait();
     const int r = threadIdx.x / PL::L, l = threadIdx.x % PL::L;
     const int kx = blockIdx.x * PassF<N>::RB + r;
     const bool valid = kx < p.nx;
@@ -123,7 +126,8 @@ __global__ void __launch_bounds__(PassF<N>::THREADS, PassF<N>::CTAS) k_two_cols(
         });
 }
 
-template <int N, class Kernel, class Params>
+// DEPENDENT: as a programmatic dependent (k_two_cols waits for the forward rows).
+template <int N, bool DEPENDENT, class Kernel, class Params>
 cudaError_t launch_f(Kernel kern, size_t smem, const Params &p, int nrows, int items, cudaStream_t s) {
     using C = PassF<N>;
     static_assert((C::SMEM + 1024) * C::CTAS <= 228 * 1024, "the CTAs of an SM share its shared memory");
@@ -140,6 +144,7 @@ cudaError_t launch_f(Kernel kern, size_t smem, const Params &p, int nrows, int i
     }
     const int gx = (nrows + C::RB - 1) / C::RB;
     if (gx == 0) return cudaSuccess;
+    if constexpr (DEPENDENT) return launch_dependent(kern, dim3(gx, 1, items), C::THREADS, smem, s, p);
     kern<<<dim3(gx, 1, items), C::THREADS, smem, s>>>(p);
     return cudaGetLastError();
 }

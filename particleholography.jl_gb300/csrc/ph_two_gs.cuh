@@ -165,17 +165,7 @@ cudaError_t launch_gs(const GsParams &p, cudaStream_t s) {
     }
     const int gx = (p.nrows + C::RB - 1) / C::RB;
     if (gx == 0) return cudaSuccess;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(gx);
-    cfg.blockDim = dim3(C::THREADS);
-    cfg.dynamicSmemBytes = C::SMEM;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, p);
+    return launch_dependent(kern, dim3(gx), C::THREADS, C::SMEM, s, p);
 }
 
 }  // namespace two
