@@ -1001,7 +1001,8 @@ struct SubArgs {
 int issue_recon_slices(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin, void *vol, int vol_dtype, int nx,
                        int ny, int nx_out, int ny_out, int x0, int y0, int slices, int batch, float4 *state, float2 *t,
                        unsigned long long *p64, const float2 *tw_x, const float2 *tw_y, bool want_proj,
-                       cudaStream_t s, float threshold = 0.0f, int first = 0, const SubArgs *sub = nullptr);
+                       cudaStream_t s, float threshold = 0.0f, int first = 0, const SubArgs *sub = nullptr,
+                       bool minima_only = false);
 
 // Shared driver of every reconstruction entry point.
 //
@@ -1033,6 +1034,18 @@ int reconstruct(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin, void 
         const unsigned char *tab = nullptr;
         PH_TRY(get_tc_table(ctx, nx, effective_form(ctx, nx, ny), s, &tab));
     }
+    // Where no slice is asked for and the two-stage row pass runs, pass B merges the
+    // minima straight into the caller's projection (every pixel gets one).  It is reset
+    // before the inputs are read, so not if it overlaps one of them.
+    const auto apart = [&](const void *in, size_t bytes) {
+        const char *p0 = reinterpret_cast<const char *>(proj), *q0 = static_cast<const char *>(in);
+        return in == nullptr || p0 + sizeof(float) * nx_out * ny_out <= q0 || q0 + bytes <= p0;
+    };
+    const size_t field = sizeof(float2) * nx * ny;
+    const bool minima_only =
+        proj != nullptr && argmin == nullptr && packed == nullptr && recon_b_ctas(nx, 1) > 0 &&
+        (kind == RK_PROJ ? effective_form(ctx, nx, ny) == PH_FORM_FP32 : kind == RK_VOL || kind == RK_PADDED) &&
+        apart(wf, sizeof(float2) * nin_x * nin_y) && apart(hf, field) && apart(hdz, field) && apart(lpf, field / 2);
     const ph_tuning *tu = tuning_of(ctx, nx, ny);
     char key[512];
     uint32_t thr_bits = 0;
@@ -1051,13 +1064,16 @@ int reconstruct(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin, void 
                 PH_TRY(launched(ctx, cudaGetLastError(), "packed fill"));
             }
         } else if (want_proj) {
-            PH_CUDA(cudaMemsetAsync(p64, 0xff, sizeof(unsigned long long) * npix, s), "memset");
+            if (minima_only)
+                PH_CUDA(cudaMemsetAsync(proj, 0xff, sizeof(float) * npix, s), "memset");
+            else
+                PH_CUDA(cudaMemsetAsync(p64, 0xff, sizeof(unsigned long long) * npix, s), "memset");
         }
         PH_TRY(issue_spectrum(ctx, wf, hf, hdz, nx, ny, padded, nin_x, nin_y, at<float2>(ctx, L.a1), state, tw_x,
                               tw_y, at<double>(ctx, L.acc), at<float2>(ctx, L.mean), s, nullptr, lpf));
         return issue_recon_slices(ctx, kind, proj, argmin, vol, vol_dtype, nx, ny, nx_out, ny_out, x0, y0, slices,
                                   L.batch, state, t, p64, tw_x, tw_y, want_proj && packed == nullptr, s, threshold,
-                                  first);
+                                  first, nullptr, minima_only);
     });
 }
 
@@ -1167,9 +1183,10 @@ bool t_store_map_items(CUtensorMap *tm, float2 *t, int nx, int ny, int nb, int n
 int issue_recon_slices(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin, void *vol, int vol_dtype, int nx,
                        int ny, int nx_out, int ny_out, int x0, int y0, int slices, int batch, float4 *state, float2 *t,
                        unsigned long long *p64, const float2 *tw_x, const float2 *tw_y, bool want_proj,
-                       cudaStream_t s, float threshold, int first, const SubArgs *sub) {
+                       cudaStream_t s, float threshold, int first, const SubArgs *sub, bool minima_only) {
     ReconLayout L{};
     L.batch = batch;
+    unsigned *p32 = minima_only ? reinterpret_cast<unsigned *>(proj) : nullptr;
     for (int k0 = first; k0 < first + slices; k0 += L.batch) {
         const int nb = std::min(L.batch, first + slices - k0);
         const ph_tuning *tu = tuning_of(ctx, nx, ny);
@@ -1195,7 +1212,8 @@ int issue_recon_slices(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin
             PH_TRY(pass(ctx, s, "recon_b_tc", [&] { return launch_recon_b_tc(nx, form, b, s); }));
         } else if (kind == RK_PROJ) {
             ReconB<EPI_PROJ> b{};
-            b.t = t; b.tw = tw_x; b.proj64 = p64; b.rows = ny_out; b.nx_out = nx_out; b.x0 = 0;
+            b.t = t; b.tw = tw_x; b.proj64 = minima_only ? nullptr : p64; b.proj32 = p32;
+            b.rows = ny_out; b.nx_out = nx_out; b.x0 = 0;
             b.k0 = k0; b.nbatch = nb; b.group = group_b; b.vol_slice_stride = (long long)nx_out * ny_out;
             b.err = static_cast<int *>(ctx->small);
             PH_TRY(pass(ctx, s, "recon_b",[&] { return launch_recon_b(nx, b, s); }));
@@ -1214,7 +1232,8 @@ int issue_recon_slices(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin
             PH_TRY(pass(ctx, s, "recon_b",[&] { return launch_recon_b(nx, b, s); }));
         } else {
             ReconB<EPI_VOL> b{};
-            b.t = t; b.tw = tw_x; b.vol = vol; b.vol_dtype = vol_dtype; b.proj64 = want_proj ? p64 : nullptr;
+            b.t = t; b.tw = tw_x; b.vol = vol; b.vol_dtype = vol_dtype;
+            b.proj64 = want_proj && !minima_only ? p64 : nullptr; b.proj32 = p32;
             b.threshold = threshold;
             b.rows = ny_out; b.nx_out = nx_out; b.x0 = x0;
             b.k0 = k0; b.nbatch = nb; b.group = group_b; b.vol_slice_stride = (long long)nx_out * ny_out;
@@ -1222,7 +1241,7 @@ int issue_recon_slices(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin
             PH_TRY(pass(ctx, s, "recon_b",[&] { return launch_recon_b(nx, b, s); }));
         }
     }
-    if (want_proj && (proj != nullptr || argmin != nullptr)) {
+    if (want_proj && !minima_only && (proj != nullptr || argmin != nullptr)) {
         const size_t n = (size_t)nx_out * ny_out;
         PH_TRY(launched(ctx, launch_dependent(k_proj_finish, dim3((unsigned)((n + 255) / 256)), 256, 0, s, p64, proj, argmin,
                                               n), "projection finish"));

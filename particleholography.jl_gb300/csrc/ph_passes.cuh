@@ -633,6 +633,7 @@ struct ReconB : PassBase, std::conditional_t<GROUPED, ReconItems, NoItems> {
     const float2 *t;                 // [batch][rows][nx]
     const float2 *tw;
     unsigned long long *proj64;      // [rows_out][nx_out] or null
+    unsigned *proj32;                // two-stage lengths, proj64 null: the minima alone, as float bits
     void *vol;                       // [S][rows_out][nx_out] or null
     int *err;                        // raised if a bulk-copy wait times out
     int vol_dtype;                   // PH_N0F8 .. PH_F64, or PH_BOOL: intensity <= threshold

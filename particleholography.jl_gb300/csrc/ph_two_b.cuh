@@ -25,7 +25,10 @@ namespace two {
 // 3 * 2^a: 768^2 x 256 0.247 ms (0.357), 1536^2 x 256 1.01 ms (1.35).
 // Measured slower: the stage factors read from the W^i table (gathers of up to
 // 32 lines: 3.77 ms at 2048) or held in registers across slices (spills).
-template <int N, int EPI, bool GROUPED>
+// SLICE: the slice of every minimum is kept and merged with it (64-bit words);
+// without it the minima alone go to proj32 as float bits: half the tensor memory,
+// and neither an unpacking kernel nor a 64-bit word per pixel.
+template <int N, int EPI, bool GROUPED, bool SLICE = true>
 struct PassB {
     static constexpr int H = N == 2048 || N == 1536 ? 2 : 1;         // transforms a row is split into
     using PL = Plan<N / H>;
@@ -35,16 +38,16 @@ struct PassB {
     static constexpr int CTAS = PL::E >= 48 ? 2 : 4;         // per SM: 255 registers at 48 and 64 values, 128 below
     static constexpr int CC = PL::M * PL::L;                 // outputs per thread (with the idle ones)
     static constexpr bool MIN = EPI == EPI_PROJ || EPI == EPI_VOL;
-    static constexpr uint32_t COLS = 2 * CC;                 // minima, then slices
+    static constexpr uint32_t COLS = SLICE || CC < 32 ? 2 * CC : CC;   // minima, then slices
     static constexpr size_t IN = (size_t)N * 8;
     static constexpr size_t XB = (size_t)PL::XWORDS * 4;
     using F = Factors<N / H, true, H>;
     static constexpr size_t SMEM = ROWS * (IN + H * XB) + F::BYTES + ROWS * 8 + 16;
 };
 
-template <int N, int EPI, bool GROUPED>
-__global__ void __launch_bounds__(128, PassB<N, EPI, GROUPED>::CTAS) k_two_b(const ReconB<EPI, GROUPED> p) {
-    using C = PassB<N, EPI, GROUPED>;
+template <int N, int EPI, bool GROUPED, bool SLICE>
+__global__ void __launch_bounds__(128, PassB<N, EPI, GROUPED, SLICE>::CTAS) k_two_b(const ReconB<EPI, GROUPED> p) {
+    using C = PassB<N, EPI, GROUPED, SLICE>;
     using PL = typename C::PL;
     constexpr int E = PL::E, L = PL::L, H = C::H, ROWS = C::ROWS;
     extern __shared__ __align__(128) unsigned char ph_smem[];
@@ -69,7 +72,7 @@ __global__ void __launch_bounds__(128, PassB<N, EPI, GROUPED>::CTAS) k_two_b(con
     const int r = threadIdx.x / C::TPR, h = threadIdx.x / L % H, l = threadIdx.x % L;
     const int y = blockIdx.x * ROWS + r;
     const bool valid = y < p.rows;
-    const bool track = EPI == EPI_PROJ || (EPI == EPI_VOL && proj64 != nullptr);
+    const bool track = EPI == EPI_PROJ || (EPI == EPI_VOL && (SLICE ? proj64 != nullptr : p.proj32 != nullptr));
     if constexpr (C::MIN) {
         if (warp == 0) tc::tmem_alloc(slot, C::COLS);
     }
@@ -111,7 +114,7 @@ __global__ void __launch_bounds__(128, PassB<N, EPI, GROUPED>::CTAS) k_two_b(con
 #pragma unroll
             for (int c = 0; c < C::CC; c += 16) {
                 tmem_st16(tm + c, inf);
-                tmem_st16(tm + C::CC + c, zero);
+                if constexpr (SLICE) tmem_st16(tm + C::CC + c, zero);
             }
             tmem_wait_st();
         }
@@ -211,15 +214,18 @@ __global__ void __launch_bounds__(128, PassB<N, EPI, GROUPED>::CTAS) k_two_b(con
                         if (track) {
                             float mv[16], mk[16];
                             tmem_ld16(tm + m * L + c, mv);
-                            tmem_ld16(tm + C::CC + m * L + c, mk);
+                            if constexpr (SLICE) tmem_ld16(tm + C::CC + m * L + c, mk);
                             tmem_wait(mv);
-                            tmem_wait(mk);
+                            if constexpr (SLICE) tmem_wait(mk);
 #pragma unroll
                             for (int i = 0; i < 16; ++i) {
-                                if (i2[i] < mv[i]) { mv[i] = i2[i]; mk[i] = __int_as_float(k); }
+                                if (i2[i] < mv[i]) {
+                                    mv[i] = i2[i];
+                                    if constexpr (SLICE) mk[i] = __int_as_float(k);
+                                }
                             }
                             tmem_st16(tm + m * L + c, mv);
-                            tmem_st16(tm + C::CC + m * L + c, mk);
+                            if constexpr (SLICE) tmem_st16(tm + C::CC + m * L + c, mk);
                         }
                     }
                 } else {
@@ -255,15 +261,18 @@ __global__ void __launch_bounds__(128, PassB<N, EPI, GROUPED>::CTAS) k_two_b(con
                 for (int c = 0; c < C::CC; c += 16) {
                     float mv[16], mk[16];
                     tmem_ld16(tm + c, mv);
-                    tmem_ld16(tm + C::CC + c, mk);
+                    if constexpr (SLICE) tmem_ld16(tm + C::CC + c, mk);
                     tmem_wait(mv);
-                    tmem_wait(mk);
+                    if constexpr (SLICE) tmem_wait(mk);
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
                         const int m = (c + i) / L, o = (c + i) % L;
                         const int xo = H * (l + L * m + E * o) + h - p.x0;
-                        if (valid && (PL::M * L == E || l + L * m < E) && xo >= 0 && xo < p.nx_out)
-                            atomicMin(proj64 + (size_t)y * p.nx_out + xo, pack_min(mv[i], __float_as_int(mk[i])));
+                        if (valid && (PL::M * L == E || l + L * m < E) && xo >= 0 && xo < p.nx_out) {
+                            const size_t at = (size_t)y * p.nx_out + xo;
+                            if constexpr (SLICE) atomicMin(proj64 + at, pack_min(mv[i], __float_as_int(mk[i])));
+                            else atomicMin(p.proj32 + at, __float_as_uint(mv[i]));   // (non-negative: ordered as bits)
+                        }
                     }
                 }
             }
@@ -277,11 +286,11 @@ __global__ void __launch_bounds__(128, PassB<N, EPI, GROUPED>::CTAS) k_two_b(con
     }
 }
 
-template <int N, int EPI, bool GROUPED>
-cudaError_t launch_b(const ReconB<EPI, GROUPED> &p, int groups, int items, cudaStream_t s) {
-    using C = PassB<N, EPI, GROUPED>;
+template <int N, int EPI, bool GROUPED, bool SLICE>
+cudaError_t launch_b_form(const ReconB<EPI, GROUPED> &p, int groups, int items, cudaStream_t s) {
+    using C = PassB<N, EPI, GROUPED, SLICE>;
     static_assert((C::SMEM + 1024) * C::CTAS <= 228 * 1024, "the CTAs of an SM share its shared memory");
-    auto kern = k_two_b<N, EPI, GROUPED>;
+    auto kern = k_two_b<N, EPI, GROUPED, SLICE>;
     static unsigned long long done_mask = 0;   // per-device opt-in to more than 48 KB of dynamic shared memory
     int dev = 0;
     cudaGetDevice(&dev);
@@ -294,6 +303,14 @@ cudaError_t launch_b(const ReconB<EPI, GROUPED> &p, int groups, int items, cudaS
     const int gx = (p.rows + C::ROWS - 1) / C::ROWS;
     if (gx == 0 || groups == 0) return cudaSuccess;
     return launch_dependent(kern, dim3(gx, groups, items), C::THREADS, C::SMEM, s, p);
+}
+
+template <int N, int EPI, bool GROUPED>
+cudaError_t launch_b(const ReconB<EPI, GROUPED> &p, int groups, int items, cudaStream_t s) {
+    if constexpr (!GROUPED && (EPI == EPI_PROJ || EPI == EPI_VOL)) {
+        if (p.proj64 == nullptr) return launch_b_form<N, EPI, GROUPED, false>(p, groups, items, s);
+    }
+    return launch_b_form<N, EPI, GROUPED, true>(p, groups, items, s);
 }
 
 }  // namespace two

@@ -39,6 +39,7 @@ def test_rows_and_slices_at_the_edges(ph, cuda, nx, ny, slices):
     p_ref, a_ref = ref.reconst_xyprojection(wave, hf, hdz, slices, with_argmin=True)
     assert rel_l2(to_np(proj), p_ref) < TOL
     assert np.mean(to_np(arg) == a_ref) >= 0.999
+    assert torch.equal(ph.cu_get_reconst_xyprojection(*args), proj)     # merged without the slices: the same minima
     vol, vproj = ph.cu_get_reconst_vol_and_xyprojection(*args, torch.float32)
     want = np.clip(np.abs(field.astype(np.complex128)) ** 2, 0.0, 1.0)
     assert rel_l2(to_np(vol), want) < TOL
