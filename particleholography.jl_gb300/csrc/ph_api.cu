@@ -237,33 +237,14 @@ __device__ __forceinline__ float2 transfer_value(float d, const TurnRate &a, con
     return make_float2(w.x + (w.y + fmaf(w.x, cs1, -w.z * sn)), w.z + (w.w + fmaf(w.z, cs1, w.x * sn)));
 }
 
-// VEC: four pixels per load (16-byte aligned arrays, n a multiple of 4).
-template <bool VEC>
-__global__ void __launch_bounds__(256)
-    k_transfer(float2 *out, const float *__restrict__ d_sqr, size_t n, const TurnRate a, const float4 *__restrict__ ptab) {
-    __shared__ float4 tab[kTurnTable];
-    tab[threadIdx.x] = __ldg(ptab + threadIdx.x * (kPhaseTable / kTurnTable));
-    __syncthreads();
-    const size_t step = (size_t)gridDim.x * 256, first = (size_t)blockIdx.x * 256 + threadIdx.x;
-    if constexpr (VEC) {
-        for (size_t i = first; i < n / 4; i += step) {
-            const float4 d = __ldg(reinterpret_cast<const float4 *>(d_sqr) + i);
-            const float2 v0 = transfer_value(d.x, a, tab), v1 = transfer_value(d.y, a, tab);
-            const float2 v2 = transfer_value(d.z, a, tab), v3 = transfer_value(d.w, a, tab);
-            reinterpret_cast<float4 *>(out)[2 * i] = make_float4(v0.x, v0.y, v1.x, v1.y);
-            reinterpret_cast<float4 *>(out)[2 * i + 1] = make_float4(v2.x, v2.y, v3.x, v3.y);
-        }
-    } else {
-        for (size_t i = first; i < n; i += step) out[i] = transfer_value(d_sqr[i], a, tab);
-    }
+// The stored planes keep the FP64 form: Float16 and N0f8 volumes carry a last bit of
+// theirs on.  (The fixed-point form serves propagation, which does not store the plane.)
+__global__ void __launch_bounds__(256) k_transfer(float2 *out, const float *d_sqr, size_t n, double c) {
+    const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+    if (i < n) out[i] = transfer_value_fp64(sqrtf(d_sqr[i]), c);
 }
-cudaError_t transfer_launch(float2 *out, const float *d_sqr, size_t n, double c, const float4 *ptab, cudaStream_t s) {
-    static_assert(kTurnTable == 256, "one table entry per thread");
-    const bool vec = n % 4 == 0 && (((uintptr_t)out | (uintptr_t)d_sqr) & 15) == 0;
-    const size_t work = vec ? n / 4 : n;
-    const unsigned g = (unsigned)std::min<size_t>((work + 255) / 256, 2048);
-    if (vec) k_transfer<true><<<g, 256, 0, s>>>(out, d_sqr, n, turn_rate(c), ptab);
-    else k_transfer<false><<<g, 256, 0, s>>>(out, d_sqr, n, turn_rate(c), ptab);
+cudaError_t transfer_launch(float2 *out, const float *d_sqr, size_t n, double c, cudaStream_t s) {
+    k_transfer<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(out, d_sqr, n, c);
     return cudaGetLastError();
 }
 
@@ -876,20 +857,50 @@ EncodeTiledFn encode_tiled() {
     return fn;
 }
 
+// Tensor map of a centred transfer [ny][nx] (8-byte elements) for the staged
+// spectrum pass: boxes of `rows` columns x 256 rows.
+bool tf_load_map(CUtensorMap *tm, const float2 *h, int nx, int ny, int rows) {
+    const EncodeTiledFn enc = encode_tiled();
+    if (enc == nullptr || ((uintptr_t)h & 15) != 0 || nx % 2 != 0 || rows < 2 || rows > 32) return false;
+    const cuuint64_t dims[2] = {(cuuint64_t)nx, (cuuint64_t)ny};
+    const cuuint64_t strides[1] = {(cuuint64_t)nx * 8};
+    const cuuint32_t box[2] = {(cuuint32_t)rows, 256};
+    const cuuint32_t estr[2] = {1, 1};
+    return enc(tm, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, const_cast<float2 *>(h), dims, strides, box, estr,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Which transform a reconstruction runs.  Projections, Float32, Float64, complex and
+// Boolean volumes (a Float32 volume compared) take the two-stage transform.  Outputs
+// that round the intensity to few bits (Float16, N0f8; padded and sub-volumes are N0f8)
+// stay on the row engine and keep their values: a last bit of Float32 that differs moves
+// whole steps of theirs, up to 2^-10 in a Float16 volume's projection.  (1024^2 x 27
+// Float16: 0.208 ms; Float32 volumes 1.4 .. 3.7 times faster than on the row engine.)
+enum ReconPath { PATH_ROWS, PATH_TWO };
+bool two_rows(ReconPath path, int n) { return path == PATH_TWO && recon_two(n); }
+
+// Forward rows of a reconstruction.
+template <int MODE>
+int fwd_rows(ph_ctx *ctx, int n, const FwdRowsT<MODE> &f, ReconPath path, cudaStream_t s) {
+    return pass(ctx, s, "fwd_rows",
+                [&] { return two_rows(path, n) ? launch_fwd_rows_two(n, f, s) : launch_fwd_rows(n, f, s); });
+}
+
 // Forward FFT of the (optionally mean-padded) wavefront and the spectrum state.
 // nx, ny: transform size; a1: scratch [nx][ny] complex.  With `holo` (and wf
 // NULL) the wavefront is sqrt(holo) + 0i, formed in the first FFT stage.
 int issue_spectrum(ph_ctx *ctx, const float2 *wf, const float2 *hf, const float2 *hdz, int nx, int ny,
                    bool padded, int nin_x, int nin_y, float2 *a1, float4 *state, const float2 *tw_x,
                    const float2 *tw_y, double *acc, float2 *mean, cudaStream_t s, const float *holo = nullptr,
-                   const float *lpf = nullptr) {
+                   const float *lpf = nullptr, ReconPath path = PATH_TWO) {
     if (holo != nullptr) {
         FwdRowsT<FWD_SQRT_REAL> f{};
         f.src_real = holo;
         f.dst = a1;
         f.tw = tw_x;
         f.nrows = ny;
-        PH_TRY(pass(ctx, s, "fwd_rows", [&] { return launch_fwd_rows(nx, f, s); }));
+        PH_TRY(fwd_rows(ctx, nx, f, path, s));
     } else if (padded) {
         PH_CUDA(cudaMemsetAsync(acc, 0, 2 * sizeof(double), s), "cudaMemsetAsync");
         k_sum_c64<<<256, 256, 0, s>>>(wf, (size_t)nin_x * nin_y, acc);
@@ -911,7 +922,7 @@ int issue_spectrum(ph_ctx *ctx, const float2 *wf, const float2 *hf, const float2
         f.dst = a1;
         f.tw = tw_x;
         f.nrows = ny;
-        PH_TRY(pass(ctx, s, "fwd_rows",[&] { return launch_fwd_rows(nx, f, s); }));
+        PH_TRY(fwd_rows(ctx, nx, f, path, s));
     }
     SpectrumCols c{};
     c.a1 = a1;
@@ -924,7 +935,22 @@ int issue_spectrum(ph_ctx *ctx, const float2 *wf, const float2 *hf, const float2
     c.nx = nx;
     c.ny = ny;
     c.scale = (float)(1.0 / ((double)nx * (double)ny));
-    PH_TRY(pass(ctx, s, "spectrum", [&] { return launch_spectrum(ny, c, s); }, spectrum_launches(ny)));
+    if (two_rows(path, ny)) {
+        PH_TRY(pass(ctx, s, "spectrum", [&] { return launch_spectrum_two(ny, c, s); }, 2));
+        return PH_OK;
+    }
+    // the transfers staged by tensor-map boxes where the lengths allow it
+    const int rows = spectrum_staged_rows(ny);
+    CUtensorMap tm_hf, tm_hdz;
+    if (lpf == nullptr && rows > 0 && nx % (2 * rows) == 0 &&
+        tf_load_map(&tm_hf, hf, nx, ny, rows) && tf_load_map(&tm_hdz, hdz, nx, ny, rows)) {
+        SpectrumColsT ct{};
+        static_cast<SpectrumCols &>(ct) = c;
+        ct.err = static_cast<int *>(ctx->small);
+        PH_TRY(pass(ctx, s, "spectrum", [&] { return launch_spectrum_staged(ny, ct, tm_hf, tm_hdz, s); }));
+        return PH_OK;
+    }
+    PH_TRY(pass(ctx, s, "spectrum", [&] { return launch_spectrum(ny, c, s); }));
     return PH_OK;
 }
 
@@ -1002,7 +1028,7 @@ int issue_recon_slices(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin
                        int ny, int nx_out, int ny_out, int x0, int y0, int slices, int batch, float4 *state, float2 *t,
                        unsigned long long *p64, const float2 *tw_x, const float2 *tw_y, bool want_proj,
                        cudaStream_t s, float threshold = 0.0f, int first = 0, const SubArgs *sub = nullptr,
-                       bool minima_only = false);
+                       bool minima_only = false, ReconPath path = PATH_TWO);
 
 // Shared driver of every reconstruction entry point.
 //
@@ -1042,10 +1068,17 @@ int reconstruct(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin, void 
         return in == nullptr || p0 + sizeof(float) * nx_out * ny_out <= q0 || q0 + bytes <= p0;
     };
     const size_t field = sizeof(float2) * nx * ny;
+    const bool merge32 = proj != nullptr && argmin == nullptr && packed == nullptr && apart(wf, field) &&
+                         apart(hf, field) && apart(hdz, field) && apart(lpf, field / 2);
+    // (a volume whose projection cannot be merged there keeps the row engine's 64-bit words)
+    const ReconPath path = kind == RK_PROJ || kind == RK_CVOL ||
+                                   (kind == RK_VOL && vol_dtype != PH_F16 && vol_dtype != PH_N0F8 &&
+                                    (merge32 || !want_proj))
+                               ? PATH_TWO
+                               : PATH_ROWS;
     const bool minima_only =
-        proj != nullptr && argmin == nullptr && packed == nullptr && recon_b_ctas(nx, 1) > 0 &&
-        (kind == RK_PROJ ? effective_form(ctx, nx, ny) == PH_FORM_FP32 : kind == RK_VOL || kind == RK_PADDED) &&
-        apart(wf, sizeof(float2) * nin_x * nin_y) && apart(hf, field) && apart(hdz, field) && apart(lpf, field / 2);
+        merge32 && two_rows(path, nx) &&
+        (kind == RK_PROJ ? effective_form(ctx, nx, ny) == PH_FORM_FP32 : kind == RK_VOL);
     const ph_tuning *tu = tuning_of(ctx, nx, ny);
     char key[512];
     uint32_t thr_bits = 0;
@@ -1070,19 +1103,17 @@ int reconstruct(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin, void 
                 PH_CUDA(cudaMemsetAsync(p64, 0xff, sizeof(unsigned long long) * npix, s), "memset");
         }
         PH_TRY(issue_spectrum(ctx, wf, hf, hdz, nx, ny, padded, nin_x, nin_y, at<float2>(ctx, L.a1), state, tw_x,
-                              tw_y, at<double>(ctx, L.acc), at<float2>(ctx, L.mean), s, nullptr, lpf));
+                              tw_y, at<double>(ctx, L.acc), at<float2>(ctx, L.mean), s, nullptr, lpf, path));
         return issue_recon_slices(ctx, kind, proj, argmin, vol, vol_dtype, nx, ny, nx_out, ny_out, x0, y0, slices,
                                   L.batch, state, t, p64, tw_x, tw_y, want_proj && packed == nullptr, s, threshold,
-                                  first, nullptr, minima_only);
+                                  first, nullptr, minima_only, path);
     });
 }
 
-// Slices one pass A / pass B CTA transforms: up to 32, fewer when the batch
-// would then leave pass A with less than about four CTAs per SM.  Where pass A
-// runs the product chain, up to 64 (half the chain starts, each an accurate
-// sin/cos per value) as long as pass A keeps at least 16 waves of CTAs: 1.2 %
-// faster per 2048^2 x 512 frame.  (A 64 cap without the wave condition made
-// 1024^2 x 256 frames 7 % slower: 5 waves, the last one nearly empty.)
+// Slices one pass A / pass B CTA of the row engine transforms: up to 32, fewer
+// when the batch would then leave pass A with less than about four CTAs per SM.
+// Where pass A runs the product chain, up to 64 (half the chain starts, each an
+// accurate sin/cos per value) as long as pass A keeps at least 16 waves of CTAs.
 int recon_group(int nbatch, int nx_rows_a, bool chain, int cap_override = 0) {
     if (cap_override > 0) return std::max(1, std::min(cap_override, nbatch));
     int dev = 0, sms = 0;
@@ -1121,15 +1152,18 @@ int rounds_group(int nbatch, int ctas, int per_sm, int start, int cap_override) 
 
 // Slices per CTA of pass A (rows kx of length ny) and of pass B (`items` frames
 // of rows y of length nx) over a batch of nbatch slices.
-int recon_group_a(int nbatch, int nx, int ny, int y0, int ny_out, int cap_override) {
-    if (recon_a_two(ny, y0, ny_out)) {
+bool two_a(ReconPath path, int ny, int y0, int ny_out) { return path == PATH_TWO && recon_a_two(ny, y0, ny_out); }
+bool tstore_a(int ny, int y0, int ny_out) { return recon_a_tstore(ny) && y0 == 0 && ny_out == ny; }
+int recon_group_a(ReconPath path, int nbatch, int nx, int ny, int y0, int ny_out, int cap_override) {
+    if (two_a(path, ny, y0, ny_out)) {
         const int box = recon_a_two_box(ny);
         return rounds_group(nbatch, (nx + box - 1) / box, recon_a_two_ctas_per_sm(ny), 3, cap_override);
     }
-    return recon_group(nbatch, (nx + recon_a_rows(ny) - 1) / recon_a_rows(ny), recon_a_chain(ny), cap_override);
+    return recon_group(nbatch, (nx + recon_a_rows(ny) - 1) / recon_a_rows(ny),
+                       recon_a_chain(ny, path == PATH_ROWS && tstore_a(ny, y0, ny_out)), cap_override);
 }
-int recon_group_b(int nbatch, int nx, int rows, int items, int group_a, int cap_override) {
-    const int ctas = recon_b_ctas(nx, rows) * items;
+int recon_group_b(ReconPath path, int nbatch, int nx, int rows, int items, int group_a, int cap_override) {
+    const int ctas = two_rows(path, nx) ? recon_b_ctas(nx, rows) * items : 0;
     return ctas > 0 ? rounds_group(nbatch, ctas, recon_b_ctas_per_sm(nx), 2, cap_override) : group_a;
 }
 
@@ -1144,6 +1178,19 @@ bool t_store_map(CUtensorMap *tm, float2 *t, int nx, int ny_out, int nb, int box
     const cuuint32_t estr[3] = {1, 1, 1};
     return enc(tm, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, t, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                box_kx == 8 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// The same for the row engine's tiled store: boxes of box_kx kx x 256 y x 1 slice.
+bool t_store_map_plain(CUtensorMap *tm, float2 *t, int nx, int ny_out, int nb, int box_kx) {
+    const EncodeTiledFn enc = encode_tiled();
+    if (enc == nullptr || ((uintptr_t)t & 15) != 0 || nx % 4 != 0 || box_kx < 4 || box_kx > 32) return false;
+    const cuuint64_t dims[3] = {(cuuint64_t)nx, (cuuint64_t)ny_out, (cuuint64_t)nb};
+    const cuuint64_t strides[2] = {(cuuint64_t)nx * 8, (cuuint64_t)nx * ny_out * 8};
+    const cuuint32_t box[3] = {(cuuint32_t)box_kx, (cuuint32_t)ReconATStore::kBoxY, 1};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    return enc(tm, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, t, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -1183,7 +1230,8 @@ bool t_store_map_items(CUtensorMap *tm, float2 *t, int nx, int ny, int nb, int n
 int issue_recon_slices(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin, void *vol, int vol_dtype, int nx,
                        int ny, int nx_out, int ny_out, int x0, int y0, int slices, int batch, float4 *state, float2 *t,
                        unsigned long long *p64, const float2 *tw_x, const float2 *tw_y, bool want_proj,
-                       cudaStream_t s, float threshold, int first, const SubArgs *sub, bool minima_only) {
+                       cudaStream_t s, float threshold, int first, const SubArgs *sub, bool minima_only,
+                       ReconPath path) {
     ReconLayout L{};
     L.batch = batch;
     unsigned *p32 = minima_only ? reinterpret_cast<unsigned *>(proj) : nullptr;
@@ -1191,15 +1239,23 @@ int issue_recon_slices(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin
         const int nb = std::min(L.batch, first + slices - k0);
         const ph_tuning *tu = tuning_of(ctx, nx, ny);
         const int cap = tu ? tu->group_cap : 0;
-        const int group = recon_group_a(nb, nx, ny, y0, ny_out, cap);
-        const int group_b = recon_group_b(nb, nx, ny_out, 1, group, cap);
+        const int group = recon_group_a(path, nb, nx, ny, y0, ny_out, cap);
+        const int group_b = recon_group_b(path, nb, nx, ny_out, 1, group, cap);
+        const auto fill_a = [&](auto &a) {
+            a.state = state; a.t = t; a.tw = tw_y; a.nx = nx; a.ny_out = ny_out; a.y0 = y0;
+            a.k0 = k0; a.nbatch = nb; a.group = group;
+            a.err = static_cast<int *>(ctx->small);
+        };
         ReconA a{};
-        a.state = state; a.t = t; a.tw = tw_y; a.nx = nx; a.ny_out = ny_out; a.y0 = y0;
-        a.k0 = k0; a.nbatch = nb; a.group = group;
-        a.err = static_cast<int *>(ctx->small);
+        fill_a(a);
         CUtensorMap tm;
-        if (recon_a_two(ny, y0, ny_out) && t_store_map(&tm, t, nx, ny_out, nb, recon_a_two_box(ny), recon_a_two_box_y(ny))) {
+        if (two_a(path, ny, y0, ny_out) && t_store_map(&tm, t, nx, ny_out, nb, recon_a_two_box(ny), recon_a_two_box_y(ny))) {
             PH_TRY(pass(ctx, s, "recon_a", [&] { return launch_recon_a_two(ny, a, tm, nb, s); }));
+        } else if (path == PATH_ROWS && tstore_a(ny, y0, ny_out) &&
+                   t_store_map_plain(&tm, t, nx, ny_out, nb, recon_a_tstore_box(ny))) {
+            ReconATStore at{};
+            fill_a(at);
+            PH_TRY(pass(ctx, s, "recon_a", [&] { return launch_recon_a_tstore(ny, at, tm, nb, s); }));
         } else {
             PH_TRY(pass(ctx, s, "recon_a", [&] { return launch_recon_a(ny, a, nb, s); }));
         }
@@ -1216,7 +1272,7 @@ int issue_recon_slices(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin
             b.rows = ny_out; b.nx_out = nx_out; b.x0 = 0;
             b.k0 = k0; b.nbatch = nb; b.group = group_b; b.vol_slice_stride = (long long)nx_out * ny_out;
             b.err = static_cast<int *>(ctx->small);
-            PH_TRY(pass(ctx, s, "recon_b",[&] { return launch_recon_b(nx, b, s); }));
+            PH_TRY(pass(ctx, s, "recon_b", [&] { return two_rows(path, nx) ? launch_recon_b_two(nx, b, s) : launch_recon_b(nx, b, s); }));
         } else if (kind == RK_SUB) {
             ReconB<EPI_SUB> b{};
             b.t = t; b.tw = tw_x; b.vol = vol; b.rows = ny_out; b.nx_out = nx_out; b.x0 = 0;
@@ -1229,7 +1285,7 @@ int issue_recon_slices(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin
             b.t = t; b.tw = tw_x; b.vol = vol; b.rows = ny_out; b.nx_out = nx_out; b.x0 = 0;
             b.k0 = k0; b.nbatch = nb; b.group = group_b; b.vol_slice_stride = (long long)nx_out * ny_out;
             b.err = static_cast<int *>(ctx->small);
-            PH_TRY(pass(ctx, s, "recon_b",[&] { return launch_recon_b(nx, b, s); }));
+            PH_TRY(pass(ctx, s, "recon_b", [&] { return two_rows(path, nx) ? launch_recon_b_two(nx, b, s) : launch_recon_b(nx, b, s); }));
         } else {
             ReconB<EPI_VOL> b{};
             b.t = t; b.tw = tw_x; b.vol = vol; b.vol_dtype = vol_dtype;
@@ -1238,7 +1294,7 @@ int issue_recon_slices(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin
             b.rows = ny_out; b.nx_out = nx_out; b.x0 = x0;
             b.k0 = k0; b.nbatch = nb; b.group = group_b; b.vol_slice_stride = (long long)nx_out * ny_out;
             b.err = static_cast<int *>(ctx->small);
-            PH_TRY(pass(ctx, s, "recon_b",[&] { return launch_recon_b(nx, b, s); }));
+            PH_TRY(pass(ctx, s, "recon_b", [&] { return two_rows(path, nx) ? launch_recon_b_two(nx, b, s) : launch_recon_b(nx, b, s); }));
         }
     }
     if (want_proj && !minima_only && (proj != nullptr || argmin != nullptr)) {
@@ -1259,7 +1315,7 @@ int issue_propagate(ph_ctx *ctx, float2 *out, const float2 *in, const float2 *h,
     f.dst = bufa;
     f.tw = tw_x;
     f.nrows = ny;
-    PH_TRY(pass(ctx, s, "fwd_rows",[&] { return launch_fwd_rows(nx, f, s); }));
+    PH_TRY(fwd_rows(ctx, nx, f, PATH_TWO, s));
     GsCol c{};
     c.src = bufa;
     c.h = h;
@@ -1343,7 +1399,7 @@ int serve_transfer(ph_server *srv, cudaStream_t ls, float *dsqr, int nx, int ny,
         }
         PH_TRY(launched(ctx, transfer_sqrt_launch(dsqr, nx, ny, wavlen, dx, ls), "serve transfer"));
         const size_t n = (size_t)nx * ny;
-        PH_TRY(launched(ctx, transfer_launch(e.buf, dsqr, n, (2.0 * M_PI * (-z)) / wavlen, ctx->phase_tab, ls),
+        PH_TRY(launched(ctx, transfer_launch(e.buf, dsqr, n, (2.0 * M_PI * (-z)) / wavlen, ls),
                         "serve transfer"));
         PH_CUDA(cudaEventRecord(e.ready, ls), "cudaEventRecord");
         it = srv->tfs.emplace(key, e).first;
@@ -1390,7 +1446,7 @@ int issue_recon_group(ph_ctx *ctx, const std::vector<const ph_recon_item *> &its
         f.tw = tw_x;
         f.nrows = ny;
         f.nitems = G;
-        PH_TRY(pass(ctx, s, "fwd_rows", [&] { return launch_fwd_rows(nx, f, s); }));
+        PH_TRY(fwd_rows(ctx, nx, f, PATH_TWO, s));
     } else {
         FwdRowsT<FWD_COMPLEX> f{};
         f.src = static_cast<const float2 *>(its[0]->wavefront);
@@ -1400,7 +1456,7 @@ int issue_recon_group(ph_ctx *ctx, const std::vector<const ph_recon_item *> &its
         f.tw = tw_x;
         f.nrows = ny;
         f.nitems = G;
-        PH_TRY(pass(ctx, s, "fwd_rows", [&] { return launch_fwd_rows(nx, f, s); }));
+        PH_TRY(fwd_rows(ctx, nx, f, PATH_TWO, s));
     }
     SpectrumCols c{};
     c.a1 = reinterpret_cast<const float2 *>(slot(0, L.a1));
@@ -1420,7 +1476,8 @@ int issue_recon_group(ph_ctx *ctx, const std::vector<const ph_recon_item *> &its
     c.ny = ny;
     c.scale = (float)(1.0 / ((double)nx * (double)ny));
     c.nitems = G;
-    PH_TRY(pass(ctx, s, "spectrum", [&] { return launch_spectrum(ny, c, s); }, spectrum_launches(ny)));
+    if (recon_two(ny)) PH_TRY(pass(ctx, s, "spectrum", [&] { return launch_spectrum_two(ny, c, s); }, 2));
+    else PH_TRY(pass(ctx, s, "spectrum", [&] { return launch_spectrum(ny, c, s); }));
     const ph_tuning *tu = tuning_of(ctx, nx, ny);
     const int cap = tu ? tu->group_cap : 0;
     for (int k0 = 0; k0 < smax; k0 += L.batch) {
@@ -1428,9 +1485,9 @@ int issue_recon_group(ph_ctx *ctx, const std::vector<const ph_recon_item *> &its
         ReconB<EPI_PROJ, true> b{};
         for (int i = 0; i < G; ++i) {
             const int nb = std::max(0, std::min(L.batch, (int)its[i]->slices - k0));
-            const int grp = nb > 0 ? recon_group_a(nb, nx, ny, 0, ny, cap) : 1;
+            const int grp = nb > 0 ? recon_group_a(PATH_TWO, nb, nx, ny, 0, ny, cap) : 1;
             a.set_item(i, nb, grp);
-            b.set_item(i, nb, nb > 0 ? recon_group_b(nb, nx, ny, G, grp, cap) : 1);
+            b.set_item(i, nb, nb > 0 ? recon_group_b(PATH_TWO, nb, nx, ny, G, grp, cap) : 1);
         }
         a.state = reinterpret_cast<const float4 *>(slot(0, L.state));
         a.t = reinterpret_cast<float2 *>(slot(0, L.t));
@@ -1465,7 +1522,7 @@ int issue_recon_group(ph_ctx *ctx, const std::vector<const ph_recon_item *> &its
         b.vol_slice_stride = (long long)npix;
         b.nitems = G;
         b.err = static_cast<int *>(ctx->small);
-        PH_TRY(pass(ctx, s, "recon_b", [&] { return launch_recon_b_group(nx, b, s); }));
+        PH_TRY(pass(ctx, s, "recon_b", [&] { return recon_two(nx) ? launch_recon_b_group_two(nx, b, s) : launch_recon_b_group(nx, b, s); }));
     }
     for (int i = 0; i < G; ++i) {
         PH_TRY(launched(ctx, launch_dependent(k_proj_finish, dim3((unsigned)((npix + 255) / 256)), 256, 0, s,
@@ -1651,7 +1708,7 @@ int32_t ph_transfer(ph_ctx *ctx, void *out, const float *d_sqr, int32_t n_fast, 
     if (n_fast <= 0 || n_slow <= 0) { set_err(ctx, "sizes must be positive"); return PH_ERR_SIZE; }
     const size_t n = (size_t)n_fast * n_slow;
     const double c = (2.0 * M_PI * z0) / wavlen;
-    PH_TRY(launched(ctx, transfer_launch(static_cast<float2 *>(out), d_sqr, n, c, ctx->phase_tab, s), "transfer"));
+    PH_TRY(launched(ctx, transfer_launch(static_cast<float2 *>(out), d_sqr, n, c, s), "transfer"));
     PH_LEAVE(ctx);
 }
 
@@ -1765,7 +1822,7 @@ int32_t ph_phase_retrieval(ph_ctx *ctx, void *out, const float *holo1, const flo
     f.dst = bufa;
     f.tw = tw_x;
     f.nrows = ny;
-    PH_TRY(pass(ctx, s, "fwd_rows",[&] { return launch_fwd_rows(nx, f, s); }));
+    PH_TRY(fwd_rows(ctx, nx, f, PATH_TWO, s));
     for (int it = 0; it < priter && two_stage; ++it) {
         const bool last = it == priter - 1;
         two::GsParams c{};
@@ -1876,7 +1933,7 @@ int32_t ph_asm_prop(ph_ctx *ctx, void *out, const void *in, const float *d_sqr, 
         f.dst = bufa;
         f.tw = tw_x;
         f.nrows = ny;
-        PH_TRY(pass(ctx, s, "fwd_rows", [&] { return launch_fwd_rows(nx, f, s); }));
+        PH_TRY(fwd_rows(ctx, nx, f, PATH_TWO, s));
         two::GsParams g{};
         g.src = bufa; g.ht = h; g.dst = bufb; g.tw = tw_y; g.nrows = nx;
         PH_TRY(pass(ctx, s, "gs_col", [&] { return launch_gs_two_col(ny, g, s); }));
@@ -1884,7 +1941,7 @@ int32_t ph_asm_prop(ph_ctx *ctx, void *out, const void *in, const float *d_sqr, 
         PH_TRY(pass(ctx, s, "inv_rows", [&] { return launch_gs_two_inv(nx, g, s); }));
         PH_LEAVE(ctx);
     }
-    PH_TRY(launched(ctx, transfer_launch(h, d_sqr, n, c, ctx->phase_tab, s), "transfer"));
+    PH_TRY(launched(ctx, transfer_launch(h, d_sqr, n, c, s), "transfer"));
     PH_TRY(issue_propagate(ctx, static_cast<float2 *>(out), static_cast<const float2 *>(in), h, nullptr, nx, ny,
                            at<float2>(ctx, oa), at<float2>(ctx, ob), tw_x, tw_y, s));
     PH_LEAVE(ctx);
@@ -2142,9 +2199,9 @@ int32_t ph_autotune(ph_ctx *ctx, int32_t n_fast, int32_t n_slow, int32_t slices,
     }
     float2 *wf = buf, *hf = buf + n, *hdz = buf + 2 * n;
     if (transfer_sqrt_launch(dsqr, n_fast, n_slow, 0.6328, 10.0, s) != cudaSuccess ||
-        transfer_launch(wf, dsqr, n, (2.0 * M_PI * 3000.0) / 0.6328, ctx->phase_tab, s) != cudaSuccess ||
-        transfer_launch(hf, dsqr, n, (2.0 * M_PI * -1000.0) / 0.6328, ctx->phase_tab, s) != cudaSuccess ||
-        transfer_launch(hdz, dsqr, n, (2.0 * M_PI * -200.0) / 0.6328, ctx->phase_tab, s) != cudaSuccess) { cleanup(); return cuda_status(ctx, cudaErrorLaunchFailure, "tuning inputs"); }
+        transfer_launch(wf, dsqr, n, (2.0 * M_PI * 3000.0) / 0.6328, s) != cudaSuccess ||
+        transfer_launch(hf, dsqr, n, (2.0 * M_PI * -1000.0) / 0.6328, s) != cudaSuccess ||
+        transfer_launch(hdz, dsqr, n, (2.0 * M_PI * -200.0) / 0.6328, s) != cudaSuccess) { cleanup(); return cuda_status(ctx, cudaErrorLaunchFailure, "tuning inputs"); }
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -3058,11 +3115,11 @@ int32_t ph_reconst_subvolumes(ph_ctx *ctx, uint8_t *out, int64_t *offsets_host, 
     float4 *state = at<float4>(ctx, L.state);
     PH_TRY(issue_spectrum(ctx, static_cast<const float2 *>(wf), static_cast<const float2 *>(tf_front),
                           static_cast<const float2 *>(tf_dz), nx, ny, false, nx, ny, at<float2>(ctx, L.a1), state, tw_x,
-                          tw_y, at<double>(ctx, L.acc), at<float2>(ctx, L.mean), s));
+                          tw_y, at<double>(ctx, L.acc), at<float2>(ctx, L.mean), s, nullptr, nullptr, PATH_ROWS));
     const SubArgs sub{at<int>(ctx, o_rp), at<int>(ctx, o_rb), at<SubBox>(ctx, o_bx)};
     PH_TRY(issue_recon_slices(ctx, RK_SUB, nullptr, nullptr, out, PH_N0F8, nx, ny, nx, ny, 0, 0, nz, L.batch, state,
                               at<float2>(ctx, L.t), at<unsigned long long>(ctx, L.p64), tw_x, tw_y, false, s, 0.0f,
-                              zlo, &sub));
+                              zlo, &sub, false, PATH_ROWS));
     PH_LEAVE(ctx);
 }
 

@@ -1,7 +1,7 @@
 // Grouped launches of reconstruction passes A and B (projection): one launch
 // for up to kMaxItems holograms of one transform shape, grid z = item, grid y
 // = the largest item's slice groups (ph_passes.cuh, GROUPED forms).
-#include "ph_two_b.cuh"
+#include "ph_launch.cuh"
 
 namespace ph {
 
@@ -14,11 +14,6 @@ cudaError_t launch_recon_a_group(int n, const ReconAGrouped &b, cudaStream_t s) 
 cudaError_t launch_recon_b_group(int n, const ReconB<EPI_PROJ, true> &b, cudaStream_t s) {
     int gy = 1;
     for (int i = 0; i < b.nitems; ++i) gy = std::max(gy, (b.item_nb(i) + b.item_group(i) - 1) / b.item_group(i));
-    switch (n) {
-#define PH_TWO_CASE(N) case N: return two::launch_b<N>(b, gy, b.nitems, s);
-        PH_FOR_EACH_N_TWO(PH_TWO_CASE)
-#undef PH_TWO_CASE
-    }
     return launch_engine_len<false>(n, b, b.rows, gy, s, b.nitems);
 }
 

@@ -13,8 +13,8 @@ namespace ph {
     X(1) X(2) X(4) X(8) X(16) X(32) X(64) X(128) X(256) X(512) X(1024) X(2048) X(4096) X(8192) X(3) X(6) \
         X(12) X(24) X(48) X(96) X(192) X(384) X(768) X(1536) X(3072) X(6144)
 
-// The lengths whose pass B runs the row engine of ph_fft.cuh (the others run the
-// two-stage transform of ph_two.cuh).
+// The lengths without a two-stage transform (ph_two.cuh): projections and complex
+// volumes run the row engine's pass B at these alone.
 #define PH_FOR_EACH_N_ENGINE(X) \
     X(1) X(2) X(4) X(8) X(16) X(32) X(64) X(8192) X(3) X(6) X(12) X(24) X(48) X(96) X(6144)
 
@@ -190,6 +190,31 @@ cudaError_t launch_one_tm(const Body &body, const CUtensorMap &tm, int nrows, in
     return cudaLaunchKernelEx(&cfg, kern, body, tm);
 }
 
+// A plain launch of k_pass_tm2 (two tensor maps), one grid row.
+template <int N, bool ROW_FAST, class Body>
+cudaError_t launch_one_tm2(const Body &body, const CUtensorMap &tm0, const CUtensorMap &tm1, int nrows,
+                           cudaStream_t s) {
+    auto kern = k_pass_tm2<N, ROW_FAST, Body>;
+    constexpr size_t smem = Body::template smem<N, ROW_FAST>();
+    static_assert(smem <= kSmemMax, "pass needs more shared memory than a CTA has");
+    if constexpr (smem > 48 * 1024) {
+        static unsigned long long done_mask = 0;
+        int dev = 0;
+        cudaGetDevice(&dev);
+        const unsigned long long bit = 1ull << (dev & 63);
+        if (!(__atomic_load_n(&done_mask, __ATOMIC_ACQUIRE) & bit)) {
+            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            if (e != cudaSuccess) return e;
+            __atomic_fetch_or(&done_mask, bit, __ATOMIC_ACQ_REL);
+        }
+    }
+    using S = Shape<N, Body::EPT, Body::TT>;
+    const int gx = (nrows + S::ROWS - 1) / S::ROWS;
+    if (gx == 0) return cudaSuccess;
+    kern<<<gx, S::THREADS, smem, s>>>(body, tm0, tm1);
+    return cudaGetLastError();
+}
+
 // Launch of a pass that exists only for the lengths where Body::staged<N>() holds.
 template <bool ROW_FAST, class Body>
 cudaError_t launch_staged_len(int n, const Body &body, int nrows, cudaStream_t s) {
@@ -241,21 +266,43 @@ cudaError_t launch_engine_len(int n, const Body &body, int nrows, int grid_y, cu
 cudaError_t launch_fwd_rows(int n, const FwdRowsT<FWD_COMPLEX> &b, cudaStream_t s);
 cudaError_t launch_fwd_rows(int n, const FwdRowsT<FWD_SQRT_REAL> &b, cudaStream_t s);
 cudaError_t launch_fwd_rows(int n, const FwdRowsT<FWD_PADDED> &b, cudaStream_t s);
-cudaError_t launch_spectrum(int n, const SpectrumCols &b, cudaStream_t s);   // overwrites a1 at the two-stage lengths
-int spectrum_launches(int n);   // its kernels
+cudaError_t launch_spectrum(int n, const SpectrumCols &b, cudaStream_t s);
+// The spectrum pass with staged transfers (lengths 512 .. 2048; spectrum_staged_rows
+// gives the rows per CTA, 0 elsewhere); tm_hf, tm_hdz: the centred transfers
+// as [n_slow][n_fast] 8-byte elements, boxes of rows x 256.
+int spectrum_staged_rows(int n);
+cudaError_t launch_spectrum_staged(int n, const SpectrumColsT &b, const CUtensorMap &tm_hf, const CUtensorMap &tm_hdz,
+                                   cudaStream_t s);
 cudaError_t launch_recon_a(int n, const ReconA &b, int nbatch, cudaStream_t s);
-// Pass A on the two-stage transform with the tensor-map store (ph_two_a.cuh):
-// lengths 128 .. 4096, frames whose stored rows [y0, y0 + ny_out) are whole
-// boxes.  tm: T as (kx, y, slice) or, grouped, (kx, y, slice, item), 8-byte
-// elements, boxes of recon_a_two_box(n) kx x recon_a_two_box_y(n) y, swizzled by
-// the box's row of kx.  Its CTAs per SM.
+// Pass A with the tensor-map transposed store (lengths where recon_a_tstore holds;
+// tm: T as [nbatch][ny_out = n][nx] 8-byte elements, boxes of 4 x 256 x 1).
+bool recon_a_tstore(int n);
+int recon_a_tstore_box(int n);   // kx per box (rows per CTA x CTAs per cluster)
+cudaError_t launch_recon_a_tstore(int n, const ReconATStore &b, const CUtensorMap &tm, int nbatch, cudaStream_t s);
+cudaError_t launch_recon_a_group(int n, const ReconAGrouped &b, cudaStream_t s);
+// The two-stage forms of the reconstruction's passes (ph_two_*.cuh; lengths where
+// recon_two holds).  Forward rows; the spectrum (two kernels; overwrites a1).
+bool recon_two(int n);
+cudaError_t launch_fwd_rows_two(int n, const FwdRowsT<FWD_COMPLEX> &b, cudaStream_t s);
+cudaError_t launch_fwd_rows_two(int n, const FwdRowsT<FWD_SQRT_REAL> &b, cudaStream_t s);
+cudaError_t launch_spectrum_two(int n, const SpectrumCols &b, cudaStream_t s);
+// Pass A: frames whose stored rows [y0, y0 + ny_out) are whole boxes.  tm: T as
+// (kx, y, slice) or, grouped, (kx, y, slice, item), 8-byte elements, boxes of
+// recon_a_two_box(n) kx x recon_a_two_box_y(n) y, swizzled by the box's row of kx.
+// Its CTAs per SM.
 bool recon_a_two(int n, int y0, int ny_out);
 int recon_a_two_box(int n);
 int recon_a_two_box_y(int n);
 int recon_a_two_ctas_per_sm(int n);
 cudaError_t launch_recon_a_two(int n, const ReconA &b, const CUtensorMap &tm, int nbatch, cudaStream_t s);
 cudaError_t launch_recon_a_group_two(int n, const ReconAGrouped &b, const CUtensorMap &tm, cudaStream_t s);
-cudaError_t launch_recon_a_group(int n, const ReconAGrouped &b, cudaStream_t s);
+// Pass B: its CTAs per slice group over `rows` rows, and per SM (0 at other lengths).
+int recon_b_ctas(int n, int rows);
+int recon_b_ctas_per_sm(int n);
+cudaError_t launch_recon_b_two(int n, const ReconB<EPI_PROJ> &b, cudaStream_t s);
+cudaError_t launch_recon_b_two(int n, const ReconB<EPI_VOL> &b, cudaStream_t s);
+cudaError_t launch_recon_b_two(int n, const ReconB<EPI_CVOL> &b, cudaStream_t s);
+cudaError_t launch_recon_b_group_two(int n, const ReconB<EPI_PROJ, true> &b, cudaStream_t s);
 // The persistent GS passes with the tensor-map store (lengths where
 // gs_tstore_len holds; tm: dst as a 2-D tensor of 8-byte elements, inner
 // dimension the rows' index, boxes of rows-per-block x 256).
@@ -265,11 +312,8 @@ cudaError_t launch_gs_col_ts(int n, const GsColT &b, const CUtensorMap &tm, cuda
 cudaError_t launch_gs_row_ts(int n, const GsRowMidT &b, const CUtensorMap &tm, cudaStream_t s);
 cudaError_t launch_recon_b_group(int n, const ReconB<EPI_PROJ, true> &b, cudaStream_t s);
 int recon_a_rows(int n);   // rows per pass A CTA for transform length n
-bool recon_a_chain(int n);   // whether the row engine's pass A at length n advances X by the product chain
-// Pass B at 128 .. 4096 runs the two-stage transform (ph_two_b.cuh): its CTAs
-// per slice group over `rows` rows, and per SM (0 at the other lengths).
-int recon_b_ctas(int n, int rows);
-int recon_b_ctas_per_sm(int n);
+bool recon_a_chain(int n, bool tstore = false);   // whether pass A at length n (in the tensor-map
+                                                  // store form) advances X by the product chain
 cudaError_t launch_recon_b(int n, const ReconB<EPI_PROJ> &b, cudaStream_t s);
 cudaError_t launch_recon_b(int n, const ReconB<EPI_VOL> &b, cudaStream_t s);
 cudaError_t launch_recon_b(int n, const ReconB<EPI_CVOL> &b, cudaStream_t s);

@@ -155,6 +155,17 @@ __global__ void __launch_bounds__(Shape<N, Body::EPT, Body::TT>::THREADS, min_bl
     body.template run<N, ROW_FAST>(ph_smem, r, j, &tm);
 }
 
+// A pass whose body takes two tensor maps.
+template <int N, bool ROW_FAST, class Body>
+__global__ void __launch_bounds__(Shape<N, Body::EPT, Body::TT>::THREADS, min_blocks<N, Body>())
+    k_pass_tm2(const Body body, const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1) {
+    extern __shared__ __align__(128) unsigned char ph_smem[];
+    const int t = threadIdx.x;
+    const int r = ThreadMap<N, Body::EPT, Body::TT, ROW_FAST>::row(t);
+    const int j = ThreadMap<N, Body::EPT, Body::TT, ROW_FAST>::j(t);
+    body.template run<N, ROW_FAST>(ph_smem, r, j, &tm0, &tm1);
+}
+
 __device__ __forceinline__ int shift_idx(int i, int n) {   // centred index of natural frequency i
     int s = i + (n >> 1);
     return s >= n ? s - n : s;
@@ -337,6 +348,70 @@ struct SpectrumCols : PassBase {
     }
 };
 
+// The spectrum pass with the transfers staged: the columns of the front and
+// slice transfers that the CTA's ROWS rows kx need are loaded into shared
+// memory as [ky][kx mod ROWS] by tensor-map boxes of ROWS x 256 (issued before
+// the transform, so they overlap it; kx's centred column is one of ROWS
+// consecutive ones, ky's centred row range of a box is contiguous because N/2
+// is a multiple of 256).  The outputs then read them conflict-free instead of
+// gathering ROWS-element pieces from ROWS different lines per warp load.  One
+// item, no low-pass mask, N a multiple of 512 (so that N/2 is one of 256),
+// nx a multiple of 2 ROWS.
+struct SpectrumColsT : SpectrumCols {
+    int *err;   // raised if the staging wait times out
+    template <int N, bool RF>
+    static constexpr size_t xbytes() { return round128(Shape<N, EPT, TT>::template smem_bytes<RF>()); }
+    template <int N>
+    static constexpr size_t tbytes() { return (size_t)N * Shape<N, EPT, TT>::ROWS * 8; }   // one staged transfer
+    template <int N, bool RF>
+    static constexpr size_t smem() { return xbytes<N, RF>() + 2 * tbytes<N>() + 16; }
+    template <int N>
+    static constexpr bool staged() {
+        return N % 512 == 0 && Shape<N, EPT, TT>::ROWS >= 4 && Shape<N, EPT, TT>::ROWS <= 32 &&
+               smem<N, true>() <= kSmemMax;
+    }
+    template <int N, bool RF>
+    __device__ __forceinline__ void run(unsigned char *smem, int r, int j, const void *tm_hf,
+                                        const void *tm_hdz) const {
+        using S = Shape<N, EPT, TT>;
+        constexpr int ROWS = S::ROWS;
+        float2 *shf = reinterpret_cast<float2 *>(smem + xbytes<N, RF>());
+        float2 *shdz = shf + (size_t)N * ROWS;
+        uint64_t *bar = reinterpret_cast<uint64_t *>(smem + xbytes<N, RF>() + 2 * tbytes<N>());
+        const int kx0 = blockIdx.x * ROWS;
+        const int kx = kx0 + r;
+        const bool valid = kx < nx;
+        const int sx0 = shift_idx(kx0, nx);   // the centred columns of kx0 .. kx0 + ROWS - 1
+        if (threadIdx.x == 0) {
+            mbar_init(bar, 1);
+            mbar_fence_init();
+            mbar_arrive_expect_tx(bar, (uint32_t)(2 * tbytes<N>()));
+#pragma unroll 1
+            for (int q = 0; q < N / 256; ++q) {
+                const int sy = shift_idx(q * 256, N);
+                tma_load_2d(shf + (size_t)q * 256 * ROWS, tm_hf, sx0, sy, bar);
+                tma_load_2d(shdz + (size_t)q * 256 * ROWS, tm_hdz, sx0, sy, bar);
+            }
+        }
+        __syncthreads();   // the barrier is initialised before any thread waits on it
+        bool ready = false;
+        fft_row<N, S::E, false>(
+            xrow<N, EPT, TT, RF>(smem, r), j, tw,
+            [&](int, int y) -> float2 { return valid ? a1[(size_t)kx * N + y] : make_float2(0.f, 0.f); },
+            [&](int, int ky, float2 v) {
+                if (!ready) {   // (the first output: the boxes have landed)
+                    mbar_wait(bar, 0, err);
+                    ready = true;
+                }
+                if (!valid) return;
+                const float2 x0 = cscale(cmul(v, shf[ky * ROWS + r]), scale);
+                const float2 d = shdz[ky * ROWS + r];
+                state[(size_t)kx * N + ky] =
+                    make_float4(x0.x, x0.y, __uint_as_float(phase_turns_u32(d, ptab)), log2_modulus(d));
+            });
+    }
+};
+
 // ---------------------------------------------------------------- reconstruction pass A
 
 // Slice k of rows kx: X_k = X0 * Hdz^k; inverse FFT along ky; transposed store
@@ -355,7 +430,7 @@ struct SpectrumCols : PassBase {
 // and after a cluster barrier each stores a 1 / (4 / ROWS) share of the y
 // range for all 4 rows, reading its peers' rows through distributed shared
 // memory.  (Stores of 2 consecutive kx, 16 bytes, ran 2-4x slower.)
-template <bool GROUPED = false>   // GROUPED: the grouped-launch form (grid z = item)
+template <bool GROUPED = false, bool TSTORE = false>   // GROUPED: the grouped-launch form (grid z = item)
 struct ReconAT : PassBase, std::conditional_t<GROUPED, ReconItems, NoItems> {
     // 4 rows of 128 threads at N = 2048: one CTA per SM.  (One row per CTA in
     // clusters of 4, or two in clusters of 2, measured 65 % / 59 % slower.)
@@ -387,14 +462,15 @@ struct ReconAT : PassBase, std::conditional_t<GROUPED, ReconItems, NoItems> {
     // The chain saves the per-voxel sin/cos; the direct forms move fewer
     // shared-memory bytes per voxel and need fewer registers.  Measured per
     // pass A launch, chain against the staged state: 2048 3.7 % and 512 2.7 %
-    // faster; 1024 18 % slower (register spills); 4096 6 % slower (its
-    // distributed loads compete for shared-memory bandwidth); 256 22 % slower
-    // (slice groups of 6 slices do not repay the chain's start).  Other lengths keep the
+    // faster; 4096 with the tensor-map store 1.5 % faster; 1024 18 % slower
+    // (register spills; 6 % slower in the tensor-map store form, unspilled); 4096 with the pull store 6 % slower (its distributed
+    // loads compete for shared-memory bandwidth); 256 22 % slower (slice groups
+    // of 6 slices do not repay the chain's start).  Other lengths keep the
     // direct form.
     enum { FORM_NONE = 0, FORM_X0 = 1, FORM_STATE = 2, FORM_CHAIN = 3 };
     template <int N>
     static constexpr bool chain() {
-        return PH_RECONA_CHAIN >= 0 ? PH_RECONA_CHAIN != 0 : (N == 2048 || N == 512);
+        return PH_RECONA_CHAIN >= 0 ? PH_RECONA_CHAIN != 0 : (N == 2048 || N == 512 || (TSTORE && N == 4096));
     }
     template <int N, bool RF>
     static constexpr int rec_stride() {   // float2 between rows: conflict-free for the load pattern
@@ -446,11 +522,33 @@ struct ReconAT : PassBase, std::conditional_t<GROUPED, ReconItems, NoItems> {
         return cmul(make_float2(s.x, s.y), make_float2(cs * mag, sn * mag));
     }
 
+    // TSTORE: the transposed store through a tensor map, in boxes of 4 kx x
+    // 256 y (whole 32-byte sectors: boxes of 2 kx, 16-byte halves, measured
+    // 2-5x slower).  The last stage writes the 4 rows of kx to shared memory
+    // as [y][kx mod 4] (over the exchange rows, after a barrier) and one
+    // thread stores the boxes: the LSU no longer carries 8 sectors of 8
+    // different lines per warp store.
+    //  - 4 rows or more per CTA (lengths 256 .. 2048: 8192 / N rows, boxes of
+    //    that many kx): the CTA stages and stores all y.
+    //  - 2 rows per CTA, clusters of 2: CTA c stages y in [c N/2, (c+1) N/2)
+    //    of all 4 rows; each CTA writes its outputs into the owner's staging
+    //    (distributed shared memory for the peer's half) between two cluster
+    //    barriers (the owner's last-stage reads are done; the writes are
+    //    complete), then each stores its half.
+    // Full-size frames only (y0 = 0, ny_out = N, nx a multiple of 4).
+    static constexpr int kBoxY = 256;
+    template <int N>
+    static constexpr bool tstore_ok() {
+        constexpr int R = Shape<N, EPT, TT>::ROWS;
+        return N % kBoxY == 0 && ((R >= 4 && R <= 32 && cluster<N>() == 1) || (R == 2 && cluster<N>() == 2 && (N / 2) % kBoxY == 0));
+    }
+
     template <int N, bool RF>
-    __device__ __forceinline__ void run(unsigned char *smem, int r, int j) const {
+    __device__ __forceinline__ void run(unsigned char *smem, int r, int j, const void *tmap = nullptr) const {
         using S = Shape<N, EPT, TT>;
         constexpr int ROWS = S::ROWS;
         constexpr int FORM = form<N, RF>();
+        static_assert(!TSTORE || tstore_ok<N>(), "tensor-map store: 4..32 rows per CTA or 2 in a cluster of 2, N a multiple of 256");
         unsigned char *xbase = smem + stage_total<N, RF>();
         constexpr int CS = cluster<N>();
         // The CTAs of one row block (its `gridDim.y` slice groups) are consecutive
@@ -524,7 +622,7 @@ struct ReconAT : PassBase, std::conditional_t<GROUPED, ReconItems, NoItems> {
             srow = reinterpret_cast<const float4 *>(smem + (size_t)r * SS);
         }
         float2 *xr = xrow<N, EPT, TT, RF>(xbase, r);
-        if constexpr (CS > 1) cluster_arrive_relaxed();   // pairs with the first slice's wait
+        if constexpr (CS > 1 && !TSTORE) cluster_arrive_relaxed();   // pairs with the first slice's wait
         for (int b = b0; b < b1; ++b) {
             const uint32_t k = (uint32_t)(k0 + b);
             float2 *tb = t + (size_t)b * ny_out * nx;
@@ -541,7 +639,81 @@ struct ReconAT : PassBase, std::conditional_t<GROUPED, ReconItems, NoItems> {
                     return direct(srow[ky], k);
                 }
             };
-            if constexpr (CS == 1) {
+            if constexpr (TSTORE && CS == 2) {
+                // stg: [y - rank N/2][4] for this CTA's half of y, over the exchange rows
+                constexpr int YH = N / 2;
+                constexpr int LAST_SYNC = 2 * (FftPlan<N, S::E>::NSTAGES - 1);   // the one before store()
+                const uint32_t rank = cluster_ctarank();
+                const uint32_t stg_own = smem_addr(xbase);
+                const uint32_t stg_peer = map_to_rank(stg_own, rank ^ 1u);
+                int nsync = 0;
+                // First barrier: the previous slice's boxes have left the
+                // staging.  Last: both CTAs have read their last stage's
+                // inputs, so the staging (the peer's included) may be written.
+                // Its arrival is relaxed: the butterfly has consumed every
+                // value read, so the reads are complete (a release arrival
+                // made `membar` the third stall of the capture).
+                const auto sync = [&nsync]() {
+                    const int i = nsync++;
+                    if (i == 0 && threadIdx.x == 0) bulk_wait_read_all();
+                    if (i == LAST_SYNC) {
+                        cluster_arrive_relaxed();
+                        cluster_wait();
+                    } else {
+                        __syncthreads();
+                    }
+                };
+                fft_row_sync<N, S::E, true, false, true>(
+                    xr, j, tw, load,
+                    [&](int, int y, float2 v) {
+                        const uint32_t owner = (uint32_t)(y / YH);
+                        const uint32_t off = (uint32_t)((((y % YH) * 4) + (int)rank * ROWS + r) * 8);
+                        if (owner == rank) {
+                            st_shared_f2(stg_own + off, v);
+                        } else {
+                            st_cluster_f2(stg_peer + off, v);
+                        }
+                    },
+                    sync);
+                fence_proxy_async_cluster();   // the staging writes (local and remote), before the copy engine reads them
+                cluster_sync();                // every write into this CTA's staging has landed
+                if (threadIdx.x == 0) {
+#pragma unroll 1
+                    for (int q = 0; q < YH / kBoxY; ++q)
+                        tma_store_3d(tmap, reinterpret_cast<const float2 *>(xbase) + (size_t)q * kBoxY * 4,
+                                     kx0 - (int)rank * ROWS, (int)rank * YH + q * kBoxY, b);
+                    bulk_commit();
+                }
+            } else if constexpr (TSTORE) {
+                float2 *stg = reinterpret_cast<float2 *>(xbase);   // [y][ROWS], over the exchange rows
+                int nsync = 0;
+                // The first barrier of the transform precedes its first exchange
+                // write: the previous slice's boxes must have left the staging.
+                const auto sync = [&nsync]() {
+                    if (nsync++ == 0 && threadIdx.x == 0) bulk_wait_read_all();
+                    __syncthreads();
+                };
+                fft_row_sync<N, S::E, true, false, true>(
+                    xr, j, tw, load, [&](int, int y, float2 v) { stg[y * ROWS + r] = v; }, sync);
+                fence_proxy_async_smem();   // the staging writes, before the copy engine reads them
+                if (threadIdx.x < 32) {
+                    named_bar_sync(1, S::THREADS);
+                    if (threadIdx.x == 0) {
+#pragma unroll 1
+                        for (int q = 0; q < N / kBoxY; ++q) {
+                            if constexpr (GROUPED) {   // one map over the items' slots: (kx, y, slice, item)
+                                tma_store_4d(tmap, stg + (size_t)q * kBoxY * ROWS, kx0, q * kBoxY, b,
+                                             (int)blockIdx.z);
+                            } else {
+                                tma_store_3d(tmap, stg + (size_t)q * kBoxY * ROWS, kx0, q * kBoxY, b);
+                            }
+                        }
+                        bulk_commit();
+                    }
+                } else {
+                    named_bar_arrive(1, S::THREADS);
+                }
+            } else if constexpr (CS == 1) {
                 fft_row<N, S::E, true>(xr, j, tw, load, [&](int, int y, float2 v) {
                     const int yo = y - y0;
                     // streaming store: T passes through L2 once
@@ -584,11 +756,15 @@ struct ReconAT : PassBase, std::conditional_t<GROUPED, ReconItems, NoItems> {
                 cluster_arrive_relaxed();
             }
         }
-        if constexpr (CS > 1) cluster_wait();   // no CTA leaves while a peer reads its rows
+        if constexpr (CS > 1 && !TSTORE) cluster_wait();   // no CTA leaves while a peer reads its rows
+        if constexpr (TSTORE) {
+            if (threadIdx.x == 0) bulk_wait_all();   // the shared memory outlives the last boxes' reads
+        }
     }
 };
 
 using ReconA = ReconAT<false>;
+using ReconATStore = ReconAT<false, true>;
 using ReconAGrouped = ReconAT<true>;
 
 // ---------------------------------------------------------------- reconstruction pass B
@@ -617,9 +793,7 @@ __device__ __forceinline__ float clamp01(float v) { return fminf(fmaxf(v, 0.0f),
 // first the bulk-copy target (dense rows) and then, after the first stage has
 // read it, the exchange rows of that slice's transform.  CTAs are small (128
 // threads: one row at N >= 2048) so that the barriers of the FFT stages span
-// only the warps that exchange data, and RTS / 128 CTAs share an SM.  The
-// lengths 256 .. 4096 run the two-stage transform instead (ph_two_b.cuh), with
-// these parameters.
+// only the warps that exchange data, and RTS / 128 CTAs share an SM.
 template <int EPI, bool GROUPED = false>   // GROUPED: the grouped-launch form (EPI_PROJ, grid z = item)
 struct ReconB : PassBase, std::conditional_t<GROUPED, ReconItems, NoItems> {
     static constexpr int TT = 128;
@@ -633,7 +807,7 @@ struct ReconB : PassBase, std::conditional_t<GROUPED, ReconItems, NoItems> {
     const float2 *t;                 // [batch][rows][nx]
     const float2 *tw;
     unsigned long long *proj64;      // [rows_out][nx_out] or null
-    unsigned *proj32;                // two-stage lengths, proj64 null: the minima alone, as float bits
+    unsigned *proj32;                // two-stage pass: the minima alone, as float bits, or null
     void *vol;                       // [S][rows_out][nx_out] or null
     int *err;                        // raised if a bulk-copy wait times out
     int vol_dtype;                   // PH_N0F8 .. PH_F64, or PH_BOOL: intensity <= threshold

@@ -120,6 +120,18 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t saddr, uint32_t rank) {
     return r;
 }
 
+__device__ __forceinline__ void st_cluster_f2(uint32_t addr, float2 v) {
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(v.x), "f"(v.y) : "memory");
+}
+__device__ __forceinline__ void st_shared_f2(uint32_t addr, float2 v) {
+    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(v.x), "f"(v.y) : "memory");
+}
+// Generic-proxy writes to the shared memory of any CTA of the cluster, before
+// the async proxy (a bulk copy issued after a cluster barrier) reads them.
+__device__ __forceinline__ void fence_proxy_async_cluster() {
+    asm volatile("fence.proxy.async.shared::cluster;" ::: "memory");
+}
+
 __device__ __forceinline__ float2 ld_cluster_f2(uint32_t addr) {
     float2 v;
     asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
@@ -146,6 +158,33 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
 
 // ---- tiled bulk stores (shared -> global through a tensor map)
 
+// One box of a 3-D tensor map from shared memory (128-byte aligned) to the
+// tensor at element coordinates (x, y, z); x times the element size must be a
+// multiple of 16 bytes and no coordinate negative.  Elements outside the
+// tensor are not written.  The issuing thread tracks it in its bulk group.
+__device__ __forceinline__ void tma_store_3d(const void *tmap, const void *src, int x, int y, int z) {
+    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(tmap),
+                 "r"(smem_addr(src)), "r"(x), "r"(y), "r"(z)
+                 : "memory");
+}
+// ---- tiled bulk loads (global -> shared through a tensor map)
+
+// One box of a 2-D tensor map at element coordinates (x, y) into shared
+// memory (128-byte aligned); completion counts the box's bytes on `bar`.
+__device__ __forceinline__ void tma_load_2d(void *dst, const void *tmap, int x, int y, uint64_t *bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+            smem_addr(dst)),
+        "l"(tmap), "r"(x), "r"(y), "r"(smem_addr(bar))
+        : "memory");
+}
+
+// The 4-D form: element coordinates (x, y, z, w).
+__device__ __forceinline__ void tma_store_4d(const void *tmap, const void *src, int x, int y, int z, int w) {
+    asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(tmap),
+                 "r"(smem_addr(src)), "r"(x), "r"(y), "r"(z), "r"(w)
+                 : "memory");
+}
 // L2 policy of data that is written (or read) once and not used again before it
 // would be evicted anyway: it makes room first.
 __device__ __forceinline__ uint64_t l2_evict_first() {
@@ -153,11 +192,7 @@ __device__ __forceinline__ uint64_t l2_evict_first() {
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
     return p;
 }
-// One box of a 3-D (4-D) tensor map from shared memory (128-byte aligned) to the
-// tensor at element coordinates (x, y, z (, w)), with an L2 policy; x times the
-// element size must be a multiple of 16 bytes and no coordinate negative.
-// Elements outside the tensor are not written.  The issuing thread tracks it in
-// its bulk group.
+// The 3-D and 4-D stores with an L2 policy.
 __device__ __forceinline__ void tma_store_3d(const void *tmap, const void *src, int x, int y, int z, uint64_t policy) {
     asm volatile(
         "cp.async.bulk.tensor.3d.global.shared::cta.bulk_group.L2::cache_hint [%0, {%2, %3, %4}], [%1], %5;" ::"l"(tmap),

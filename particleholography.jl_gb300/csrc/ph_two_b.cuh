@@ -118,10 +118,6 @@ __global__ void __launch_bounds__(128, PassB<N, EPI, GROUPED, SLICE>::CTAS) k_tw
             }
             tmem_wait_st();
         }
-        int sub_b = 0, sub_e = 0;   // EPI_SUB: this row's box list
-        if constexpr (EPI == EPI_SUB) {
-            if (valid) { sub_b = p.row_ptr[y]; sub_e = p.row_ptr[y + 1]; }
-        }
         uint32_t parity = 0;
         for (int b = b0; b < b1; ++b) {
             const int k = p.k0 + b;
@@ -172,43 +168,24 @@ __global__ void __launch_bounds__(128, PassB<N, EPI, GROUPED, SLICE>::CTAS) k_tw
                             i2[i] = fmaf(q.x, q.x, q.y * q.y);
                         }
                         if constexpr (EPI == EPI_VOL) {
-                            // store() converts and stores one value and gives back what it stored; the
-                            // type is chosen once per 16 values
-                            const size_t row = (size_t)k * p.vol_slice_stride + (size_t)y * p.nx_out;
-                            const unsigned width = valid && live ? (unsigned)p.nx_out : 0u;
+                            // the type is chosen once per 16 values
+                            const size_t row = (size_t)k * p.vol_slice_stride + (size_t)y * N + H * (l + L * m + E * c) + h;
                             const auto store16 = [&](auto *vol, auto &&convert) {
                                 auto *out = vol + row;
 #pragma unroll
                                 for (int i = 0; i < 16; ++i) {
-                                    const int xo = H * (l + L * m + E * (c + i)) + h - p.x0;
                                     i2[i] = clamp01(i2[i]);
                                     const auto q = convert(i2[i]);
-                                    if ((unsigned)xo < width) out[xo] = q;
+                                    if (valid && live) out[H * E * i] = q;
                                 }
                             };
-                            switch (p.vol_dtype) {
-                                case 0:   // N0f8
-                                    store16(reinterpret_cast<uint8_t *>(p.vol), [](float &v) {
-                                        const unsigned q = __float2uint_rn(v * 255.0f);
-                                        v = __fdiv_rn((float)q, 255.0f);
-                                        return (uint8_t)q;
-                                    });
-                                    break;
-                                case 1:
-                                    store16(reinterpret_cast<__half *>(p.vol), [](float &v) {
-                                        const __half h = __float2half_rn(v);
-                                        v = __half2float(h);
-                                        return h;
-                                    });
-                                    break;
-                                case 3: store16(reinterpret_cast<double *>(p.vol), [](float &v) { return (double)v; }); break;
-                                case 5: {   // binary volume: the clamped Float32 intensity <= threshold
-                                    const float thr = p.threshold;
-                                    store16(reinterpret_cast<uint8_t *>(p.vol),
-                                            [thr](float &v) { return (uint8_t)(v <= thr ? 1 : 0); });
-                                    break;
-                                }
-                                default: store16(reinterpret_cast<float *>(p.vol), [](float &v) { return v; }); break;
+                            if (p.vol_dtype == 3) {
+                                store16(reinterpret_cast<double *>(p.vol), [](float v) { return (double)v; });
+                            } else if (p.vol_dtype == 5) {   // binary volume: the clamped Float32 intensity <= threshold
+                                const float thr = p.threshold;
+                                store16(reinterpret_cast<uint8_t *>(p.vol), [thr](float v) { return (uint8_t)(v <= thr ? 1 : 0); });
+                            } else {
+                                store16(reinterpret_cast<float *>(p.vol), [](float v) { return v; });
                             }
                         }
                         if (track) {
@@ -232,24 +209,8 @@ __global__ void __launch_bounds__(128, PassB<N, EPI, GROUPED, SLICE>::CTAS) k_tw
 #pragma unroll
                     for (int i = 0; i < L; ++i) {
                         const int x = H * (l + L * m + E * i) + h;
-                        if (!live) continue;
-                        if constexpr (EPI == EPI_SUB) {
-                            if (sub_b == sub_e) continue;
-                            const float i2 = clamp01(fmaf(u[i].x, u[i].x, u[i].y * u[i].y));
-                            const uint8_t q = (uint8_t)__float2uint_rn(i2 * 255.0f);
-                            for (int s = sub_b; s < sub_e; ++s) {
-                                const SubBox bx = p.boxes[p.row_box[s]];
-                                if (k >= bx.z0 && k <= bx.z1 && x >= bx.fx0 && x <= bx.fx1)
-                                    reinterpret_cast<uint8_t *>(
-                                        p.vol)[bx.off + ((long long)(k - bx.z0) * bx.nyb + (y - bx.sy0)) * bx.nxb +
-                                               (x - bx.fx0)] = q;
-                            }
-                        } else {
-                            const int xo = x - p.x0;
-                            if (valid && xo >= 0 && xo < p.nx_out)
-                                reinterpret_cast<float2 *>(
-                                    p.vol)[(size_t)k * p.vol_slice_stride + (size_t)y * p.nx_out + xo] = u[i];
-                        }
+                        if (valid && live)
+                            reinterpret_cast<float2 *>(p.vol)[(size_t)k * p.vol_slice_stride + (size_t)y * N + x] = u[i];
                     }
                 }
             }
@@ -267,9 +228,9 @@ __global__ void __launch_bounds__(128, PassB<N, EPI, GROUPED, SLICE>::CTAS) k_tw
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
                         const int m = (c + i) / L, o = (c + i) % L;
-                        const int xo = H * (l + L * m + E * o) + h - p.x0;
-                        if (valid && (PL::M * L == E || l + L * m < E) && xo >= 0 && xo < p.nx_out) {
-                            const size_t at = (size_t)y * p.nx_out + xo;
+                        const int xo = H * (l + L * m + E * o) + h;
+                        if (valid && (PL::M * L == E || l + L * m < E)) {
+                            const size_t at = (size_t)y * N + xo;
                             if constexpr (SLICE) atomicMin(proj64 + at, pack_min(mv[i], __float_as_int(mk[i])));
                             else atomicMin(p.proj32 + at, __float_as_uint(mv[i]));   // (non-negative: ordered as bits)
                         }
@@ -307,10 +268,10 @@ cudaError_t launch_b_form(const ReconB<EPI, GROUPED> &p, int groups, int items, 
 
 template <int N, int EPI, bool GROUPED>
 cudaError_t launch_b(const ReconB<EPI, GROUPED> &p, int groups, int items, cudaStream_t s) {
-    if constexpr (!GROUPED && (EPI == EPI_PROJ || EPI == EPI_VOL)) {
-        if (p.proj64 == nullptr) return launch_b_form<N, EPI, GROUPED, false>(p, groups, items, s);
-    }
-    return launch_b_form<N, EPI, GROUPED, true>(p, groups, items, s);
+    if constexpr (EPI == EPI_PROJ && !GROUPED)
+        if (p.proj32 == nullptr) return launch_b_form<N, EPI, GROUPED, true>(p, groups, items, s);
+    if constexpr (GROUPED) return launch_b_form<N, EPI, GROUPED, true>(p, groups, items, s);
+    else return launch_b_form<N, EPI, GROUPED, false>(p, groups, items, s);
 }
 
 }  // namespace two
