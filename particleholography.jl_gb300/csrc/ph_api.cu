@@ -1060,16 +1060,20 @@ int reconstruct(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin, void 
         const unsigned char *tab = nullptr;
         PH_TRY(get_tc_table(ctx, nx, effective_form(ctx, nx, ny), s, &tab));
     }
-    // Where no slice is asked for and the two-stage row pass runs, pass B merges the
-    // minima straight into the caller's projection (every pixel gets one).  It is reset
-    // before the inputs are read, so not if it overlaps one of them.
-    const auto apart = [&](const void *in, size_t bytes) {
-        const char *p0 = reinterpret_cast<const char *>(proj), *q0 = static_cast<const char *>(in);
-        return in == nullptr || p0 + sizeof(float) * nx_out * ny_out <= q0 || q0 + bytes <= p0;
+    // An output that is reset before the inputs are read: not if it overlaps one of them.
+    const size_t npix = (size_t)nx_out * ny_out, field = sizeof(float2) * nx * ny;
+    const auto apart = [&](const void *out, size_t out_bytes) {
+        const char *p0 = static_cast<const char *>(out);
+        const auto from = [&](const void *in, size_t bytes) {
+            const char *q0 = static_cast<const char *>(in);
+            return in == nullptr || p0 + out_bytes <= q0 || q0 + bytes <= p0;
+        };
+        return from(wf, field) && from(hf, field) && from(hdz, field) && from(lpf, field / 2);
     };
-    const size_t field = sizeof(float2) * nx * ny;
-    const bool merge32 = proj != nullptr && argmin == nullptr && packed == nullptr && apart(wf, field) &&
-                         apart(hf, field) && apart(hdz, field) && apart(lpf, field / 2);
+    // Where no slice is asked for and the two-stage row pass runs, pass B merges the
+    // minima straight into the caller's projection (every pixel gets one).
+    const bool merge32 = proj != nullptr && argmin == nullptr && packed == nullptr && apart(proj, sizeof(float) * npix);
+    const bool fill_first = packed != nullptr && apart(packed, sizeof(unsigned long long) * npix);
     // (a volume whose projection cannot be merged there keeps the row engine's 64-bit words)
     const ReconPath path = kind == RK_PROJ || kind == RK_CVOL ||
                                    (kind == RK_VOL && vol_dtype != PH_F16 && vol_dtype != PH_N0F8 &&
@@ -1088,14 +1092,13 @@ int reconstruct(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin, void 
              (const void *)hdz, ctx->scratch, (int)ctx->opt_loop_limit, (const void *)lpf, thr_bits, (void *)packed,
              (int)accumulate, first, effective_form(ctx, nx, ny) * 1000 + (tu ? tu->group_cap : 0));
     return run_graph(ctx, s, key, [&](cudaStream_t s) -> int {
-        // (before the passes, so that these follow one another as programmatic dependents)
-        const size_t npix = (size_t)nx_out * ny_out;
+        // (resets before the passes, so that these follow one another as programmatic dependents)
+        const auto fill = [&]() -> int {
+            k_fill_u64<<<(unsigned)std::min<size_t>((npix + 255) / 256, 4096), 256, 0, s>>>(p64, npix, kPackedEmpty);
+            return launched(ctx, cudaGetLastError(), "packed fill");
+        };
         if (packed != nullptr) {
-            if (!accumulate) {
-                k_fill_u64<<<(unsigned)std::min<size_t>((npix + 255) / 256, 4096), 256, 0, s>>>(p64, npix,
-                                                                                               kPackedEmpty);
-                PH_TRY(launched(ctx, cudaGetLastError(), "packed fill"));
-            }
+            if (!accumulate && fill_first) PH_TRY(fill());
         } else if (want_proj) {
             if (minima_only)
                 PH_CUDA(cudaMemsetAsync(proj, 0xff, sizeof(float) * npix, s), "memset");
@@ -1104,6 +1107,7 @@ int reconstruct(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin, void 
         }
         PH_TRY(issue_spectrum(ctx, wf, hf, hdz, nx, ny, padded, nin_x, nin_y, at<float2>(ctx, L.a1), state, tw_x,
                               tw_y, at<double>(ctx, L.acc), at<float2>(ctx, L.mean), s, nullptr, lpf, path));
+        if (packed != nullptr && !accumulate && !fill_first) PH_TRY(fill());
         return issue_recon_slices(ctx, kind, proj, argmin, vol, vol_dtype, nx, ny, nx_out, ny_out, x0, y0, slices,
                                   L.batch, state, t, p64, tw_x, tw_y, want_proj && packed == nullptr, s, threshold,
                                   first, nullptr, minima_only, path);
