@@ -1246,7 +1246,7 @@ int issue_recon_slices(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin
         const int group = recon_group_a(path, nb, nx, ny, y0, ny_out, cap);
         const int group_b = recon_group_b(path, nb, nx, ny_out, 1, group, cap);
         const auto fill_a = [&](auto &a) {
-            a.state = state; a.t = t; a.tw = tw_y; a.nx = nx; a.ny_out = ny_out; a.y0 = y0;
+            a.state = state; a.t = t; a.tw = tw_y; a.ptab = ctx->phase_tab; a.nx = nx; a.ny_out = ny_out; a.y0 = y0;
             a.k0 = k0; a.nbatch = nb; a.group = group;
             a.err = static_cast<int *>(ctx->small);
         };
@@ -1498,6 +1498,7 @@ int issue_recon_group(ph_ctx *ctx, const std::vector<const ph_recon_item *> &its
         a.item_state_stride = ib / sizeof(float4);
         a.item_t_stride = ib / sizeof(float2);
         a.tw = tw_y;
+        a.ptab = ctx->phase_tab;
         a.nx = nx;
         a.ny_out = ny;
         a.y0 = 0;

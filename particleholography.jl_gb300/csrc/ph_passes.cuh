@@ -442,6 +442,7 @@ struct ReconAT : PassBase, std::conditional_t<GROUPED, ReconItems, NoItems> {
     const float4 *state;   // [nx][ny]
     float2 *t;             // [batch][ny_out][nx]
     const float2 *tw;
+    const float4 *ptab;    // two-stage pass: kPhaseTable unit vectors as FP32 pairs
     int *err;              // raised if a bulk-copy wait times out
     int nx, ny_out, y0;
     int k0;                // global slice index of batch slot 0

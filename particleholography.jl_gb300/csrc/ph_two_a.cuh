@@ -13,13 +13,18 @@ namespace two {
 // at 128 .. 512, two warps per row at 3072 and 4096), so that the exchange needs no CTA
 // barrier.  X_k and Hdz of a thread's values live in tensor memory (4 E columns
 // of its own lane): every slice reads both and writes back X_{k+1} = X_k Hdz.  X
-// is formed anew from the spectrum state at every multiple of CHAIN slices, so
-// that a projection is as near to the 64-bit one as with every slice formed
-// directly: relative error 4.1e-7 at 1024^2 (CHAIN = 8; 4.2e-7 direct), 2.7e-7 at
-// the short lengths (CHAIN = 4; 2.3e-7 direct, 4.0e-7 at 8).  At 2048 and 4096,
-// where the row engine ran chains of 64 slices (5.1e-6 at 4096, now 1.4e-6), 16.
-// Shorter chains cost: 1024^2 x 256 0.49 ms at 8, 0.51 at 4; 2048^2 x 256 2.21 ms
-// at 16, 2.30 at 8.
+// is formed anew from the spectrum state at every multiple of CHAIN slices.
+//
+// Precision: a projection is as near to the 64-bit one as with every slice formed
+// directly by the row engine (relative errors at 12 random distances, there and here:
+// 256^2 3.5e-7 and 3.2e-7, 1024^2 3.9e-7 and 3.7e-7, 2048 x 1536 3.7e-7 and 3.7e-7; the
+// engine's chains at 2048^2 8.4e-7, here 4.0e-7).  For that Hdz has to be right to well
+// below a rounding, since its error adds up along the chain, and that of the zero
+// frequency shows in every pixel (with Hdz from sincospif and exp2f: 4.3e-7 at 1024^2,
+// 4.5e-7 at 2048 x 1536); and X from the polynomials of `rotated` rather than __sincosf,
+// which is good to 1e-7 only.  CHAIN is as long as that leaves room for: at 256^2 x 32
+// 27 us with 4 and 29 with 8 (small groups walk to their start), at 512^2 x 64 87 and 83;
+// at 1024^2 x 256 863 with 8 and 842 with 16; at 2048 x 1536 x 157 16 gives 4.0e-7.
 //
 // In the row engine this pass moved 87 bytes per voxel through the shared-memory
 // data path (chain 24, two exchanges 32, staging 16, twiddles 15); here 32 to 40.
@@ -59,7 +64,7 @@ struct PassA {
     static constexpr size_t SMEM = STAGE + RB * XB + F::BYTES + 24;
     static constexpr int BOX_Y = box_y(N);
     // slices between two formations of X
-    static constexpr uint32_t CHAIN = N <= 768 ? 4 : PL::E == 64 ? 16 : 8;
+    static constexpr uint32_t CHAIN = N <= 256 ? 4 : N == 1024 || PL::E == 64 ? 16 : 8;
 };
 
 // Byte offset of (y, row r) in the staging [y][RB], with the tensor map's
@@ -70,6 +75,39 @@ template <int RB>
 __device__ __forceinline__ uint32_t stage_offset(int y, int r) {
     const uint32_t a = (uint32_t)(y * RB + r) * 8;
     return a ^ ((a >> 3) & (RB == 8 ? 0x30u : 0x10u));
+}
+
+// exp(2 pi i turns / 2^32) 2^w, off by at most 1e-8 before its one rounding where the
+// modulus is near one, so that a stored Float32 factor comes out as it was.  `angle`: lane
+// i's entry of the 32 angles 2 pi i / 32, (cos hi, cos lo, sin hi, sin lo); the whole warp calls.
+__device__ __forceinline__ float2 unit_power(uint32_t turns, float w, const float4 angle) {
+    const uint32_t i = (turns + (1u << 26)) >> 27;                 // the nearest of them
+    const float x = (float)(int32_t)(turns - (i << 27)) * 1.46291807926715968e-9f, x2 = x * x;   // 2 pi / 2^32
+    const float ch = __shfl_sync(0xffffffffu, angle.x, i & 31), cl = __shfl_sync(0xffffffffu, angle.y, i & 31);
+    const float sh = __shfl_sync(0xffffffffu, angle.z, i & 31), sl = __shfl_sync(0xffffffffu, angle.w, i & 31);
+    const float sn = fmaf(x * x2, fmaf(x2, 1.0f / 120.0f, -1.0f / 6.0f), x);
+    const float cs1 = x2 * fmaf(x2, fmaf(x2, -1.0f / 720.0f, 1.0f / 24.0f), -0.5f);   // cos - 1
+    float c1 = cl + fmaf(ch, cs1, -sh * sn), s1 = sl + fmaf(sh, cs1, ch * sn);
+    if (fabsf(w) < 0.015625f) {   // the modulus minus one, whose rounding is not that of a value near one
+        const float y = w * 0.69314718055994530942f, m1 = y * fmaf(y, fmaf(y, 1.0f / 6.0f, 0.5f), 1.0f);
+        c1 = fmaf(ch + c1, m1, c1);
+        s1 = fmaf(sh + s1, m1, s1);
+        return make_float2(ch + c1, sh + s1);
+    }
+    const float mag = exp2f(w);
+    return make_float2((ch + c1) * mag, (sh + s1) * mag);
+}
+
+// x0 exp(2 pi i turns / 2^32) 2^w: the nearest quarter turn, and Taylor polynomials of the
+// rest (at most pi / 4; truncated below 4e-9).
+__device__ __forceinline__ float2 rotated(float2 x0, uint32_t turns, float w) {
+    const uint32_t q = (turns + (1u << 29)) >> 30;
+    const float x = (float)(int32_t)(turns - (q << 30)) * 1.46291807926715968e-9f, x2 = x * x;   // 2 pi / 2^32
+    const float sn = fmaf(x * x2, fmaf(x2, fmaf(x2, fmaf(x2, 1.0f / 362880.0f, -1.0f / 5040.0f), 1.0f / 120.0f), -1.0f / 6.0f), x);
+    const float cs = fmaf(x2, fmaf(x2, fmaf(x2, fmaf(x2, 1.0f / 40320.0f, -1.0f / 720.0f), 1.0f / 24.0f), -0.5f), 1.0f);
+    const float a = q & 1 ? sn : cs, b = q & 1 ? cs : sn, mag = exp2f(w);
+    const float c = (q + 1) & 2 ? -a : a, s = q & 2 ? -b : b;
+    return cmul(x0, make_float2(c * mag, s * mag));
 }
 
 template <int N, bool GROUPED>
@@ -145,7 +183,8 @@ __global__ void __launch_bounds__(PassA<N>::THREADS, PassA<N>::CTAS)
         if (first || ahead == 0) {
             // X at the last multiple of CHAIN, then the chain's own products: X_k does
             // not depend on where a group or a range of slices starts.  The first time
-            // also Hdz, by the accurate sin/cos, as its error grows along the chain.
+            // also Hdz.
+            const float4 angle = __ldg(p.ptab + (threadIdx.x & 31) * (kPhaseTable / 32));
             float4 st[P];
             const auto read = [&](int n2) {
 #pragma unroll
@@ -160,16 +199,13 @@ __global__ void __launch_bounds__(PassA<N>::THREADS, PassA<N>::CTAS)
                 if (n2 + 1 < Q) read(n2 + 1);   // the next group's state is on its way
                 float2 t[P];
 #pragma unroll
-                for (int n1 = 0; n1 < P; ++n1) t[n1] = ReconAT<GROUPED>::direct(cur[n1], k - ahead);
+                for (int n1 = 0; n1 < P; ++n1)
+                    t[n1] = rotated(make_float2(cur[n1].x, cur[n1].y), (k - ahead) * __float_as_uint(cur[n1].z),
+                                    (float)(k - ahead) * cur[n1].w);
                 if (first) {
                     float2 hd[P];
 #pragma unroll
-                    for (int n1 = 0; n1 < P; ++n1) {
-                        float sn, cs;
-                        sincospif((float)(int32_t)__float_as_uint(cur[n1].z) * 4.656612873077392578125e-10f, &sn, &cs);
-                        const float mag = exp2f(cur[n1].w);
-                        hd[n1] = make_float2(cs * mag, sn * mag);
-                    }
+                    for (int n1 = 0; n1 < P; ++n1) hd[n1] = unit_power(__float_as_uint(cur[n1].z), cur[n1].w, angle);
                     put(tm + n2 * 4 * P + 2 * P, hd);
 #pragma unroll 1
                     for (uint32_t i = 0; i < ahead; ++i)
