@@ -154,6 +154,12 @@ __global__ void k_two_factors(float2 *out, int n, int lanes, int p, int q) {
     out[i] = twiddle_fp64(l * (j < p - 1 ? j + 1 : p * (j - p + 2)), n);
 }
 
+// Its stage twiddles W^(l k) as [k][l < lanes].
+__global__ void k_two_twiddles(float2 *out, int n, int lanes) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = twiddle_fp64(i % lanes * (i / lanes), n);
+}
+
 // holofunc.jl:8-15 with the reference's Float64 operation order; the
 // intrinsics keep the compiler from contracting into fma.
 __device__ __forceinline__ double sqr_term(int i1, int n, double wavlen, double dx) {
@@ -678,14 +684,12 @@ int get_twiddles(ph_ctx *ctx, int n, cudaStream_t s, const float2 **out) {
     }
     if (two_stage) {
         const int E = two::values(n), L = n / E;
-        const auto fill = [&](int offset, int r, int lanes) {
-            const int pp = two::split_p_of(r), qq = r / pp, cnt = two::factors_of(r, lanes);
-            k_two_factors<<<(cnt + 255) / 256, 256, 0, s>>>(p + offset, n, lanes, pp, qq);
-            ctx->launches++;
-            return cudaGetLastError();
-        };
-        PH_CUDA(fill(two::factors_offset(n), E, L), "k_two_factors");
-        PH_CUDA(fill(two::mirror_offset(n), L, E), "k_two_factors");
+        const int pp = two::split_p_of(E), cnt = two::factors_of(E, L);
+        k_two_factors<<<(cnt + 255) / 256, 256, 0, s>>>(p + two::factors_offset(n), n, L, pp, E / pp);
+        k_two_twiddles<<<(n + 255) / 256, 256, 0, s>>>(p + two::twiddle_offset(n), n, L);
+        k_two_twiddles<<<(n + 255) / 256, 256, 0, s>>>(p + two::mirror_offset(n), n, E);
+        ctx->launches += 3;
+        PH_CUDA(cudaGetLastError(), "k_two_twiddles");
     }
     ctx->tw[n] = p;
     *out = p;

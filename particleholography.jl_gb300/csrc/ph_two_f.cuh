@@ -48,9 +48,7 @@ __device__ __forceinline__ void transform(const float2 *__restrict__ tw, float *
     {
         float2 v[E], w[E];
         level1<E, INV>(w, load);
-        Factors<N, INV> f;   // (each factor is used once: straight from the table)
-        f.load_global(tw, l);
-        level2<E, INV>(w, [&](int o, float2 x) { v[o] = f.apply(o, x); });
+        level2<E, INV>(w, [&](int o, float2 x) { v[o] = stage_twiddle<INV>(tw, twiddle_offset(N), o, L, l, x); });
         exchange<N>(v, z, ex, l, sync);
     }
 #pragma unroll

@@ -58,8 +58,6 @@ __global__ void __launch_bounds__(PassG<N>::THREADS, PassG<N>::CTAS) k_two_gs(co
     const bool valid = row < p.nrows;
     const size_t at = (size_t)min(row, p.nrows - 1) * N;     // (rows beyond the last: its values again, not stored)
     grid_dependents_launch();
-    Factors<N, INV1> f;
-    f.load_global(p.tw, l);
     grid_dependency_wait();                                  // the previous pass wrote src and may still read dst
 
     // the operand of value k = l + L m + E o: the transfer or the amplitude
@@ -74,7 +72,7 @@ __global__ void __launch_bounds__(PassG<N>::THREADS, PassG<N>::CTAS) k_two_gs(co
     {
         float2 v[E], w[E], z[M * L];
         level1<E, INV1>(w, [&](int i) { return p.src[at + l + L * i]; });
-        level2<E, INV1>(w, [&](int o, float2 x) { v[o] = f.apply(o, x); });
+        level2<E, INV1>(w, [&](int o, float2 x) { v[o] = stage_twiddle<INV1>(p.tw, twiddle_offset(N), o, L, l, x); });
         if constexpr (EARLY) {
 #pragma unroll
             for (int o = 0; o < L; ++o) op[o] = operand(0, o);
@@ -124,11 +122,10 @@ __global__ void __launch_bounds__(PassG<N>::THREADS, PassG<N>::CTAS) k_two_gs(co
             float2 v[M * L];
 #pragma unroll
             for (int m = 0; m < M; ++m) {
-                MirrorFactors<N, !INV1> g;
-                g.load_global(p.tw, M * L == E ? l + L * m : min(l + L * m, E - 1));
+                const int t = M * L == E ? l + L * m : min(l + L * m, E - 1);
                 float2 q[L];
                 level1<L, !INV1>(q, [&](int i) { return u[m * L + i]; });
-                level2<L, !INV1>(q, [&](int o, float2 x) { v[m * L + o] = g.apply(o, x); });
+                level2<L, !INV1>(q, [&](int o, float2 x) { v[m * L + o] = stage_twiddle<!INV1>(p.tw, mirror_offset(N), o, E, t, x); });
             }
             mirror_exchange<N>(v, y, ex, l, sync);
         }

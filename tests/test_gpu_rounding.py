@@ -29,3 +29,20 @@ def test_slices_of_a_uniform_field(ph, cuda, ny):
     # 2 components x 2 roundings per product; 7.5 products of the chain on average, and four
     # more for the first slice's phase, modulus, rotation and scale; half as much again
     assert np.sqrt(np.mean(np.square(off))) <= 1.5 * ROUNDING * np.sqrt(2 * 2 * (7.5 + 4))
+
+
+def test_propagation_by_nothing(ph, cuda):
+    """White noise through two transforms each way at 128 = 8 x 16, with a transfer of one.
+    Per transform: 7 levels of additions at 2.75e-8 each (a rounding over the spread of
+    mantissas), and 1.75 twiddle products (the stage's, half of radix 16's and a quarter of
+    radix 8's are not trivial) of 4.4e-8: the factor's rounding and the product's two.
+    1.86e-7 in all; stage twiddles formed as products of two rounded factors make it 2.04e-7."""
+    n = 128
+    g = torch.Generator(device=cuda)
+    g.manual_seed(128)
+    u = torch.randn((n, n), dtype=torch.complex64, generator=g, device=cuda)
+    out = ph.CuWavefront(torch.empty_like(u))
+    one = ph.CuTransferSqrtPart(torch.ones((n, n), dtype=torch.float32, device=cuda))
+    ph.cu_asm_prop_(out, ph.CuWavefront(u), one, 0.0, n, LAM)
+    off = (out.data.to(torch.complex128) - u).abs().square().sum() / u.to(torch.complex128).abs().square().sum()
+    assert float(off.sqrt()) <= 1.95e-7
