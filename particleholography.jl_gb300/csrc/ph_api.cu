@@ -1688,12 +1688,37 @@ int64_t ph_profile_report(ph_ctx *ctx, char *buf, int64_t cap) {
 size_t ph_scratch_bytes(const ph_ctx *ctx) { return ctx ? ctx->scratch_bytes : 0; }
 int64_t ph_kernel_launches(const ph_ctx *ctx) { return ctx ? ctx->launches.load() : 0; }
 
+// Scratch of a phase retrieval: two fields, and for the staged forms the transfers and
+// amplitudes of both planes.
+struct GsLayout {
+    size_t oa, ob, oh, ohi, oa1, oa2, total;
+};
+static GsLayout gs_layout(size_t n, bool staged) {
+    GsLayout g{};
+    Arena a;
+    g.oa = a.take<float2>(n);
+    g.ob = a.take<float2>(n);
+    if (staged) {
+        g.oh = a.take<float2>(n);
+        g.ohi = a.take<float2>(n);
+        g.oa1 = a.take<float>(n);
+        g.oa2 = a.take<float>(n);
+    }
+    g.total = a.off;
+    return g;
+}
+static bool gs_persistent(int nx, int ny) { return gs_row_staged(nx) && gs_col_staged(ny); }
+
 int32_t ph_reserve(ph_ctx *ctx, int32_t n_fast, int32_t n_slow, int32_t slices, void *stream) {
     PH_ENTER(ctx, stream);
     PH_TRY(check_len(ctx, n_fast, n_slow));
     ReconLayout L = recon_layout(ctx, n_fast, n_slow, n_slow, n_fast, std::max(1, (int)slices));
-    const size_t gs = 2 * sizeof(float2) * (size_t)n_fast * n_slow + 2 * kAlign;
-    PH_TRY(ensure_scratch(ctx, std::max(L.total, gs), s));
+    // (the smallest form of phase retrieval where there is no room for the staged one)
+    const size_t n = (size_t)n_fast * n_slow;
+    const bool staged = gs_persistent(n_fast, n_slow) || (gs_two(n_fast) && gs_two(n_slow));
+    int st = ensure_scratch(ctx, std::max(L.total, gs_layout(n, staged).total), s);
+    if (st == PH_ERR_OOM && staged) st = ensure_scratch(ctx, std::max(L.total, gs_layout(n, false).total), s);
+    PH_TRY(st);
     const float2 *tw = nullptr;
     PH_TRY(get_twiddles(ctx, n_fast, s, &tw));
     PH_TRY(get_twiddles(ctx, n_slow, s, &tw));
@@ -1791,21 +1816,22 @@ int32_t ph_phase_retrieval(ph_ctx *ctx, void *out, const float *holo1, const flo
         PH_LEAVE(ctx);
     }
     // The persistent staged passes (1024, 2048 and 4096) and the two-stage passes take
-    // the transfers as [kx][ky] rows and the amplitudes; a context whose budget has no
-    // room for them runs the one-shot passes where it did.  Two-stage where the
-    // persistent form does not exist: per pass, one-shot and two-stage, 12.6 and 3.0 us
-    // at 256^2, 12.3 and 5.8 at 512^2, 19.2 and 6.3 at 768^2, 43.5 and 28.7 at 1536^2;
-    // persistent and two-stage, 8.2 and 8.4 us at 1024^2, 28 and 45 at 2048^2, 149 and
-    // 163 at 4096^2 (there 64 values per thread leave 8 warps per SM).
-    const bool persistent = gs_row_staged(nx) && gs_col_staged(ny);
-    const size_t rows_bytes = n * (4 * sizeof(float2) + 2 * sizeof(float)) + 6 * kAlign;
-    const bool two_stage = !persistent && gs_two(nx) && gs_two(ny) && (ctx->budget == 0 || rows_bytes <= ctx->budget);
+    // the transfers as [kx][ky] rows and the amplitudes; a context that has no room for
+    // them (its budget, a capture, the device) runs the one-shot passes where it did.
+    // Two-stage where the persistent form does not exist: per pass, one-shot and
+    // two-stage, 12.6 and 3.0 us at 256^2, 12.3 and 5.8 at 512^2, 19.2 and 6.3 at 768^2,
+    // 43.5 and 28.7 at 1536^2; persistent and two-stage, 8.2 and 8.4 us at 1024^2, 28 and
+    // 45 at 2048^2, 149 and 163 at 4096^2 (there 64 values per thread leave 8 warps per SM).
+    const bool persistent = gs_persistent(nx, ny);
+    bool two_stage = !persistent && gs_two(nx) && gs_two(ny);
+    int st = ensure_scratch(ctx, gs_layout(n, persistent || two_stage).total, s);
+    if (st == PH_ERR_OOM && two_stage) {
+        two_stage = false;
+        st = ensure_scratch(ctx, gs_layout(n, false).total, s);
+    }
+    PH_TRY(st);
     const bool staged = persistent || two_stage;
-    Arena a;
-    const size_t oa = a.take<float2>(n), ob = a.take<float2>(n);
-    const size_t oh = staged ? a.take<float2>(n) : 0, ohi = staged ? a.take<float2>(n) : 0;
-    const size_t oa1 = staged ? a.take<float>(n) : 0, oa2 = staged ? a.take<float>(n) : 0;
-    PH_TRY(ensure_scratch(ctx, a.off, s));
+    const auto [oa, ob, oh, ohi, oa1, oa2, total] = gs_layout(n, staged);
     float2 *bufa = at<float2>(ctx, oa), *bufb = at<float2>(ctx, ob);
     float2 *ht = staged ? at<float2>(ctx, oh) : nullptr, *hti = staged ? at<float2>(ctx, ohi) : nullptr;
     float *amp1 = staged ? at<float>(ctx, oa1) : nullptr, *amp2 = staged ? at<float>(ctx, oa2) : nullptr;
