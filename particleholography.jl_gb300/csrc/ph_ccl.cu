@@ -13,6 +13,7 @@
 // once it points at its root is the reference's label.  Every loop is bounded by
 // an iteration limit that raises the context's error flag instead of running on.
 #include <cstdint>
+#include <type_traits>
 #include <cuda_runtime.h>
 
 namespace ph {
@@ -114,20 +115,22 @@ __device__ __forceinline__ void ccl_lhook(int *p, int a, int b, int64_t limit, i
     }
 }
 
-// Each 32 x 32 tile on its own, one warp per tile.  What bounds it is memory
-// (read the image, write the labels), as long as a tile costs few instructions:
-//  - an empty tile writes zeros (most tiles of a thresholded volume);
-//  - a tile with one foreground value is a bit mask, one 32-bit word per row, lane
-//    = row.  Its nodes are the runs of each row: a run starts at the first run of
-//    the row above that it touches (its range widened by one, 8-connectivity) and
-//    hooks the others; then pointer doubling over the runs;
-//  - a tile of several values is hooked pixel by pixel.
-// Inside a tile, row-major order is linear order, so a local root is the minimum
-// index of its local component.  A row that starts a slice has no row above.
-// (100 x 1024^2 Bool, about 1 % foreground: 0.32 ms with one 256-thread CTA per
-// tile and pixel-wise hooks, 0.137 ms in this form, where the copy rate allows
-// 0.077; what follows it, border, compression and background, 0.66 ms before and
-// 0.10 ms now.)
+// Each 32 x 32 tile on its own, one warp per tile, lane = column.  What bounds it is
+// memory (read the image, write the labels) where most tiles are empty, as in a
+// thresholded volume, and the latency of one warp's instructions in a small image.
+// The tile's rows are read first (an empty tile writes zeros); then the rows are
+// joined from the top, so that every pixel is given a root of the rows above:
+//  - a pixel takes the root of the equal pixel above it, or of an upper neighbour on
+//    a diagonal; a run of equal pixels takes that of its first pixel that has one, or
+//    is a root itself at its first pixel;
+//  - where a run meets a second root, the two trees are hooked, and the roots that
+//    the lanes hold are found again.
+// So the trees are about one level deep, and what a row costs does not depend on how
+// many runs it holds: with lane = row, each lane walking its own runs, stripes at 512^2
+// took 71 us, now 28 (256 threads per tile, pixel by pixel: 29), and 5 % noise at 2048^2
+// 56 and 40 (72).  Inside a tile, row-major order is linear order, so a local
+// root is the minimum index of its local component.  A row that starts a slice has no
+// row above.
 template <class T>
 struct CclLocal {
     static constexpr int WARPS = sizeof(T) == 1 ? 8 : 4;
@@ -136,146 +139,126 @@ struct CclLocal {
 template <class T>
 __global__ void __launch_bounds__(CclLocal<T>::WARPS * 32)
     k_ccl_local(const T *__restrict__ img, uint32_t *__restrict__ lab, uint32_t rows, uint32_t cols, uint32_t tiles_x,
-                uint64_t tiles, uint32_t slice_rows, int64_t limit, int *err) {
+                uint32_t tiles, uint32_t slice_rows, int64_t limit, int *err) {
     constexpr int WARPS = CclLocal<T>::WARPS;
+    constexpr bool BOOL = sizeof(T) == 1;
+    constexpr unsigned ALL = 0xffffffffu;
     __shared__ int s_parent[WARPS][kTile * kTile];
-    __shared__ T s_value[sizeof(T) == 1 ? 1 : WARPS][sizeof(T) == 1 ? 1 : kTile * kTile];
+    __shared__ T s_value[BOOL ? 1 : WARPS][BOOL ? 1 : kTile * kTile];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint64_t tile = (uint64_t)blockIdx.x * WARPS + warp;
+    const uint32_t tile = blockIdx.x * WARPS + warp;
     if (tile >= tiles) return;
     int *sp = s_parent[warp];
-    const uint32_t y0 = (uint32_t)(tile / tiles_x) * kTile, x0 = (uint32_t)(tile % tiles_x) * kTile;
-    const uint32_t nrows = min((uint32_t)kTile, rows - y0);
+    T *sv = s_value[BOOL ? 0 : warp];
+    const uint32_t y0 = tile / tiles_x * kTile, x0 = tile % tiles_x * kTile;
+    const int nrows = (int)min((uint32_t)kTile, rows - y0);
     const bool xin = x0 + lane < cols;
     const size_t at = (size_t)y0 * cols + x0 + lane;   // pixel (0, lane) of the tile
-    // lane = column while the rows are read; the ballots leave row r's mask in lane r
-    T v[sizeof(T) == 1 ? 1 : kTile];
-    uint32_t m = 0;
-    T first = T(0);
+    uint32_t mask = 0;                                 // lane r: the foreground of row r
 #pragma unroll
     for (int r = 0; r < kTile; ++r) {
         const T q = (xin && r < nrows) ? img[at + (size_t)r * cols] : T(0);
-        const uint32_t b = __ballot_sync(0xffffffffu, ccl_fg<T>(q));
-        if (lane == r) m = b;
-        if constexpr (sizeof(T) != 1) {
-            v[r] = q;
-            if (!ccl_fg<T>(first)) first = ccl_fg<T>(q) ? q : first;
-        }
+        const uint32_t b = __ballot_sync(ALL, ccl_fg<T>(q));
+        if (lane == r) mask = b;
+        if constexpr (!BOOL) sv[r * kTile + lane] = q;
     }
-    if (!__any_sync(0xffffffffu, m != 0)) {
+    if (!__any_sync(ALL, mask != 0)) {
         if (xin)
-            for (uint32_t r = 0; r < nrows; ++r) lab[at + (size_t)r * cols] = 0;
+            for (int r = 0; r < nrows; ++r) lab[at + (size_t)r * cols] = 0;
         return;
     }
-    // lane = row from here: its index within its slice
-    const uint32_t yl = (y0 + lane) % slice_rows;
-    bool one_value = true;
-    if constexpr (sizeof(T) != 1) {
-        const T v0 = __shfl_sync(0xffffffffu, first, __ffs(__ballot_sync(0xffffffffu, ccl_fg<T>(first))) - 1);
-#pragma unroll
-        for (int r = 0; r < kTile; ++r) one_value = one_value && (!ccl_fg<T>(v[r]) || ccl_eq(v[r], v0));
-        one_value = __all_sync(0xffffffffu, one_value);
+    __syncwarp();
+    const uint32_t yl = (y0 + lane) % slice_rows;   // lane r: the index of row r within its slice
+    const uint32_t first = __shfl_sync(ALL, yl, 0);
+    if (BOOL && __all_sync(ALL, mask == ALL && yl == first + lane)) {   // one component: no joining
+        const uint32_t l = first * cols + x0 + 1u;
+        for (int r = 0; r < kTile; ++r) lab[at + (size_t)r * cols] = l;
+        return;
     }
-    if (one_value) {
-        uint32_t up = __shfl_up_sync(0xffffffffu, m, 1);
-        if (lane == 0 || yl == 0) up = 0;
-        const uint32_t starts = m & ~(m << 1), up_starts = up & ~(up << 1);
-        // the bits of up that the run starting at s touches; the run of up that holds bit b
-        const auto touching = [&](int s) {
-            const uint32_t run = m & ~(m + (1u << s)) & (~0u << s);   // s and the ones above it
-            return up & (run | (run << 1) | (run >> 1));
-        };
-        const auto up_run = [&](int b) { return 31 - __clz(up_starts & ((2u << b) - 1u)); };
-        for (uint32_t t = starts; t; t &= t - 1) {
-            const int s = __ffs(t) - 1;
-            const uint32_t ov = touching(s);
-            sp[lane * kTile + s] = ov ? (lane - 1) * kTile + up_run(__ffs(ov) - 1) : lane * kTile + s;
+    const uint32_t tops = __ballot_sync(ALL, yl == 0), filled = __ballot_sync(ALL, mask != 0);
+    const uint32_t upto = ~0u >> (31 - lane);       // this lane and the ones before it
+    int root = 0;                                   // of the pixel above, where that is foreground
+    uint32_t up = 0;
+    T above = T(0);
+    for (uint32_t left_over = filled; left_over; left_over &= left_over - 1) {
+        const int r = __ffs(left_over) - 1;
+        const uint32_t m = __shfl_sync(ALL, mask, r);
+        const T v = BOOL ? T(0) : sv[r * kTile + lane];
+        if (((tops | ~(filled << 1)) >> r) & 1u) up = 0;   // the slice's first row, or an empty row above
+        const bool fg = (m >> lane) & 1u;
+        // the equal neighbours: above, above left, above right; the first pixels of the
+        // runs, and the pixels that have an equal one above
+        bool n = fg && ((up >> lane) & 1u), nw = fg && (((up << 1) >> lane) & 1u), ne = fg && (((up >> 1) >> lane) & 1u);
+        uint32_t starts, held;
+        if constexpr (BOOL) {
+            starts = m & ~(m << 1);
+            held = m & (up | (up << 1) | (up >> 1));
+        } else {
+            const T *sr = sv + r * kTile;
+            const int left = max(lane - 1, 0), row_up = r > 0 ? kTile : 0;
+            n = n && ccl_eq(above, v);
+            nw = nw && ccl_eq(sr[left - row_up], v);
+            ne = ne && ccl_eq(sr[min(lane + 1, 31) - row_up], v);
+            starts = __ballot_sync(ALL, fg && !(((m << 1) >> lane) & 1u && ccl_eq(sr[left], v)));
+            held = __ballot_sync(ALL, n || nw || ne);
         }
-        __syncwarp();
-        for (uint32_t t = starts; t; t &= t - 1) {
-            const int s = __ffs(t) - 1;
-            uint32_t ov = touching(s);
-            for (bool linked = true; ov; linked = false) {   // the first run is the parent already
-                const int u = up_run(__ffs(ov) - 1);
-                if (!linked) ccl_lhook(sp, lane * kTile + s, (lane - 1) * kTile + u, limit, err);
-                ov &= up + (1u << u);                         // past that run
-            }
-        }
-        __syncwarp();
-        for (int i = 0; i < 5; ++i) {   // pointer doubling: the usual depth, a row each
-            for (uint32_t t = starts; t; t &= t - 1) {
-                const int n = lane * kTile + __ffs(t) - 1;
-                sp[n] = sp[sp[n]];
-            }
+        const int rw = __shfl_up_sync(ALL, root, 1), re = __shfl_down_sync(ALL, root, 1);
+        const bool has = n || nw || ne;
+        const int cand = n ? root : nw ? rw : re;   // (an equal pixel above joins both diagonals)
+        // the run of this pixel, [s, e), and the first pixel of it that has a root
+        const int s = max(31 - __clz(starts & upto), 0);
+        const uint32_t past = (starts | ~m) & ~upto;
+        const uint32_t in_run = fg ? held & (past ? (1u << (__ffs(past) - 1)) - 1u : ALL) & (ALL << s) : 0u;
+        const int from = __shfl_sync(ALL, cand, in_run ? __ffs(in_run) - 1 : lane);
+        root = in_run ? from : r * kTile + s;
+        sp[r * kTile + lane] = root;
+        // a second root: of another pixel of the run, or this pixel's other diagonal
+        const bool second = has && cand != root, other = !n && nw && ne && re != rw;
+        if (__any_sync(ALL, second || other)) {
+            const int before = __shfl_up_sync(ALL, cand, 1);   // (once for neighbours that share it)
+            const bool shared = lane != s && ((held << 1) >> lane & 1u) && before == cand;
+            __syncwarp();   // (the earlier rows' parents)
+            if (second && !shared) ccl_lhook(sp, cand, root, limit, err);
+            if (other) ccl_lhook(sp, re, root, limit, err);
             __syncwarp();
+            if (fg) root = ccl_lroot(sp, root, limit, err);
         }
-        for (uint32_t t = starts; t; t &= t - 1) {   // (each writes its own root only)
-            const int n = lane * kTile + __ffs(t) - 1;
-            sp[n] = ccl_lroot(sp, n, limit, err);
-        }
-        __syncwarp();
-        for (int r = 0; r < (int)nrows; ++r) {
-            const uint32_t mr = __shfl_sync(0xffffffffu, m, r), yr = __shfl_sync(0xffffffffu, yl, r);
-            uint32_t l = 0;
-            if ((mr >> lane) & 1u) {
-                const int q = sp[r * kTile + 31 - __clz((mr & ~(mr << 1)) & ((2u << lane) - 1u))];
-                l = (yr - (uint32_t)(r - q / kTile)) * cols + x0 + (uint32_t)(q % kTile) + 1u;
-            }
-            if (xin) lab[at + (size_t)r * cols] = l;
-        }
-        return;
+        up = m;
+        above = v;
     }
-    if constexpr (sizeof(T) != 1) {   // several values: pixel by pixel, lane = column
-        T *sv = s_value[warp];
+    __syncwarp();
+    for (int r0 = 0; r0 < nrows; r0 += 4) {   // (four rows' walks, nearly all of one step, side by side)
+        int q[4], g[4];
+        bool on[4];
+        if (((filled >> r0) & 15u) == 0) {
 #pragma unroll
-        for (int r = 0; r < kTile; ++r) sv[r * kTile + lane] = v[r];
-        __syncwarp();
-        for (int r = 0; r < kTile; ++r) {
-            const int l = r * kTile + lane;
-            const T q = sv[l];
-            const bool top = r == 0 || __shfl_sync(0xffffffffu, yl, r) == 0;
-            int p = l;
-            if (ccl_fg<T>(q)) {
-                if (lane > 0 && ccl_eq(sv[l - 1], q)) p = l - 1;
-                if (!top) {
-                    if (lane + 1 < kTile && ccl_eq(sv[l - kTile + 1], q)) p = l - kTile + 1;
-                    if (ccl_eq(sv[l - kTile], q)) p = l - kTile;
-                    if (lane > 0 && ccl_eq(sv[l - kTile - 1], q)) p = l - kTile - 1;
-                }
-            }
-            sp[l] = p;
+            for (int i = 0; i < 4; ++i)
+                if (xin && r0 + i < nrows) lab[at + (size_t)(r0 + i) * cols] = 0;
+            continue;
         }
-        __syncwarp();
-        for (int r = 0; r < kTile; ++r) {
-            const int l = r * kTile + lane;
-            const T q = sv[l];
-            const bool top = r == 0 || __shfl_sync(0xffffffffu, yl, r) == 0;
-            if (!ccl_fg<T>(q)) continue;
-            if (lane > 0 && ccl_eq(sv[l - 1], q)) ccl_lhook(sp, l, l - 1, limit, err);
-            if (!top) {
-                if (lane > 0 && ccl_eq(sv[l - kTile - 1], q)) ccl_lhook(sp, l, l - kTile - 1, limit, err);
-                if (ccl_eq(sv[l - kTile], q)) ccl_lhook(sp, l, l - kTile, limit, err);
-                if (lane + 1 < kTile && ccl_eq(sv[l - kTile + 1], q)) ccl_lhook(sp, l, l - kTile + 1, limit, err);
-            }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            on[i] = (__shfl_sync(ALL, mask, r0 + i) >> lane) & 1u;
+            q[i] = on[i] ? sp[(r0 + i) * kTile + lane] : 0;
         }
-        __syncwarp();
-        for (int r = 0; r < (int)nrows; ++r) {
-            const int l = r * kTile + lane;
-            const uint32_t yr = __shfl_sync(0xffffffffu, yl, r);
-            uint32_t out = 0;
-            if (ccl_fg<T>(sv[l])) {
-                const int q = ccl_lroot(sp, l, limit, err);
-                out = (yr - (uint32_t)(r - q / kTile)) * cols + x0 + (uint32_t)(q % kTile) + 1u;
-            }
-            if (xin) lab[at + (size_t)r * cols] = out;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) g[i] = on[i] ? sp[q[i]] : 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = r0 + i;
+            const uint32_t yr = __shfl_sync(ALL, yl, r);
+            if (g[i] != q[i]) q[i] = ccl_lroot(sp, g[i], limit, err);
+            const uint32_t out = on[i] ? (yr - (uint32_t)(r - q[i] / kTile)) * cols + x0 + (uint32_t)(q[i] % kTile) + 1u : 0u;
+            if (xin && r < nrows) lab[at + (size_t)r * cols] = out;
         }
     }
 }
 
 // ---- merge across tile borders: the pairs whose earlier neighbour lies in
 // another tile (W, NW of the left column; NW, N, NE of the top row; NE of the
-// right column) are hooked in the global parents.  One warp per tile, its 94
-// border pixels in three rounds.  Within a warp, pairs whose current parents are
+// right column) are hooked in the global parents.  One warp per tile, whose three
+// sides are read together; or one per tile and side (gridDim.y = 3) where the tiles
+// alone would not fill the device.  Within a warp, pairs whose current parents are
 // the same two nodes link the same two trees, so one lane of each such set hooks
 // (between tiles of one value, as in a near-total foreground, one hook per
 // neighbour tile instead of one per border pixel).
@@ -294,75 +277,122 @@ __device__ __forceinline__ void ccl_hook_dedup(uint32_t *lab, bool cond, size_t 
 
 template <class T>
 __global__ void __launch_bounds__(256)
-    k_ccl_border(const T *__restrict__ img, uint32_t *lab, uint32_t rows, uint32_t cols, uint32_t tiles_x, uint64_t tiles,
+    k_ccl_border(const T *__restrict__ img, uint32_t *lab, uint32_t rows, uint32_t cols, uint32_t tiles_x, uint32_t tiles,
                  uint32_t slice_rows, int64_t limit, int *err) {
-    const uint64_t tile = (uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    const uint32_t tile = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (tile >= tiles) return;
     const int lane = threadIdx.x & 31;
-    const uint32_t y0 = (uint32_t)(tile / tiles_x) * kTile, x0 = (uint32_t)(tile % tiles_x) * kTile;
-    // lane = column of the top row, then row of the left and of the right column
+    const uint32_t y0 = tile / tiles_x * kTile, x0 = tile % tiles_x * kTile;
+    // lane = column of the top row, or row of the left or the right column
+    bool fg[3];
+    T v[3];
+    bool any = false;
 #pragma unroll
-    for (int round = 0; round < 3; ++round) {
-        const uint32_t y = y0 + (round == 0 ? 0 : lane), x = x0 + (round == 0 ? lane : round == 1 ? 0 : kTile - 1);
-        const bool on = y < rows && x < cols && (round == 0 || lane > 0);
-        const size_t i = (size_t)y * cols + x;
-        const T v = on ? img[i] : T(0);
-        const bool fg = on && ccl_fg<T>(v);
-        if (!__any_sync(0xffffffffu, fg)) continue;
+    for (int side = 0; side < 3; ++side) {
+        const uint32_t y = y0 + (side == 0 ? 0 : lane), x = x0 + (side == 0 ? lane : side == 1 ? 0 : kTile - 1);
+        const bool on = (gridDim.y == 1 || side == (int)blockIdx.y) && y < rows && x < cols && (side == 0 || lane > 0);
+        v[side] = on ? img[(size_t)y * cols + x] : T(0);
+        fg[side] = on && ccl_fg<T>(v[side]);
+        any = any || fg[side];
+    }
+    if (!__any_sync(0xffffffffu, any)) return;
+#pragma unroll
+    for (int side = 0; side < 3; ++side) {
+        if (!__any_sync(0xffffffffu, fg[side])) continue;
+        const uint32_t y = y0 + (side == 0 ? 0 : lane), x = x0 + (side == 0 ? lane : side == 1 ? 0 : kTile - 1);
         const uint32_t yl = y % slice_rows;
-        const size_t base = (size_t)(y - yl) * cols, u = i - cols;
-        const bool up = fg && yl != 0;
-        if (round == 0) {
-            ccl_hook_dedup(lab, fg && lane == 0 && x > 0 && ccl_eq(img[i - 1], v), base, i, i - 1, limit, err);
-            ccl_hook_dedup(lab, up && x > 0 && ccl_eq(img[u - 1], v), base, i, u - 1, limit, err);
-            ccl_hook_dedup(lab, up && ccl_eq(img[u], v), base, i, u, limit, err);
-            ccl_hook_dedup(lab, up && x + 1 < cols && ccl_eq(img[u + 1], v), base, i, u + 1, limit, err);
-        } else if (round == 1) {
-            ccl_hook_dedup(lab, fg && x > 0 && ccl_eq(img[i - 1], v), base, i, i - 1, limit, err);
-            ccl_hook_dedup(lab, up && x > 0 && ccl_eq(img[u - 1], v), base, i, u - 1, limit, err);
+        const size_t i = (size_t)y * cols + x, base = (size_t)(y - yl) * cols, u = i - cols;
+        const bool up = fg[side] && yl != 0;
+        if (side == 0) {
+            ccl_hook_dedup(lab, fg[side] && lane == 0 && x > 0 && ccl_eq(img[i - 1], v[side]), base, i, i - 1, limit, err);
+            ccl_hook_dedup(lab, up && x > 0 && ccl_eq(img[u - 1], v[side]), base, i, u - 1, limit, err);
+            ccl_hook_dedup(lab, up && ccl_eq(img[u], v[side]), base, i, u, limit, err);
+            ccl_hook_dedup(lab, up && x + 1 < cols && ccl_eq(img[u + 1], v[side]), base, i, u + 1, limit, err);
+        } else if (side == 1) {
+            ccl_hook_dedup(lab, fg[side] && x > 0 && ccl_eq(img[i - 1], v[side]), base, i, i - 1, limit, err);
+            ccl_hook_dedup(lab, up && x > 0 && ccl_eq(img[u - 1], v[side]), base, i, u - 1, limit, err);
         } else {
-            ccl_hook_dedup(lab, up && x + 1 < cols && ccl_eq(img[u + 1], v), base, i, u + 1, limit, err);
+            ccl_hook_dedup(lab, up && x + 1 < cols && ccl_eq(img[u + 1], v[side]), base, i, u + 1, limit, err);
         }
     }
 }
 
 // Every foreground pixel takes its root's label.  The foreground is found in the
-// smaller array: the image where a pixel is one byte (16 per load, VEC), else the
-// labels (4 per load), both 16-byte aligned.
-template <class T, bool VEC>
+// smaller array: the image where a pixel is one byte (K = 16 per thread, or 4 where 16
+// would leave most of the device without a thread), else the labels (4 per thread);
+// K-byte or 16-byte aligned, else K = 1.  A thread's pixels follow their parents
+// together, so that the walks cost the latency of the deepest (one after the other
+// they took 15 us of a 100^2 image's 40); a run of equal labels walks once.
+template <class T, int K>
 __global__ void __launch_bounds__(256)
     k_ccl_flatten(const T *__restrict__ img, uint32_t *lab, int64_t n, int64_t slice_n, int64_t limit, int *err) {
-    constexpr int K = !VEC ? 1 : sizeof(T) == 1 ? 16 : 4;
-    const int64_t i0 = ((int64_t)blockIdx.x * 256 + threadIdx.x) * K;
-    if (i0 >= n) return;
-    uint32_t last = 0, last_root = 0;
-    int64_t base = (i0 / slice_n) * slice_n;
-    const auto flatten = [&](int64_t i) {
-        if (i - base >= slice_n) { base = (i / slice_n) * slice_n; last = 0; }
-        uint32_t *p = lab + base - 1;   // node of the slice -> its parent
-        const uint32_t l = lab[i];
-        if (l != last) { last = l; last_root = ccl_root(p, l, limit, err); }   // a run's pixels hold one label
-        if (last_root != l) lab[i] = last_root;
-    };
-    if constexpr (!VEC) {
-        if (ccl_fg<T>(img[i0])) flatten(i0);
-    } else if constexpr (sizeof(T) == 1) {
-        if (i0 + K <= n) {
-            const uint4 q = __ldg(reinterpret_cast<const uint4 *>(img + i0));
-            if ((q.x | q.y | q.z | q.w) == 0) return;
+    const int64_t i = ((int64_t)blockIdx.x * 256 + threadIdx.x) * K;
+    if (i >= n) return;
+    uint32_t l[K], cur[K];
+    const bool whole = i + K <= n;
+    if constexpr (K > 1 && sizeof(T) == 1) {
+        uint32_t word[K / 4] = {};
+        if (whole) {
+            if constexpr (K == 16) {
+                const uint4 q = __ldg(reinterpret_cast<const uint4 *>(img + i));
+                word[0] = q.x; word[1] = q.y; word[2] = q.z; word[3] = q.w;
+                if ((q.x | q.y | q.z | q.w) == 0) return;
+            } else {
+                word[0] = __ldg(reinterpret_cast<const uint32_t *>(img + i));
+                if (word[0] == 0) return;
+            }
         }
-        for (int64_t w = i0; w < min(i0 + K, n); w += 4) {
-            if (w + 4 <= n && *reinterpret_cast<const uint32_t *>(img + w) == 0) continue;
-            for (int64_t i = w; i < min(w + 4, n); ++i)
-                if (ccl_fg<T>(img[i])) flatten(i);
+        const bool aligned = ((uintptr_t)lab & 15) == 0;
+#pragma unroll
+        for (int w = 0; w < K / 4; ++w) {
+            uint4 v = make_uint4(0, 0, 0, 0);
+            if (word[w] != 0) {
+                const uint32_t *at = lab + i + 4 * w;
+                if (aligned) v = *reinterpret_cast<const uint4 *>(at);
+                else v = make_uint4(at[0], at[1], at[2], at[3]);
+            }
+            l[4 * w] = v.x; l[4 * w + 1] = v.y; l[4 * w + 2] = v.z; l[4 * w + 3] = v.w;
+        }
+    } else if constexpr (K > 1) {
+        if (whole) {
+            const uint4 v = *reinterpret_cast<const uint4 *>(lab + i);
+            if ((v.x | v.y | v.z | v.w) == 0) return;
+            l[0] = v.x; l[1] = v.y; l[2] = v.z; l[3] = v.w;
         }
     } else {
-        if (i0 + K <= n) {
-            const uint4 q = *reinterpret_cast<const uint4 *>(lab + i0);
-            if ((q.x | q.y | q.z | q.w) == 0) return;
+        l[0] = lab[i];
+    }
+    const int64_t base = (i / slice_n) * slice_n;
+    if (!whole || i + K > base + slice_n) {   // the array's end, or two slices
+        for (int64_t j = i; j < i + K && j < n; ++j) {
+            const uint32_t v = lab[j];
+            if (v != 0) lab[j] = ccl_root(lab + (j / slice_n) * slice_n - 1, v, limit, err);
         }
-        for (int64_t i = i0; i < min(i0 + K, n); ++i)
-            if (lab[i] != 0) flatten(i);
+        return;
+    }
+    // node of the slice -> its parent (roots do not change here, and whatever a pixel held
+    // before is an ancestor of it, so reads may come from L1)
+    uint32_t *p = lab + base - 1;
+#pragma unroll
+    for (int k = 0; k < K; ++k) cur[k] = l[k];
+    bool walking = true;
+    for (int64_t it = 0; walking; ++it) {
+        if (it > limit) { atomicExch(err, 1); break; }
+        walking = false;
+        uint32_t next[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            next[k] = l[k] != 0 && (k == 0 || l[k] != l[k > 0 ? k - 1 : 0]) ? __ldca(p + cur[k]) : cur[k];
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            walking = walking || next[k] < cur[k];
+            cur[k] = next[k];
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        if (k > 0 && l[k] == l[k > 0 ? k - 1 : 0]) cur[k] = cur[k > 0 ? k - 1 : 0];
+        if (cur[k] != l[k]) lab[i + k] = cur[k];
     }
 }
 
@@ -370,21 +400,28 @@ template <class T>
 static cudaError_t ccl_run(const T *img, uint32_t *lab, int64_t rows, int64_t cols, int64_t slice_rows, int64_t limit,
                            int *err, cudaStream_t s, int64_t *launches) {
     const int64_t n = rows * cols;
-    const uint64_t tiles_x = (uint64_t)(cols + kTile - 1) / kTile, tiles = tiles_x * (uint64_t)((rows + kTile - 1) / kTile);
+    // (fewer than 2^32 pixels: fewer than 2^28 tiles)
+    const uint32_t tiles_x = (uint32_t)((cols + kTile - 1) / kTile), tiles = tiles_x * (uint32_t)((rows + kTile - 1) / kTile);
     constexpr int W = CclLocal<T>::WARPS;
     k_ccl_local<T><<<(unsigned)((tiles + W - 1) / W), W * 32, 0, s>>>(img, lab, (uint32_t)rows, (uint32_t)cols,
-                                                                     (uint32_t)tiles_x, tiles, (uint32_t)slice_rows,
+                                                                     tiles_x, tiles, (uint32_t)slice_rows,
                                                                      limit, err);
-    k_ccl_border<T><<<(unsigned)((tiles + 7) / 8), 256, 0, s>>>(img, lab, (uint32_t)rows, (uint32_t)cols,
-                                                                (uint32_t)tiles_x, tiles, (uint32_t)slice_rows, limit,
+    k_ccl_border<T><<<dim3((tiles + 7) / 8, tiles <= 3072 ? 3 : 1), 256, 0, s>>>(img, lab, (uint32_t)rows, (uint32_t)cols,
+                                                                tiles_x, tiles, (uint32_t)slice_rows, limit,
                                                                 err);
-    const void *scanned = sizeof(T) == 1 ? static_cast<const void *>(img) : static_cast<const void *>(lab);
     const int64_t slice_n = slice_rows * cols;
-    if (((uintptr_t)scanned & 15) == 0) {
-        const int64_t k = sizeof(T) == 1 ? 16 : 4;
-        k_ccl_flatten<T, true><<<(unsigned)((n + 256 * k - 1) / (256 * k)), 256, 0, s>>>(img, lab, n, slice_n, limit, err);
+    const auto flatten = [&](auto k) {
+        constexpr int K = decltype(k)::value;
+        k_ccl_flatten<T, K><<<(unsigned)((n + 256 * K - 1) / (256 * K)), 256, 0, s>>>(img, lab, n, slice_n, limit, err);
+    };
+    const uintptr_t at = sizeof(T) == 1 ? (uintptr_t)img : (uintptr_t)lab;
+    if constexpr (sizeof(T) == 1) {
+        if (n >= (1 << 20) && at % 16 == 0) flatten(std::integral_constant<int, 16>{});
+        else if (at % 4 == 0) flatten(std::integral_constant<int, 4>{});
+        else flatten(std::integral_constant<int, 1>{});
     } else {
-        k_ccl_flatten<T, false><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(img, lab, n, slice_n, limit, err);
+        if (at % 16 == 0) flatten(std::integral_constant<int, 4>{});
+        else flatten(std::integral_constant<int, 1>{});
     }
     *launches += 3;
     return cudaGetLastError();

@@ -64,3 +64,28 @@ def test_several_values_in_a_tile(ph, cuda):
     img[20:50, 10:80] = 2.5
     labels = ph.cu_connected_component_labeling(torch.from_numpy(img).to(cuda), reference_grid=False)
     assert np.array_equal(to_np(labels.view(torch.int32)).astype(np.uint32), occl.connected_component_labeling(img))
+
+
+# more pixels than 16 per thread of the last pass need (2^20), more tiles than get a warp per side (3072)
+@pytest.mark.parametrize("kind", ["comb", "diagonal", "0.02", "0.4", "0.6"])
+@pytest.mark.parametrize("shape", [(1, 1100, 1003), (1, 2000, 2003), (5, 700, 999)])
+@pytest.mark.parametrize("dtype,offset", [(torch.bool, 0), (torch.bool, 4), (torch.float32, 0), (torch.float32, 1)])
+def test_large_images(ph, cuda, kind, shape, dtype, offset):
+    vol = _pattern(kind, shape, np.random.default_rng(shape[1]))
+    buf = torch.zeros(vol.size + 16, dtype=dtype, device=cuda)
+    img = buf[offset:offset + vol.size].view(shape)
+    img.copy_(torch.from_numpy(vol))
+    got = to_np(ph.cu_connected_component_labeling_batch(img).view(torch.int32)).astype(np.uint32)
+    for k in range(shape[0]):
+        assert np.array_equal(got[k], occl.connected_component_labeling(vol[k].astype(np.float32)))
+
+
+@pytest.mark.parametrize("cols,rows", [(45, 70), (96, 33), (130, 31)])
+def test_runs_of_several_values(ph, cuda, cols, rows):
+    """Runs that end at another value, roots that meet in one run from both sides."""
+    rng = np.random.default_rng(cols)
+    img = rng.integers(1, 3, (rows, cols)).astype(np.float32)
+    img[::3, ::2] = 0
+    img[5:9] = np.where(np.arange(cols) % 11 < 9, 1.0, 2.0)
+    labels = ph.cu_connected_component_labeling(torch.from_numpy(img).to(cuda), reference_grid=False)
+    assert np.array_equal(to_np(labels.view(torch.int32)).astype(np.uint32), occl.connected_component_labeling(img))
