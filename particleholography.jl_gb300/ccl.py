@@ -85,16 +85,25 @@ def cu_bounding_rectangles(labels: torch.Tensor) -> np.ndarray:
     ctx = _lib.default_context(dev)
     s = torch.cuda.current_stream(dev).cuda_stream
     count = ctypes.c_int64(0)
-    room = _ROOM
+    room = _room(lab.numel())
     while True:   # a second call only where there are more components than room
         out = np.empty((room, 5), dtype=np.int64)
         ctx.call("ph_ccl_boxes", out.ctypes.data, room, ctypes.byref(count), lab.data_ptr(), slices, rows, cols, s)
         if count.value <= room:
-            return out[:count.value]
+            return _first(out, count.value)
         room = count.value
 
 
-_ROOM = 1 << 16   # components a query makes room for before it knows their number
+def _room(labels: int) -> int:
+    """Components a query of so many labels makes room for before it knows their number.  A
+    second query costs two passes over the labels, room that is not enough 3 ns per
+    component; up to 2048 come back with their number."""
+    return min(max(labels >> 12, 1 << 11), 1 << 14)
+
+
+def _first(found: np.ndarray, count: int) -> np.ndarray:
+    """The rows that were filled, in an array of their own where room is left over."""
+    return found if count == len(found) else found[:count].copy()
 
 
 def _labels_on_device(labels) -> torch.Tensor:
@@ -126,7 +135,7 @@ def count_labels(labels) -> int:
 def cu_find_valid_labels(labels) -> np.ndarray:
     """ccl.jl:224-238: sorted 1-based root indices as a host Int64 vector."""
     labels = _labels_on_device(labels)
-    c, buf = _roots(labels, _ROOM)
-    if c > _ROOM:
+    c, buf = _roots(labels, _room(labels.numel()))
+    if c > len(buf):
         c, buf = _roots(labels, c)
-    return buf[:c]
+    return _first(buf, c)

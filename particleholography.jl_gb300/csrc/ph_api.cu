@@ -3322,9 +3322,10 @@ int32_t ph_ccl_batch(ph_ctx *ctx, uint32_t *labels, const void *img, int32_t img
 
 // Roots (and optionally their bounding boxes) of labels holding `slices`
 // images of rows x cols; out_host gets `per` int64 per root.  Synchronises: once
-// where there are at most kHeadRoots roots (their count, the roots and boxes
-// come back together), twice up to kPinnedRoots: the scratch for so many is small
-// enough to take, and everything to compute, before their number is known.
+// where there are at most kHeadRoots roots and the caller asked for up to kPinnedRoots
+// (the count, the roots and boxes come back together), else twice.  So they are listed
+// before their number is known, where the scratch that the context holds has room for
+// as many as were asked for; a larger request is listed by the number that was counted.
 constexpr int64_t kHeadRoots = 2048, kPinnedRoots = 16384;
 constexpr size_t kRootHeader = 64;   // bytes: total, error word
 constexpr size_t kPinnedBytes = kRootHeader + (size_t)kPinnedRoots * (sizeof(long long) + 4 * sizeof(int));
@@ -3337,89 +3338,115 @@ static int roots_common(ph_ctx *ctx, const uint32_t *labels, int64_t slices, int
     *count_host = 0;
     const int64_t n = slices * rows * cols, slice_n = rows * cols;
     if (n == 0) return PH_OK;
+    capacity = std::max<int64_t>(capacity, 0);
     if (ctx->pinned == nullptr) PH_CUDA(cudaMallocHost(&ctx->pinned, kPinnedBytes), "cudaMallocHost");
     // pinned (and the start of the device copy): total, error word, then the roots; boxes
     auto *h_total = static_cast<unsigned long long *>(ctx->pinned);
     auto *h_roots = reinterpret_cast<long long *>(static_cast<char *>(ctx->pinned) + kRootHeader);
     int *h_box = reinterpret_cast<int *>(h_roots + kPinnedRoots);
     const int64_t nb = roots_blocks(n);
-
-    // Counts the roots and, with cap > 0, lists the first cap of them (and their
-    // boxes); copies the header, then roots and boxes into the arrays given.
-    const auto query = [&](int64_t cap, long long *roots, int *bx) -> int {
+    struct Layout { size_t counts, head, rank, box, total; };
+    const auto layout = [&](int64_t cap) {   // (the counts and the header sit at the same place for any cap)
         Arena a;
-        const size_t oc = a.take<unsigned>(nb);
-        const size_t oh = a.take<char>(kRootHeader + (size_t)cap * sizeof(long long));
-        const size_t orank = boxes && cap > 0 ? a.take<unsigned>((size_t)n) : 0;
-        const size_t obox = boxes ? a.take<int>((size_t)cap * 4) : 0;
-        PH_TRY(ensure_scratch(ctx, a.off, s));
-        unsigned *counts = at<unsigned>(ctx, oc);
-        auto *total = at<unsigned long long>(ctx, oh);
-        auto *d_roots = at<long long>(ctx, oh + kRootHeader);
+        Layout l{};
+        l.counts = a.take<unsigned>(nb);
+        l.head = a.take<char>(kRootHeader + (size_t)cap * sizeof(long long));
+        if (cap > 0 && boxes) {
+            l.rank = a.take<unsigned>((size_t)n);
+            l.box = a.take<int>((size_t)cap * 4);
+        }
+        l.total = a.off;
+        return l;
+    };
+    const auto count = [&](const Layout &l) -> int {
         int64_t nl = 0;
-        PH_TRY(cuda_status(ctx, roots_count_launch(labels, n, slice_n, counts, total,
+        PH_TRY(cuda_status(ctx, roots_count_launch(labels, n, slice_n, at<unsigned>(ctx, l.counts),
+                                                   at<unsigned long long>(ctx, l.head),
                                                    static_cast<const int *>(ctx->small), s, &nl), "root count"));
-        if (cap > 0)
-            PH_TRY(cuda_status(ctx, roots_write_launch(labels, n, slice_n, counts, total, d_roots, cap,
-                                                       boxes ? at<unsigned>(ctx, orank) : nullptr, s, &nl),
-                               "root write"));
-        if (cap > 0 && boxes)
-            PH_TRY(cuda_status(ctx, boxes_launch(labels, slices * rows, cols, rows, at<unsigned>(ctx, orank),
-                                                 at<int>(ctx, obox), cap, s, &nl), "boxes"));
         ctx->launches += nl;
-        const int64_t head = std::min(cap, kHeadRoots);
-        PH_CUDA(cudaMemcpyAsync(h_total, total, kRootHeader + sizeof(long long) * head, cudaMemcpyDeviceToHost, s),
-                "copy roots");
-        if (head > 0 && boxes)
-            PH_CUDA(cudaMemcpyAsync(h_box, at<int>(ctx, obox), sizeof(int) * 4 * head, cudaMemcpyDeviceToHost, s),
-                    "copy boxes");
-        PH_CUDA(cudaStreamSynchronize(s), "cudaStreamSynchronize");
-        if (h_total[1] != 0) {
-            cudaMemsetAsync(ctx->small, 0, sizeof(int), s);
-            set_err(ctx, "a labeling loop reached its iteration limit; labels are incomplete");
-            return PH_ERR_TIMEOUT;
-        }
-        if (roots != h_roots && head > 0) std::copy(h_roots, h_roots + head, roots);
-        if (bx != h_box && head > 0 && boxes) std::copy(h_box, h_box + 4 * head, bx);
-        const int64_t rest = std::min<int64_t>((int64_t)*h_total, cap) - head;
-        if (rest > 0) {
-            PH_CUDA(cudaMemcpyAsync(roots + head, d_roots + head, sizeof(long long) * rest, cudaMemcpyDeviceToHost, s),
-                    "copy roots");
-            if (boxes)
-                PH_CUDA(cudaMemcpyAsync(bx + 4 * head, at<int>(ctx, obox) + 4 * head, sizeof(int) * 4 * rest,
-                                        cudaMemcpyDeviceToHost, s), "copy boxes");
-            PH_CUDA(cudaStreamSynchronize(s), "cudaStreamSynchronize");
-        }
         return PH_OK;
     };
-    int64_t have = std::min({std::max<int64_t>(capacity, 0), kPinnedRoots, n});
-    int st = query(have, h_roots, h_box);
-    if (st == PH_ERR_OOM && have > 0) {   // no room for ranks and boxes: they are not needed if there is no root
-        const std::string why = ctx->err;
-        PH_TRY(query(0, nullptr, nullptr));
-        if (*h_total != 0) { ctx->err = why; return PH_ERR_OOM; }
-        st = PH_OK;
+    const auto list = [&](const Layout &l, int64_t cap) -> int {
+        int64_t nl = 0;
+        PH_TRY(cuda_status(ctx, roots_write_launch(labels, n, slice_n, at<unsigned>(ctx, l.counts),
+                                                   at<unsigned long long>(ctx, l.head),
+                                                   at<long long>(ctx, l.head + kRootHeader), cap,
+                                                   boxes ? at<unsigned>(ctx, l.rank) : nullptr, s, &nl), "root write"));
+        if (boxes)
+            PH_TRY(cuda_status(ctx, boxes_launch(labels, slices * rows, cols, rows, at<unsigned>(ctx, l.rank),
+                                                 at<int>(ctx, l.box), cap, s, &nl), "boxes"));
+        ctx->launches += nl;
+        return PH_OK;
+    };
+    const auto emit = [&](int64_t from, int64_t to, const long long *roots, const int *bx) {
+        for (int64_t r = from; r < to; ++r) {   // (root, x_min, y_min, x_max, y_max), 1-based; x = slow axis
+            if (!boxes) { out_host[r] = roots[r]; continue; }
+            out_host[5 * r] = roots[r];
+            for (int q = 0; q < 4; ++q) out_host[5 * r + 1 + q] = bx[4 * r + q] + 1;
+        }
+    };
+
+    int64_t have = capacity <= kPinnedRoots ? std::min(capacity, n) : 0;
+    if (layout(have).total > ctx->scratch_bytes) have = 0;
+    Layout l = layout(have);
+    PH_TRY(ensure_scratch(ctx, l.total, s));
+    PH_TRY(count(l));
+    if (have > 0) PH_TRY(list(l, have));
+    const int64_t head = std::min(have, kHeadRoots);
+    PH_CUDA(cudaMemcpyAsync(h_total, at<char>(ctx, l.head), kRootHeader + sizeof(long long) * head,
+                            cudaMemcpyDeviceToHost, s), "copy roots");
+    if (head > 0 && boxes)
+        PH_CUDA(cudaMemcpyAsync(h_box, at<int>(ctx, l.box), sizeof(int) * 4 * head, cudaMemcpyDeviceToHost, s),
+                "copy boxes");
+    PH_CUDA(cudaStreamSynchronize(s), "cudaStreamSynchronize");
+    if (h_total[1] != 0) {
+        cudaMemsetAsync(ctx->small, 0, sizeof(int), s);
+        set_err(ctx, "a labeling loop reached its iteration limit; labels are incomplete");
+        return PH_ERR_TIMEOUT;
     }
-    PH_TRY(st);
-    const int64_t total = (int64_t)*h_total, want = std::min(total, std::max<int64_t>(capacity, 0));
+    const int64_t total = (int64_t)*h_total, want = std::min(total, capacity);
     *count_host = total;
-    const long long *roots = h_roots;
-    const int *bx = h_box;
+    int64_t done = 0;   // of the wanted roots, those in out_host
+    if (have > 0) {
+        done = std::min(want, head);
+        emit(0, done, h_roots, h_box);
+    } else if (want > 0) {
+        l = layout(want);
+        if (l.total > ctx->scratch_bytes) {
+            // more than the call needs where there is room, so that the next one lists at once
+            const size_t next = layout(std::max(want, std::min(kPinnedRoots, n))).total;
+            if (ctx->budget == 0 || next <= ctx->budget) ensure_scratch(ctx, next, s);
+            PH_TRY(ensure_scratch(ctx, l.total, s));
+            PH_TRY(count(l));   // growing discards the offsets
+        }
+        PH_TRY(list(l, want));
+    }
+    if (done == want) return PH_OK;
+    // the others
+    const size_t rest = (size_t)(want - done);
+    const auto *d_roots = at<long long>(ctx, l.head + kRootHeader) + done;
+    if (!boxes) {
+        static_assert(sizeof(long long) == sizeof(int64_t), "roots are copied as they are");
+        PH_CUDA(cudaMemcpyAsync(out_host + done, d_roots, sizeof(long long) * rest, cudaMemcpyDeviceToHost, s),
+                "copy roots");
+        PH_CUDA(cudaStreamSynchronize(s), "cudaStreamSynchronize");
+        return PH_OK;
+    }
     std::vector<long long> all_roots;
     std::vector<int> all_boxes;
-    if (want > have) {
+    long long *roots = h_roots;
+    int *bx = h_box;
+    if (want > kPinnedRoots) {
         all_roots.resize((size_t)want);
-        all_boxes.resize(boxes ? (size_t)want * 4 : 0);
-        PH_TRY(query(want, all_roots.data(), all_boxes.data()));
+        all_boxes.resize((size_t)want * 4);
         roots = all_roots.data();
         bx = all_boxes.data();
     }
-    for (int64_t r = 0; r < want; ++r) {
-        if (!boxes) { out_host[r] = roots[r]; continue; }
-        // (root, x_min, y_min, x_max, y_max), 1-based; x = slow axis
-        out_host[5 * r] = roots[r];
-        for (int q = 0; q < 4; ++q) out_host[5 * r + 1 + q] = bx[4 * r + q] + 1;
-    }
+    PH_CUDA(cudaMemcpyAsync(roots + done, d_roots, sizeof(long long) * rest, cudaMemcpyDeviceToHost, s), "copy roots");
+    PH_CUDA(cudaMemcpyAsync(bx + 4 * done, at<int>(ctx, l.box) + 4 * done, sizeof(int) * 4 * rest,
+                            cudaMemcpyDeviceToHost, s), "copy boxes");
+    PH_CUDA(cudaStreamSynchronize(s), "cudaStreamSynchronize");
+    emit(done, want, roots, bx);
     return PH_OK;
 }
 

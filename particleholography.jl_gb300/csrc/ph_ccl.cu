@@ -444,6 +444,9 @@ cudaError_t ccl_launch(const void *img, bool is_bool, uint32_t *lab, int64_t row
 // boxes[4 r .. 4 r + 3] = (min slow, min fast, max slow, max fast) over the pixels
 // of the root of rank r < count (0-based).  VEC: four pixels of one row per thread
 // (16-byte aligned labels, cols a multiple of 4), one update per run of equal labels.
+// An update that the box already covers is left out: the values only grow outwards, so
+// a value read earlier is as good (a component's pixels all update one box, and the
+// atomics on it ran one after the other: 2048^2 of ones 11 ms pixel by pixel).
 template <bool VEC>
 __global__ void __launch_bounds__(256)
     k_boxes(const uint32_t *__restrict__ lab, int64_t n, uint32_t cols, int64_t slice_n, const unsigned *__restrict__ rank,
@@ -473,10 +476,11 @@ __global__ void __launch_bounds__(256)
         const unsigned r = rank[base + l[k] - 1];
         if ((int64_t)r >= count) continue;
         int *b = boxes + 4 * (int64_t)r;
-        atomicMin(b + 0, slow);
-        atomicMin(b + 1, fast + k);
-        atomicMax(b + 2, slow);
-        atomicMax(b + 3, fast + e);
+        const int4 now = __ldcg(reinterpret_cast<const int4 *>(b));
+        if (slow < now.x) atomicMin(b + 0, slow);
+        if (fast + k < now.y) atomicMin(b + 1, fast + k);
+        if (slow > now.z) atomicMax(b + 2, slow);
+        if (fast + e > now.w) atomicMax(b + 3, fast + e);
     }
 }
 
@@ -590,29 +594,48 @@ __global__ void __launch_bounds__(kScanThreads) k_roots_scan(unsigned *counts, i
 
 // Writes the 1-based linear index of every root, in increasing order, and (rank
 // non-null) rank[i] = the root's position in that order.  offsets: the scanned
-// counts; a block without roots is done at once.
+// counts; a block without roots is done at once.  Adjacent threads write adjacent
+// roots (with 32 elements per thread, one after the other, dense roots cost more than
+// the pass over the labels).
 __global__ void __launch_bounds__(kRootThreads)
     k_roots_write(const uint32_t *__restrict__ lab, int64_t n, int64_t slice_n, const unsigned *offsets, int64_t nb,
                   const unsigned long long *total, long long *out, int64_t cap, unsigned *rank) {
-    __shared__ unsigned roots[kRootTile / 32];   // one bit per element of the block
+    constexpr int WORDS = kRootTile / 32;
+    __shared__ unsigned roots[WORDS], before[WORDS];   // one bit per element of the block; roots before its word
+    __shared__ unsigned warp_sum[WORDS / 32];
     const unsigned first = offsets[blockIdx.x];
     const unsigned last = (int64_t)blockIdx.x + 1 < nb ? offsets[blockIdx.x + 1] : (unsigned)*total;
     if (first == last) return;
-    if (threadIdx.x < kRootTile / 32) roots[threadIdx.x] = 0;
+    if (threadIdx.x < WORDS) roots[threadIdx.x] = 0;
     __syncthreads();
     block_labels(lab, n, slice_n, [&](int j, uint32_t, bool root) {
         if (root) atomicOr(&roots[j >> 5], 1u << (j & 31));
     });
     __syncthreads();
-    if (threadIdx.x < kRootTile / 32) {   // 128 threads, 32 elements each
-        unsigned m = roots[threadIdx.x], pre = first;
-        for (unsigned q = 0; q < threadIdx.x; ++q) pre += __popc(roots[q]);
-        const int64_t base = (int64_t)blockIdx.x * kRootTile + threadIdx.x * 32;
-        for (; m; m &= m - 1, ++pre) {
-            const int64_t i = base + __ffs(m) - 1;
-            if ((int64_t)pre < cap && out) out[pre] = (long long)(i + 1);
-            if (rank) rank[i] = pre;
+    unsigned c = 0, incl = 0;
+    if (threadIdx.x < WORDS) {   // (whole warps)
+        c = incl = __popc(roots[threadIdx.x]);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned u = __shfl_up_sync(0xffffffffu, incl, o);
+            if ((threadIdx.x & 31) >= o) incl += u;
         }
+        if ((threadIdx.x & 31) == 31) warp_sum[threadIdx.x >> 5] = incl;
+    }
+    __syncthreads();
+    if (threadIdx.x < WORDS) {
+        unsigned pre = first + incl - c;
+        for (unsigned w = 0; w < threadIdx.x >> 5; ++w) pre += warp_sum[w];
+        before[threadIdx.x] = pre;
+    }
+    __syncthreads();
+    const int64_t base = (int64_t)blockIdx.x * kRootTile;
+    for (int j = threadIdx.x; j < kRootTile; j += kRootThreads) {
+        const unsigned m = roots[j >> 5], bit = 1u << (j & 31);
+        if (!(m & bit)) continue;
+        const unsigned pre = before[j >> 5] + __popc(m & (bit - 1));
+        if ((int64_t)pre < cap && out) out[pre] = (long long)(base + j + 1);
+        if (rank) rank[base + j] = pre;
     }
 }
 
@@ -636,7 +659,7 @@ cudaError_t roots_write_launch(const uint32_t *lab, int64_t n, int64_t slice_n, 
     return cudaGetLastError();
 }
 
-// Boxes of the roots of rank < count (their ranks are in `rank`, see k_roots_write).
+// Boxes of the roots of rank < count (their ranks are in `rank`, see k_roots_write); 16-byte aligned.
 cudaError_t boxes_launch(const uint32_t *lab, int64_t rows, int64_t cols, int64_t slice_rows, const unsigned *rank,
                          int *boxes, int64_t count, cudaStream_t s, int64_t *launches) {
     if (count > 0) k_boxes_init<<<(unsigned)((count + 255) / 256), 256, 0, s>>>(boxes, count);
