@@ -195,9 +195,9 @@ cudaError_t transfer_sqrt_launch(float *out, int nx, int ny, double wavlen, doub
 // host forms it in double-double), times the 24-bit mantissa of s = sqrt(d),
 // shifted by its exponent, modulo 2^64: exact to 2^-40 turn.  The nearest of 256
 // table angles, as FP32 pairs hi + lo, is rotated by the rest (below pi / 256) in
-// FP32 with short Taylor series, whose result enters as a correction below 0.013:
-// the sum is within 1e-9 of the exact value before its one rounding.  0.013 ms at
-// 2048^2 (integer and FP32 arithmetic, about 35 operations per value).
+// FP32 with short Taylor series, whose result enters as a correction below 0.013, good
+// to a few roundings of that size: the sum is within 3e-9 of the exact value before its
+// one rounding.  0.013 ms at 2048^2 (integer and FP32 arithmetic, about 35 operations per value).
 // s outside [2^-30, 1], NaN: the FP64 form.
 struct TurnRate {
     unsigned long long lo;
