@@ -1162,10 +1162,10 @@ int rounds_group(int nbatch, int ctas, int per_sm, int start, int cap_override) 
 
 // Slices per CTA of pass A (rows kx of length ny) and of pass B (`items` frames
 // of rows y of length nx) over a batch of nbatch slices.
-bool two_a(ReconPath path, int ny, int y0, int ny_out) { return path == PATH_TWO && recon_a_two(ny, y0, ny_out); }
+bool two_a(ReconPath path, int ny) { return path == PATH_TWO && recon_a_two(ny); }   // (its frames are whole ones)
 bool tstore_a(int ny, int y0, int ny_out) { return recon_a_tstore(ny) && y0 == 0 && ny_out == ny; }
 int recon_group_a(ReconPath path, int nbatch, int nx, int ny, int y0, int ny_out, int cap_override) {
-    if (two_a(path, ny, y0, ny_out)) {
+    if (two_a(path, ny)) {
         const int box = recon_a_two_box(ny);
         return rounds_group(nbatch, (nx + box - 1) / box, recon_a_two_ctas_per_sm(ny), 3, cap_override);
     }
@@ -1259,7 +1259,7 @@ int issue_recon_slices(ph_ctx *ctx, ReconKind kind, float *proj, int32_t *argmin
         ReconA a{};
         fill_a(a);
         CUtensorMap tm;
-        if (two_a(path, ny, y0, ny_out) && t_store_map(&tm, t, nx, ny_out, nb, recon_a_two_box(ny), recon_a_two_box_y(ny))) {
+        if (two_a(path, ny) && t_store_map(&tm, t, nx, ny_out, nb, recon_a_two_box(ny), recon_a_two_box_y(ny))) {
             PH_TRY(pass(ctx, s, "recon_a", [&] { return launch_recon_a_two(ny, a, tm, nb, s); }));
         } else if (path == PATH_ROWS && tstore_a(ny, y0, ny_out) &&
                    t_store_map_plain(&tm, t, nx, ny_out, nb, recon_a_tstore_box(ny))) {
@@ -1514,7 +1514,7 @@ int issue_recon_group(ph_ctx *ctx, const std::vector<const ph_recon_item *> &its
         a.nitems = G;
         a.err = static_cast<int *>(ctx->small);
         CUtensorMap tm;
-        if (recon_a_two(ny, 0, ny) && t_store_map_items(&tm, a.t, nx, ny, L.batch, G, ib, recon_a_two_box(ny), recon_a_two_box_y(ny))) {
+        if (recon_a_two(ny) && t_store_map_items(&tm, a.t, nx, ny, L.batch, G, ib, recon_a_two_box(ny), recon_a_two_box_y(ny))) {
             PH_TRY(pass(ctx, s, "recon_a", [&] { return launch_recon_a_group_two(ny, a, tm, s); }));
         } else {
             PH_TRY(pass(ctx, s, "recon_a", [&] { return launch_recon_a_group(ny, a, s); }));

@@ -3,9 +3,7 @@
 
 namespace ph {
 
-bool recon_a_two(int n, int y0, int ny_out) {
-    return two::supported(n) && y0 % two::box_y(n) == 0 && ny_out % two::box_y(n) == 0;
-}
+bool recon_a_two(int n) { return two::supported(n); }
 
 int recon_a_two_box(int n) {
     switch (n) {

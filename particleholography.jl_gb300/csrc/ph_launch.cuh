@@ -286,11 +286,10 @@ bool recon_two(int n);
 cudaError_t launch_fwd_rows_two(int n, const FwdRowsT<FWD_COMPLEX> &b, cudaStream_t s);
 cudaError_t launch_fwd_rows_two(int n, const FwdRowsT<FWD_SQRT_REAL> &b, cudaStream_t s);
 cudaError_t launch_spectrum_two(int n, const SpectrumCols &b, cudaStream_t s);
-// Pass A: frames whose stored rows [y0, y0 + ny_out) are whole boxes.  tm: T as
-// (kx, y, slice) or, grouped, (kx, y, slice, item), 8-byte elements, boxes of
+// Pass A, whole frames (y0 = 0, ny_out = n).  tm: T as (kx, y, slice) or, grouped, (kx, y, slice, item), 8-byte elements, boxes of
 // recon_a_two_box(n) kx x recon_a_two_box_y(n) y, swizzled by the box's row of kx.
 // Its CTAs per SM.
-bool recon_a_two(int n, int y0, int ny_out);
+bool recon_a_two(int n);
 int recon_a_two_box(int n);
 int recon_a_two_box_y(int n);
 int recon_a_two_ctas_per_sm(int n);

@@ -549,6 +549,7 @@ struct ReconAT : PassBase, std::conditional_t<GROUPED, ReconItems, NoItems> {
         using S = Shape<N, EPT, TT>;
         constexpr int ROWS = S::ROWS;
         constexpr int FORM = form<N, RF>();
+        static_assert(!(TSTORE && GROUPED), "the tensor-map store takes one item");
         static_assert(!TSTORE || tstore_ok<N>(), "tensor-map store: 4..32 rows per CTA or 2 in a cluster of 2, N a multiple of 256");
         unsigned char *xbase = smem + stage_total<N, RF>();
         constexpr int CS = cluster<N>();
@@ -701,14 +702,8 @@ struct ReconAT : PassBase, std::conditional_t<GROUPED, ReconItems, NoItems> {
                     named_bar_sync(1, S::THREADS);
                     if (threadIdx.x == 0) {
 #pragma unroll 1
-                        for (int q = 0; q < N / kBoxY; ++q) {
-                            if constexpr (GROUPED) {   // one map over the items' slots: (kx, y, slice, item)
-                                tma_store_4d(tmap, stg + (size_t)q * kBoxY * ROWS, kx0, q * kBoxY, b,
-                                             (int)blockIdx.z);
-                            } else {
-                                tma_store_3d(tmap, stg + (size_t)q * kBoxY * ROWS, kx0, q * kBoxY, b);
-                            }
-                        }
+                        for (int q = 0; q < N / kBoxY; ++q)
+                            tma_store_3d(tmap, stg + (size_t)q * kBoxY * ROWS, kx0, q * kBoxY, b);
                         bulk_commit();
                     }
                 } else {

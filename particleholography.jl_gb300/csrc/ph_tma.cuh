@@ -179,12 +179,6 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const void *tmap, int x, 
         : "memory");
 }
 
-// The 4-D form: element coordinates (x, y, z, w).
-__device__ __forceinline__ void tma_store_4d(const void *tmap, const void *src, int x, int y, int z, int w) {
-    asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(tmap),
-                 "r"(smem_addr(src)), "r"(x), "r"(y), "r"(z), "r"(w)
-                 : "memory");
-}
 // L2 policy of data that is written (or read) once and not used again before it
 // would be evicted anyway: it makes room first.
 __device__ __forceinline__ uint64_t l2_evict_first() {
@@ -192,7 +186,7 @@ __device__ __forceinline__ uint64_t l2_evict_first() {
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
     return p;
 }
-// The 3-D and 4-D stores with an L2 policy.
+// The 3-D store with an L2 policy, and the 4-D one: element coordinates (x, y, z, w).
 __device__ __forceinline__ void tma_store_3d(const void *tmap, const void *src, int x, int y, int z, uint64_t policy) {
     asm volatile(
         "cp.async.bulk.tensor.3d.global.shared::cta.bulk_group.L2::cache_hint [%0, {%2, %3, %4}], [%1], %5;" ::"l"(tmap),

@@ -285,10 +285,8 @@ __global__ void __launch_bounds__(PassA<N>::THREADS, PassA<N>::CTAS)
 #pragma unroll 1
                 for (int q = 0; q < N / C::BOX_Y; ++q) {
                     const unsigned char *box = stage + (size_t)q * C::BOX_Y * RB * 8;
-                    const int yo = q * C::BOX_Y - p.y0;   // (a cropped frame: whole boxes inside it)
-                    if (yo < 0 || yo >= p.ny_out) continue;
-                    if constexpr (GROUPED) tma_store_4d(&tmap, box, kx0, yo, b, (int)blockIdx.z, policy);
-                    else tma_store_3d(&tmap, box, kx0, yo, b, policy);
+                    if constexpr (GROUPED) tma_store_4d(&tmap, box, kx0, q * C::BOX_Y, b, (int)blockIdx.z, policy);
+                    else tma_store_3d(&tmap, box, kx0, q * C::BOX_Y, b, policy);
                 }
                 bulk_commit();
             }

@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(128, PassB<N, EPI, GROUPED, SLICE>::CTAS) k_tw
     const int r = threadIdx.x / C::TPR, h = threadIdx.x / L % H, l = threadIdx.x % L;
     const int y = blockIdx.x * ROWS + r;
     const bool valid = y < p.rows;
-    const bool track = EPI == EPI_PROJ || (EPI == EPI_VOL && (SLICE ? proj64 != nullptr : p.proj32 != nullptr));
+    const bool track = EPI == EPI_PROJ || (EPI == EPI_VOL && p.proj32 != nullptr);   // (volumes without SLICE only)
     if constexpr (C::MIN) {
         if (warp == 0) tc::tmem_alloc(slot, C::COLS);
     }

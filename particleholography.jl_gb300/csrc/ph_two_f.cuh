@@ -64,6 +64,7 @@ __device__ __forceinline__ void transform(const float2 *__restrict__ tw, float *
 
 template <int N, int MODE>
 __global__ void __launch_bounds__(PassF<N>::THREADS, PassF<N>::CTAS) k_two_fwd(const FwdRowsT<MODE> p) {
+    static_assert(MODE == FWD_COMPLEX || MODE == FWD_SQRT_REAL, "padded frames run the row engine");
     using C = PassF<N>;
     using PL = Plan<N>;
     extern __shared__ __align__(128) unsigned char ph_smem[];
@@ -74,7 +75,6 @@ __global__ void __launch_bounds__(PassF<N>::THREADS, PassF<N>::CTAS) k_two_fwd(c
     float2 *dst = p.dst + (size_t)z * p.dst_stride;
     const int y0 = blockIdx.x * C::RB, r = threadIdx.x / PL::L, l = threadIdx.x % PL::L;
     const int y = min(y0 + r, p.nrows - 1);   // (rows beyond the last: its values again, not stored)
-    const float2 mean = MODE == FWD_PADDED ? *p.pad_mean : make_float2(0.f, 0.f);
     float2 *stage = reinterpret_cast<float2 *>(ph_smem);
     float *ex = reinterpret_cast<float *>(ph_smem + C::STAGE + r * C::XB);
     // (the square root's rare path is a branch: with each load beside its root, 32
@@ -85,15 +85,8 @@ __global__ void __launch_bounds__(PassF<N>::THREADS, PassF<N>::CTAS) k_two_fwd(c
         for (int i = 0; i < PL::E; ++i) real[i] = __ldg(src_real + (size_t)y * N + l + PL::L * i);
     }
     const auto load = [&](int i) -> float2 {
-        const int x = l + PL::L * i;
-        if constexpr (MODE == FWD_COMPLEX) {
-            return src[(size_t)y * N + x];
-        } else if constexpr (MODE == FWD_SQRT_REAL) {
-            return make_float2(sqrtf(real[i]), 0.f);
-        } else {
-            const int yi = y - p.pad_off, xi = x - p.pad_off;
-            return yi >= 0 && yi < p.ny_in && xi >= 0 && xi < p.nx_in ? src[(size_t)yi * p.nx_in + xi] : mean;
-        }
+        if constexpr (MODE == FWD_COMPLEX) return src[(size_t)y * N + l + PL::L * i];
+        else return make_float2(sqrtf(real[i]), 0.f);
     };
     transform<N, false>(p.tw, ex, r, l, load, [&](int k, float2 v) { stage[r * C::PITCH + k] = v; });
     __syncthreads();
