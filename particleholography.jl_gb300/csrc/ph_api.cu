@@ -880,7 +880,7 @@ bool tf_load_map(CUtensorMap *tm, const float2 *h, int nx, int ny, int rows) {
 // that round the intensity to few bits (Float16, N0f8; padded and sub-volumes are N0f8)
 // stay on the row engine and keep their values: a last bit of Float32 that differs moves
 // whole steps of theirs, up to 2^-10 in a Float16 volume's projection.  (1024^2 x 27
-// Float16: 0.208 ms; Float32 volumes 1.4 .. 3.7 times faster than on the row engine.)
+// Float16: 0.208 ms; Float32 volumes 1.26 .. 3.9 times faster than on the row engine.)
 enum ReconPath { PATH_ROWS, PATH_TWO };
 bool two_rows(ReconPath path, int n) { return path == PATH_TWO && recon_two(n); }
 
@@ -1821,8 +1821,8 @@ int32_t ph_phase_retrieval(ph_ctx *ctx, void *out, const float *holo1, const flo
     // the transfers as [kx][ky] rows and the amplitudes; a context that has no room for
     // them (its budget, a capture, the device) runs the one-shot passes where it did.
     // Two-stage where the persistent form does not exist: per pass, one-shot and
-    // two-stage, 12.6 and 3.0 us at 256^2, 12.3 and 5.8 at 512^2, 19.2 and 6.3 at 768^2,
-    // 43.5 and 28.7 at 1536^2; persistent and two-stage, 8.2 and 8.4 us at 1024^2, 28 and
+    // two-stage, 12.6 and 2.7 us at 256^2, 12.3 and 6.4 at 512^2, 19.2 and 6.1 at 768^2,
+    // 43.5 and 25.8 at 1536^2; persistent and two-stage, 8.2 and 8.4 us at 1024^2, 28 and
     // 45 at 2048^2, 149 and 163 at 4096^2 (there 64 values per thread leave 8 warps per SM).
     const bool persistent = gs_persistent(nx, ny);
     bool two_stage = !persistent && gs_two(nx) && gs_two(ny);

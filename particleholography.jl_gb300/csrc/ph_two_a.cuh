@@ -28,8 +28,8 @@ namespace two {
 //
 // In the row engine this pass moved 87 bytes per voxel through the shared-memory
 // data path (chain 24, two exchanges 32, staging 16, twiddles 15); here 32 to 40.
-// Per launch, before and now: 1024^2 x 256 0.68 and 0.48 ms, 2048^2 x 512 5.43
-// and 4.55 ms, 4096^2 x 128 9.3 and 5.06 ms (no more clusters).  What is left:
+// Per launch, before and now: 1024^2 x 256 0.68 and 0.47 ms, 2048^2 x 512 5.43
+// and 4.55 ms, 4096^2 x 128 9.3 and 5.15 ms (no more clusters).  What is left:
 // arithmetic and its latency (50 % of the FP32 pipe, 45 to 54 % of issue slots),
 // then the stores: without them 0.46 ms at 1024.
 //
@@ -41,9 +41,9 @@ namespace two {
 // two groups of tensor-memory columns per wait.
 //
 // 3 * 2^a lengths (12, 24 or 48 values per thread; a quarter of the threads idle
-// in stage 2), per launch in the row engine and here: 384^2 x 512 0.83 and 0.15 ms,
-// 768^2 x 256 1.13 and 0.31 ms, 1536^2 x 256 3.25 and 1.42 ms, 3072^2 x 64 3.49 and
-// 1.63 ms (the engine has no tensor-map store there and reads the phase rates from
+// in stage 2), per launch in the row engine and here: 384^2 x 512 0.83 and 0.16 ms,
+// 768^2 x 256 1.13 and 0.33 ms, 1536^2 x 256 3.25 and 1.48 ms, 3072^2 x 64 3.49 and
+// 1.74 ms (the engine has no tensor-map store there and reads the phase rates from
 // L2 for every slice).
 
 // y per box: the largest of 256, 128, 64 that divides the length.

@@ -7,8 +7,8 @@
 // a warp) per row.  What bounds it is latency: at 1024^2 a pass is 256 CTAs that run
 // once, so its time is one row's (loads, four butterflies stages, two exchanges)
 // plus the launch, which overlaps the previous pass's end (programmatic dependent
-// launch).  Per pass, against the one-shot passes of the row engine: 3.0 us (12.6)
-// at 256^2, 6.3 us (19.2) at 768^2.  A whole propagation at 2048^2, its transfer
+// launch).  Per pass, against the one-shot passes of the row engine: 2.7 us (12.6)
+// at 256^2, 6.1 us (19.2) at 768^2.  A whole propagation at 2048^2, its transfer
 // formed as the rows that the column pass reads: 90 us (the row engine's 99, with
 // the transfers gathered).
 #pragma once
