@@ -114,10 +114,10 @@ constexpr int kMaxGraphs = 32;
 
 // ---------------------------------------------------------------- setup kernels
 
-__device__ __forceinline__ float2 twiddle_fp64(int i, int n) {   // W_n^i rounded from FP64
+__device__ __forceinline__ float2 twiddle_fp64(int i, int n, double gain = 0.0) {   // W_n^i (1 + gain) rounded from FP64
     double s, c;
     sincospi(-2.0 * (double)i / (double)n, &s, &c);
-    return make_float2((float)c, (float)s);
+    return make_float2((float)(c + c * gain), (float)(s + s * gain));
 }
 
 // w_j = (cos, sin)(2 pi j / n) in FP64, stored as FP32 pairs (cos hi, cos lo, sin hi, sin lo).
@@ -145,19 +145,45 @@ __global__ void k_twiddle_stage(float2 *blk, int n, int radix, int ns) {
     blk[e] = twiddle_fp64(r * k * (n / (ns * radix)), n);
 }
 
-// The stage factors of the two-stage transform (layout in ph_two.cuh): of length r
-// over `lanes` threads, [factor][l], split r = p q.
-__global__ void k_two_factors(float2 *out, int n, int lanes, int p, int q) {
+// The stage factors of the two-stage transform (layout in ph_two.cuh): split p q over
+// `lanes` threads, [factor][h][l]; the gain goes into the first ones, of which every
+// output has at most one.
+__global__ void k_two_factors(float2 *out, int n, int lanes, int p, int q, int halves, double gain) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (p + q - 2) * lanes) return;
-    const int l = i % lanes, j = i / lanes;
-    out[i] = twiddle_fp64(l * (j < p - 1 ? j + 1 : p * (j - p + 2)), n);
+    const int first = halves > 1 ? 0 : 1, na = p - first;
+    if (i >= (na + q - 1) * halves * lanes) return;
+    const int l = i % lanes, h = i / lanes % halves, j = i / (halves * lanes);
+    const int e = j < na ? halves * (j + first) + h : halves * p * (j - na + 1);
+    out[i] = twiddle_fp64(l * e, n, j < na ? gain : 0.0);
 }
 
 // Its stage twiddles W^(l k) as [k][l < lanes].
-__global__ void k_two_twiddles(float2 *out, int n, int lanes) {
+__global__ void k_two_twiddles(float2 *out, int n, int lanes, double gain) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = twiddle_fp64(i % lanes * (i / lanes), n);
+    if (i < n) out[i] = twiddle_fp64(i % lanes * (i / lanes), n, gain);
+}
+
+// What the constants of a butterfly of size r, rounded to Float32, do to the modulus of a
+// random input, on average over its outputs: the mean of their moduli minus one, over the
+// twiddles between its two levels and the constants inside of them.
+double constant_modulus(int k, int r) {   // |W_r^k rounded| - 1; 1, i and so on are exact
+    if (4 * k % r == 0) return 0.0;
+    const double a = 2.0 * M_PI * k / r;
+    return hypot((double)(float)cos(a), (double)(float)sin(a)) - 1.0;
+}
+double butterfly_gain(int r) {
+    const double e3 = (double)(float)(0.5 * sqrt(3.0)) / (0.5 * sqrt(3.0)) - 1.0;
+    switch (r) {
+        case 1: case 2: case 4: return 0.0;
+        case 3: return e3 / 3.0;                                 // two of three outputs take two of three inputs by |W_3|
+        case 6: return e3 / 3.0 + e3 / 4.0;                      // and two of six inputs of its triples by |W_6|
+        case 8: return 0.25 * constant_modulus(1, 8);            // half of the outputs take half of the inputs by W_8
+    }
+    const int p = two::split_p_of(r), q = r / p;
+    double sum = 0.0;
+    for (int n2 = 0; n2 < q; ++n2)
+        for (int k1 = 0; k1 < p; ++k1) sum += constant_modulus(n2 * k1, r);
+    return butterfly_gain(p) + butterfly_gain(q) + sum / r;
 }
 
 // holofunc.jl:8-15 with the reference's Float64 operation order; the
@@ -683,12 +709,24 @@ int get_twiddles(ph_ctx *ctx, int n, cudaStream_t s, const float2 **out) {
         PH_CUDA(cudaGetLastError(), "k_twiddle_stage");
     }
     if (two_stage) {
-        const int E = two::values(n), L = n / E;
-        const int pp = two::split_p_of(E), cnt = two::factors_of(E, L);
-        k_two_factors<<<(cnt + 255) / 256, 256, 0, s>>>(p + two::factors_offset(n), n, L, pp, E / pp);
-        k_two_twiddles<<<(n + 255) / 256, 256, 0, s>>>(p + two::twiddle_offset(n), n, L);
-        k_two_twiddles<<<(n + 255) / 256, 256, 0, s>>>(p + two::mirror_offset(n), n, E);
-        ctx->launches += 3;
+        const auto factors = [&](int offset, int r, int lanes, int halves, double gain) {
+            const int pp = two::split_p_of(r), cnt = two::factors_of(r, lanes, halves);
+            k_two_factors<<<(cnt + 255) / 256, 256, 0, s>>>(p + offset, n, lanes, pp, r / pp, halves, gain);
+            ctx->launches++;
+        };
+        // (the first output of a stage has no twiddle, or no first factor: the others make up for it)
+        const int E = two::values(n), L = n / E, P = two::split_p_of(E);
+        const double gain = -(butterfly_gain(E) + butterfly_gain(L));
+        factors(two::factors_offset(n), E, L, 1, gain * P / (P - 1));
+        k_two_twiddles<<<(n + 255) / 256, 256, 0, s>>>(p + two::twiddle_offset(n), n, L, gain * E / (E - 1));
+        k_two_twiddles<<<(n + 255) / 256, 256, 0, s>>>(p + two::mirror_offset(n), n, E, gain * L / (L - 1));
+        ctx->launches += 2;
+        if (two::halves(n) > 1) {
+            const int e = two::values(n / 2), l = n / 2 / e;
+            double odd = 0.0;   // the odd half's W_(n / l)^i
+            for (int i = 0; i < e; ++i) odd += constant_modulus(i, n / l);
+            factors(two::half_offset(n), e, l, 2, -(butterfly_gain(e) + butterfly_gain(l) + 0.5 * odd / e));
+        }
         PH_CUDA(cudaGetLastError(), "k_two_twiddles");
     }
     ctx->tw[n] = p;

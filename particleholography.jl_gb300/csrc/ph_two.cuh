@@ -181,15 +181,33 @@ __host__ __device__ constexpr bool supported(int n) {
            n == 2048 || n == 3072 || n == 4096;
 }
 
+// The lengths whose rows pass B transforms as two of half the length (ph_two_b.cuh).
+__host__ __device__ constexpr int halves(int n) { return n == 2048 || n == 1536 ? 2 : 1; }
+
 // A length's table in global memory holds, behind the row engine's (ph_fft.cuh),
-// the stage factors of the transform L-major, [factor][l]: W^(l p), p = 1 .. P - 1,
-// then W^(l P q), q = 1 .. Q - 1; the stage twiddles themselves, W^(l k1) as [k1][l];
-// and those of its mirror (below), W^(t' q1) as [q1][t'].
-__host__ __device__ constexpr int factors_of(int r, int lanes) { return (split_p_of(r) + r / split_p_of(r) - 2) * lanes; }
+//  - the stage factors of the transform, [factor][l]: W^(l p), p = 1 .. P - 1, then
+//    W^(l P q), q = 1 .. Q - 1;
+//  - the stage twiddles themselves, W^(l k1) as [k1][l], and those of its mirror
+//    (below), W^(t' q1) as [q1][t'];
+//  - where halves(n) = 2, the factors of the two transforms of length n / 2,
+//    [factor][h][l]: W^(l (2 p + h)), p = 0 .. P - 1, then W^(2 l P q).
+// All of them but the W^(l P q) carry a gain: the constants of the butterflies round to
+// moduli below one on average (1 / sqrt(2) by 1.7e-8, sqrt(3) / 2 by 1.8e-8), so that a
+// transform shrinks its values by up to 4e-8, all of them alike.  Over the four transforms
+// of a propagation that is 1.5e-7, more than half of its error (noise at 1024^2 2.60e-7,
+// with the gain 2.13e-7, in the row engine 2.37e-7).
+__host__ __device__ constexpr int factors_of(int r, int lanes, int h) {
+    return (split_p_of(r) + r / split_p_of(r) - (h > 1 ? 1 : 2)) * h * lanes;
+}
 __host__ __device__ constexpr int factors_offset(int n) { return plan_tw_size(n, engine_e(n, PassBase::EPT)); }
-__host__ __device__ constexpr int twiddle_offset(int n) { return factors_offset(n) + factors_of(values(n), n / values(n)); }
+__host__ __device__ constexpr int twiddle_offset(int n) {
+    return factors_offset(n) + factors_of(values(n), n / values(n), 1);
+}
 __host__ __device__ constexpr int mirror_offset(int n) { return twiddle_offset(n) + n; }
-__host__ __device__ constexpr int table_size(int n) { return mirror_offset(n) + n; }
+__host__ __device__ constexpr int half_offset(int n) { return mirror_offset(n) + n; }
+__host__ __device__ constexpr int table_size(int n) {
+    return half_offset(n) + (halves(n) > 1 ? factors_of(values(n / 2), n / 2 / values(n / 2), 2) : 0);
+}
 
 template <int N>
 struct Plan {
@@ -211,18 +229,12 @@ struct Factors {
     static constexpr int COUNT = PL::P - P0 + PL::Q - 1;
     static constexpr size_t BYTES = (size_t)COUNT * H * PL::L * 8;
     float2 a[PL::P], b[PL::Q];
-    // The CTA's table [factor][h][l], so that a warp's loads are contiguous (from
-    // the W^i table they would be gathers of up to 32 lines).  tw: the table of H N.
+    // The CTA's copy of the table, [factor][h][l], so that a warp's loads are contiguous
+    // (from the W^i table they would be gathers of up to 32 lines).  tw: the table of H N.
     __device__ __forceinline__ static void fill(float2 *tab, const float2 *__restrict__ tw) {
-        if constexpr (H == 1) {   // as it stands in the length's table
-            for (int i = threadIdx.x; i < COUNT * PL::L; i += blockDim.x) tab[i] = load_tw<INV>(tw, factors_offset(N) + i);
-            return;
-        }
-        for (int i = threadIdx.x; i < COUNT * H * PL::L; i += blockDim.x) {
-            const int l = i % PL::L, h = i / PL::L % H, j = i / (PL::L * H);
-            const int e = j < PL::P - P0 ? H * (j + P0) + h : H * PL::P * (j - (PL::P - P0) + 1);
-            tab[i] = load_tw<INV>(tw, l * e);
-        }
+        static_assert(COUNT * H * PL::L == factors_of(PL::E, PL::L, H), "as the table holds them");
+        constexpr int at = H == 1 ? factors_offset(N) : half_offset(H * N);
+        for (int i = threadIdx.x; i < COUNT * H * PL::L; i += blockDim.x) tab[i] = load_tw<INV>(tw, at + i);
     }
     __device__ __forceinline__ void load(const float2 *tab, int l, int h = 0) {
         tab += h * PL::L + l;

@@ -30,7 +30,7 @@ namespace two {
 // and neither an unpacking kernel nor a 64-bit word per pixel.
 template <int N, int EPI, bool GROUPED, bool SLICE = true>
 struct PassB {
-    static constexpr int H = N == 2048 || N == 1536 ? 2 : 1;         // transforms a row is split into
+    static constexpr int H = halves(N);                      // transforms a row is split into
     using PL = Plan<N / H>;
     static constexpr int THREADS = 128;
     static constexpr int TPR = H * PL::L;                    // threads per row
