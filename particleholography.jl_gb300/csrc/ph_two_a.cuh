@@ -88,8 +88,8 @@ __device__ __forceinline__ float2 unit_power(uint32_t turns, float w, const floa
     const float sn = fmaf(x * x2, fmaf(x2, 1.0f / 120.0f, -1.0f / 6.0f), x);
     const float cs1 = x2 * fmaf(x2, fmaf(x2, -1.0f / 720.0f, 1.0f / 24.0f), -0.5f);   // cos - 1
     float c1 = cl + fmaf(ch, cs1, -sh * sn), s1 = sl + fmaf(sh, cs1, ch * sn);
-    if (fabsf(w) < 0.015625f) {   // the modulus minus one, whose rounding is not that of a value near one
-        const float y = w * 0.69314718055994530942f, m1 = y * fmaf(y, fmaf(y, 1.0f / 6.0f, 0.5f), 1.0f);
+    if (fabsf(w) < 0x1p-14f) {   // the modulus minus one, whose rounding is not that of a value near one
+        const float m1 = w * 0.69314718055994530942f;   // (its square is below 2e-9)
         c1 = fmaf(ch + c1, m1, c1);
         s1 = fmaf(sh + s1, m1, s1);
         return make_float2(ch + c1, sh + s1);
@@ -198,10 +198,15 @@ __global__ void __launch_bounds__(PassA<N>::THREADS, PassA<N>::CTAS)
                 for (int n1 = 0; n1 < P; ++n1) cur[n1] = st[n1];
                 if (n2 + 1 < Q) read(n2 + 1);   // the next group's state is on its way
                 float2 t[P];
+                if (k == ahead) {   // (the first CHAIN slices start from X_0 as it is)
 #pragma unroll
-                for (int n1 = 0; n1 < P; ++n1)
-                    t[n1] = rotated(make_float2(cur[n1].x, cur[n1].y), (k - ahead) * __float_as_uint(cur[n1].z),
-                                    (float)(k - ahead) * cur[n1].w);
+                    for (int n1 = 0; n1 < P; ++n1) t[n1] = make_float2(cur[n1].x, cur[n1].y);
+                } else {
+#pragma unroll
+                    for (int n1 = 0; n1 < P; ++n1)
+                        t[n1] = rotated(make_float2(cur[n1].x, cur[n1].y), (k - ahead) * __float_as_uint(cur[n1].z),
+                                        (float)(k - ahead) * cur[n1].w);
+                }
                 if (first) {
                     float2 hd[P];
 #pragma unroll
