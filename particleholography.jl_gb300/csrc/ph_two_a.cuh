@@ -13,7 +13,7 @@ namespace two {
 // at 128 .. 512, two warps per row at 3072 and 4096), so that the exchange needs no CTA
 // barrier.  X_k and Hdz of a thread's values live in tensor memory (4 E columns
 // of its own lane): every slice reads both and writes back X_{k+1} = X_k Hdz.  X
-// is formed anew from the spectrum state at every multiple of CHAIN slices.
+// is formed anew from the spectrum state at every multiple of `chain` slices.
 //
 // Precision: a projection is as near to the 64-bit one as with every slice formed
 // directly by the row engine (relative errors at 12 random distances, there and here:
@@ -22,9 +22,10 @@ namespace two {
 // below a rounding, since its error adds up along the chain, and that of the zero
 // frequency shows in every pixel (with Hdz from sincospif and exp2f: 4.3e-7 at 1024^2,
 // 4.5e-7 at 2048 x 1536); and X from the polynomials of `rotated` rather than __sincosf,
-// which is good to 1e-7 only.  CHAIN is as long as that leaves room for: at 256^2 x 32
-// 27 us with 4 and 29 with 8 (small groups walk to their start), at 512^2 x 64 87 and 83;
-// at 1024^2 x 256 863 with 8 and 842 with 16; at 2048 x 1536 x 157 16 gives 4.0e-7.
+// which is good to 1e-7 only.  A chain is as long as that leaves room for: at 256^2 x 32
+// 27 us with 4 and 29 with 8 (small groups walk to their start), at 4096 x 256 x 48 296
+// and 285, at 512^2 x 64 87 and 83; at 1024^2 x 256 863 with 8 and 842 with 16; at
+// 2048 x 1536 x 157 16 gives 4.0e-7.
 //
 // In the row engine this pass moved 87 bytes per voxel through the shared-memory
 // data path (chain 24, two exchanges 32, staging 16, twiddles 15); here 32 to 40.
@@ -64,7 +65,9 @@ struct PassA {
     static constexpr size_t SMEM = STAGE + RB * XB + F::BYTES + 24;
     static constexpr int BOX_Y = box_y(N);
     // slices between two formations of X
-    static constexpr uint32_t CHAIN = N <= 256 ? 4 : N == 1024 || PL::E == 64 ? 16 : 8;
+    __host__ __device__ static constexpr uint32_t chain(int nx) {
+        return N <= 256 ? (nx < 4096 ? 4 : 8) : N == 1024 || PL::E == 64 ? 16 : 8;
+    }
 };
 
 // Byte offset of (y, row r) in the staging [y][RB], with the tensor map's
@@ -178,10 +181,10 @@ __global__ void __launch_bounds__(PassA<N>::THREADS, PassA<N>::CTAS)
     const uint64_t policy = l2_evict_first();   // T is read by the next pass, long after
     for (int b = b0; b < b1; ++b) {
         tmem_wait_st();
-        const uint32_t k = (uint32_t)(p.k0 + b), ahead = k % C::CHAIN;
+        const uint32_t k = (uint32_t)(p.k0 + b), ahead = k % C::chain(p.nx);
         const bool first = b == b0;
         if (first || ahead == 0) {
-            // X at the last multiple of CHAIN, then the chain's own products: X_k does
+            // X at the last multiple of the chain, then the chain's own products: X_k does
             // not depend on where a group or a range of slices starts.  The first time
             // also Hdz.
             const float4 angle = __ldg(p.ptab + (threadIdx.x & 31) * (kPhaseTable / 32));
@@ -198,7 +201,7 @@ __global__ void __launch_bounds__(PassA<N>::THREADS, PassA<N>::CTAS)
                 for (int n1 = 0; n1 < P; ++n1) cur[n1] = st[n1];
                 if (n2 + 1 < Q) read(n2 + 1);   // the next group's state is on its way
                 float2 t[P];
-                if (k == ahead) {   // (the first CHAIN slices start from X_0 as it is)
+                if (k == ahead) {   // (the first chain starts from X_0 as it is)
 #pragma unroll
                     for (int n1 = 0; n1 < P; ++n1) t[n1] = make_float2(cur[n1].x, cur[n1].y);
                 } else {
